@@ -2,19 +2,19 @@
 // (biot_savart / biot_savart_shift, src/timestep.f90:462-507), one thread per
 // target, source segments staged tile by tile in shared memory.
 //
-// FP64 kernel: the reference's formula
-//   u += G/(2 pi) (d x s)/(4ac - b^2) [(2c+b)/sqrt(a+b+c) - b/sqrt(a)]
-// with d = x_j + shift - x_i, s = ghosti_j - x_j, a=|d|^2, b=2 d.s, c=|s|^2.
-//
-// Mixed kernel: FP32 pair terms in the stable straight-segment form the
+// Both kernels take the pair term in the stable straight-segment form the
 // reference uses for tree leaves (src/tree.f90:380-390),
 //   u += G/(4 pi) (|R1|+|R2|)/(|R1||R2|(|R1||R2| + R1.R2)) R1 x R2,
-// with R1 = x_j + shift - x_i and R2 = ghosti_j + shift - x_i recentred on the
-// target from FP64 data (every FP64 coordinate carried as a hi/lo float pair,
-// so the difference keeps FP64-level information before it is rounded), and
-// Kahan-compensated FP32 accumulation.  The two forms agree analytically; the
-// stable one avoids the (2c+b)/sqrt - b/sqrt cancellation that FP32 cannot
-// afford for far segments.
+// with R1 = x_j + shift - x_i and R2 = ghosti_j + shift - x_i.  It agrees
+// analytically with the reference's direct form
+//   u += G/(2 pi) (d x s)/(4ac - b^2) [(2c+b)/sqrt(a+b+c) - b/sqrt(a)]
+// (d = R1, s = R2 - R1, a = |d|^2, b = 2 d.s, c = |s|^2) without the
+// (2c+b)/sqrt - b/sqrt cancellation of far segments.
+//
+// Mixed kernel: FP32 pair terms, R1 and R2 recentred on the target from FP64
+// data (every FP64 coordinate carried as a hi/lo float pair, so the difference
+// keeps FP64-level information before it is rounded), and Kahan-compensated
+// FP32 accumulation.
 //
 // Skip rules differ between the unshifted and shifted sums exactly as in the
 // reference (src/timestep.f90:471 vs :496).
@@ -23,12 +23,14 @@
 // per-chunk partial sums go to a buffer and are added in fixed chunk order,
 // so results are deterministic.
 
+#include "qv_f64.cuh"
 #include "qv_internal.cuh"
 #include "qv_tma.cuh"
 
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 #define DTILE 128
+#define D64_BLOCKS 3  // FP64 kernel: resident blocks per SM (2, 3 and 4 run within 2 %)
 
 // ------------------------------------------------------------- compaction
 __global__ void k_count_active(int n, const int *__restrict__ inf, int *blk_cnt) {
@@ -200,20 +202,6 @@ __global__ void k_pack_sources(int na, const int *__restrict__ act, const double
   f[15] = __double2float_rn(e2);
 }
 
-// ------------------------------------------------------------ pair terms
-__device__ __forceinline__ void pair64(double dx, double dy, double dz, double sx, double sy,
-                                       double sz, double c, double &ax, double &ay, double &az) {
-  double a = dx * dx + dy * dy + dz * dz;
-  double b = 2. * (dx * sx + dy * sy + dz * sz);
-  double disc = 4. * a * c - b * b;
-  if (disc == 0.) return;  // src/timestep.f90:476
-  double fac = (2. * c + b) * rsqrt(a + b + c) - b * rsqrt(a);
-  double sc = fac / disc;
-  ax += (dy * sz - dz * sy) * sc;
-  ay += (dz * sx - dx * sz) * sc;
-  az += (dx * sy - dy * sx) * sc;
-}
-
 struct Kahan3 {
   float s[3], c[3];
   __device__ __forceinline__ void zero() {
@@ -233,11 +221,6 @@ struct Kahan3 {
   __device__ __forceinline__ double get(int k) const { return (double)s[k] - (double)c[k]; }
 };
 
-
-template <int BC>
-__device__ __forceinline__ void img_mul(int m, int &a, int &b, int &c) {
-  qv_img_shift(BC, m, &a, &b, &c);
-}
 
 __device__ __forceinline__ double shifted(double v, int a, double L) {
   return a == 0 ? v : (a > 0 ? v + L : v - L);
@@ -327,23 +310,130 @@ __device__ __forceinline__ TilePipe make_pipe(const void *src, int j0, int j1, c
 }
 
 // ------------------------------------------------------------ FP64 kernel
+// One thread per target, each staged source summed against it in all images.
+// u = f (R1 x s) per image, and s is the same for all of them: the kernel sums
+// f and f R1 over the images and takes one cross product per source.  R1 takes,
+// per axis, one of three values (shift -L, 0, L), so |R1|^2, R1.s and |R2|^2 =
+// |R1|^2 + 2 R1.s + |s|^2 are sums of per-axis parts, and sum f R1 per axis is
+// the sum over the three shifts of (R1 component) x (sum of f at that shift).
+//
+// Bound: FP64 issue, about 27 operations a pair (two rsqrt_pos and one div_pos
+// are 14 of them).  24,700 points, 27 images: 70.3 ms with the reference's
+// formula pair by pair (library rsqrt and division, 1.3 waves of blocks), 26.4
+// ms now = 6.2e11 pairs/s, 90 % of the FP64 rate (148 SM x 64 lanes x 1.965
+// GHz) at that operation count.
 template <int BC>
-__global__ void __launch_bounds__(DTILE) k_direct64(int na, const int *__restrict__ act,
+struct Img {
+  static constexpr int PX = BC == QV_BC_PERIODIC ? 3 : 1;
+  static constexpr int PY = (BC == QV_BC_PERIODIC || BC == QV_BC_OPENX) ? 3 : 1;
+  static constexpr int PZ = BC == QV_BC_OPEN ? 1 : 3;
+};
+
+template <int P>
+__device__ __forceinline__ void axis_shifts(double d, double L, double *r) {
+  if (P == 3) {
+    r[0] = d - L;
+    r[1] = d;
+    r[2] = d + L;
+  } else {
+    r[0] = d;
+  }
+}
+template <int P>
+__device__ __forceinline__ double least(const double *v) {
+  return P == 3 ? fmin(fmin(v[0], v[1]), v[2]) : v[0];
+}
+
+// Adds the terms of one source (main image unless skip_main, and the images)
+// to (ax, ay, az).  dx, dy, dz = x_j - x_i, c = |s|^2.  fast: every image has
+// |R1| > |s|, hence R1.R2 >= |R1| (|R1| - |s|) > 0 (seg_f_pos).
+template <int BC>
+__device__ __forceinline__ void source64(double dx, double dy, double dz, double sx, double sy,
+                                         double sz, double c, double L, bool fast, bool skip_main,
+                                         const double *rx, const double *px, const double *ry,
+                                         const double *py, const double *rz, const double *pz,
+                                         double &ax, double &ay, double &az) {
+  constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
+  double fx[PX], fy[PY], fz[PZ];  // sum of f at each shift of an axis
+#pragma unroll
+  for (int k = 0; k < PX; k++) fx[k] = 0.;
+#pragma unroll
+  for (int k = 0; k < PY; k++) fy[k] = 0.;
+#pragma unroll
+  for (int k = 0; k < PZ; k++) fz[k] = 0.;
+  if (fast) {
+    // per-axis parts of A = |R1|^2 (p), d = R1.R2 = A + R1.s (g), B = |R2|^2 =
+    // d + R1.s + |s|^2 (t)
+    double gx[PX], tx[PX], gy[PY], ty[PY], gz[PZ], tz[PZ];
+#pragma unroll
+    for (int k = 0; k < PX; k++) { gx[k] = fma(rx[k], sx, px[k]); tx[k] = fma(rx[k], sx, gx[k] + c); }
+#pragma unroll
+    for (int k = 0; k < PY; k++) { gy[k] = fma(ry[k], sy, py[k]); ty[k] = fma(ry[k], sy, gy[k]); }
+#pragma unroll
+    for (int k = 0; k < PZ; k++) { gz[k] = fma(rz[k], sz, pz[k]); tz[k] = fma(rz[k], sz, gz[k]); }
+#pragma unroll
+    for (int a = 0; a < PX; a++) {
+#pragma unroll
+      for (int b = 0; b < PY; b++) {
+        const double pxy = px[a] + py[b], gxy = gx[a] + gy[b], txy = tx[a] + ty[b];
+        double row = 0.;
+#pragma unroll
+        for (int k = 0; k < PZ; k++) {
+          const double f = seg_f_pos(pxy + pz[k], txy + tz[k], gxy + gz[k]);
+          row += f;
+          fz[k] += f;
+        }
+        fx[a] += row;
+        fy[b] += row;
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int m = 0; m < PX * PY * PZ; m++) {
+      const int a = m / (PY * PZ), b = (m / PZ) % PY, k = m % PZ;
+      if (skip_main && m == PX * PY * PZ / 2) continue;  // the middle one is unshifted
+      const double X = PX == 3 ? dx + (a - 1) * L : dx, Y = PY == 3 ? dy + (b - 1) * L : dy,
+                   Z = PZ == 3 ? dz + (k - 1) * L : dz;
+      const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
+      const double cx = Y * sz - Z * sy, cy = Z * sx - X * sz, cz = X * sy - Y * sx;
+      const double ex = X + sx, ey = Y + sy, ez = Z + sz;
+      const double f = seg_f_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
+      ax += f * cx;
+      ay += f * cy;
+      az += f * cz;
+    }
+    return;
+  }
+  double gx = 0., gy = 0., gz = 0.;
+#pragma unroll
+  for (int k = 0; k < PX; k++) gx = fma(fx[k], rx[k], gx);
+#pragma unroll
+  for (int k = 0; k < PY; k++) gy = fma(fy[k], ry[k], gy);
+#pragma unroll
+  for (int k = 0; k < PZ; k++) gz = fma(fz[k], rz[k], gz);
+  ax += gy * sz - gz * sy;
+  ay += gz * sx - gx * sz;
+  az += gx * sy - gy * sx;
+}
+
+template <int BC>
+__global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const int *__restrict__ act,
                                                     const double *__restrict__ x,
                                                     const int *__restrict__ beh,
                                                     const double *__restrict__ src, int chunk_len,
                                                     double L, double *part, int *status,
                                                     int stage_fail) {
-  constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
+  constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
   __shared__ __align__(128) double tiles[2][DTILE * 8];
   __shared__ __align__(8) unsigned long long bars[2];
-  int q = blockIdx.x * DTILE + threadIdx.x;
-  bool live = q < na;
-  int i = live ? act[q] : 0;
-  double xi0 = live ? x[3 * i] : 0., xi1 = live ? x[3 * i + 1] : 0., xi2 = live ? x[3 * i + 2] : 0.;
-  int bi = live ? beh[i] : -1, ii = i + 1;
-  double a0x = 0., a0y = 0., a0z = 0., a1x = 0., a1y = 0., a1z = 0.;
-  int j0 = blockIdx.y * chunk_len, j1 = min(na, j0 + chunk_len);
+  const int q = blockIdx.x * DTILE + threadIdx.x;
+  const bool live = q < na;
+  const int i = live ? act[q] : 0;
+  const double xi0 = live ? x[3 * i] : 0., xi1 = live ? x[3 * i + 1] : 0.,
+               xi2 = live ? x[3 * i + 2] : 0.;
+  const int bi = live ? beh[i] : -1, ii = i + 1;
+  double ax = 0., ay = 0., az = 0.;
+  const int j0 = blockIdx.y * chunk_len, j1 = min(na, j0 + chunk_len);
   const TilePipe pipe = make_pipe(src, j0, j1, tiles, bars, stage_fail);
   pipe.begin();
   for (int t = 0; t < pipe.ntile; t++) {
@@ -353,26 +443,35 @@ __global__ void __launch_bounds__(DTILE) k_direct64(int na, const int *__restric
     }
     const int m = min(DTILE, j1 - (j0 + t * DTILE));
     const double *tile = tiles[t & 1];
+#pragma unroll 1
     for (int k = 0; k < m; k++) {
       const double *s = tile + 8 * k;
-      int jj = (int)s[7];
-      double dx = s[0] - xi0, dy = s[1] - xi1, dz = s[2] - xi2;
-      if (jj != ii && jj != bi) pair64(dx, dy, dz, s[3], s[4], s[5], s[6], a0x, a0y, a0z);
-      if (NIMG > 0 && jj != bi) {
+      const int jj = (int)s[7];
+      const double dx = s[0] - xi0, dy = s[1] - xi1, dz = s[2] - xi2, c = s[6];
+      double rx[PX], ry[PY], rz[PZ], px[PX], py[PY], pz[PZ];
+      axis_shifts<PX>(dx, L, rx);
+      axis_shifts<PY>(dy, L, ry);
+      axis_shifts<PZ>(dz, L, rz);
 #pragma unroll
-        for (int im = 0; im < NIMG; im++) {
-          int ma, mb, mc;
-          img_mul<BC>(im, ma, mb, mc);
-          pair64(shifted(dx, ma, L), shifted(dy, mb, L), shifted(dz, mc, L), s[3], s[4], s[5],
-                 s[6], a1x, a1y, a1z);
-        }
-      }
+      for (int e = 0; e < PX; e++) px[e] = rx[e] * rx[e];
+#pragma unroll
+      for (int e = 0; e < PY; e++) py[e] = ry[e] * ry[e];
+#pragma unroll
+      for (int e = 0; e < PZ; e++) pz[e] = rz[e] * rz[e];
+      // the warp takes the cancellation-free form together when all its targets
+      // may; the margin covers the rounding of both sides
+      const double m1 = least<PX>(px) + least<PY>(py) + least<PZ>(pz);
+      const bool skip = !live || jj == bi;  // src/timestep.f90:471, 496
+      const bool fast = __all_sync(0xffffffffu, skip || m1 > 1.0001 * c);
+      if (skip) continue;
+      source64<BC>(dx, dy, dz, s[3], s[4], s[5], c, L, fast, jj == ii, rx, px, ry, py, rz, pz, ax,
+                   ay, az);
     }
     pipe.release();
   }
   if (live) {
-    double *o = part + ((size_t)blockIdx.y * na + q) * 6;
-    o[0] = a0x; o[1] = a0y; o[2] = a0z; o[3] = a1x; o[4] = a1y; o[5] = a1z;
+    double *o = part + ((size_t)blockIdx.y * na + q) * 3;
+    o[0] = ax; o[1] = ay; o[2] = az;
   }
 }
 
@@ -588,6 +687,7 @@ static void launch_direct32(dim3 grid, cudaStream_t s, int na, const int *act, c
                                            stage_fail);
 }
 
+// Mixed kernel's partial sums (main image, other images: 6 values):
 // u_bs = s0 + s1, u = (u_li + s0) + s1, in fixed chunk order.
 __global__ void k_direct_reduce(int na, int nchunk, const int *__restrict__ act,
                                 const double *__restrict__ part, double scale,
@@ -605,6 +705,56 @@ __global__ void k_direct_reduce(int na, int nchunk, const int *__restrict__ act,
     u_bs[3 * i + c] = b0 + b1;
     u[3 * i + c] = (u_li[3 * i + c] + b0) + b1;
   }
+}
+
+// FP64 kernel's partial sums (3 values, main image and images together), one
+// thread per component: u_bs and, where u is given, u = u_li + u_bs.
+__global__ void k_direct_reduce64(int na, int nchunk, const int *__restrict__ act,
+                                  const double *__restrict__ part, double scale,
+                                  const double *__restrict__ u_li, double *u, double *u_bs) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * na) return;
+  const size_t stride = 3 * (size_t)na;
+  double s = 0.;
+#pragma unroll 8
+  for (int k = 0; k < nchunk; k++) s += part[k * stride + t];
+  const int q = t / 3, o = 3 * act[q] + (t - 3 * q);
+  s *= scale;
+  u_bs[o] = s;
+  if (u) u[o] = u_li[o] + s;
+}
+
+// How the direct sum is split: bx tiles of DTILE targets x nchunk chunks of
+// chunk_len sources, with `width` partial values per target and chunk.
+struct DirectPlan {
+  int bx, nchunk, chunk_len, width;
+};
+
+// cap: partial values that fit (per target), 0 = no limit.
+static DirectPlan direct_plan(int na, int sm_count, int bc, bool mixed, int cap) {
+  DirectPlan d;
+  d.bx = nblk(na, DTILE);
+  if (mixed) {
+    // enough chunks to fill ~4 blocks per SM, each chunk at least 4 tiles
+    d.width = 6;
+    int want = (4 * sm_count + d.bx - 1) / d.bx;
+    int maxch = max(1, na / (4 * DTILE));
+    int nchunk = max(1, min(want, maxch));
+    if (cap) nchunk = min(nchunk, cap / 6);
+    d.chunk_len = ((nblk(na, nchunk) + DTILE - 1) / DTILE) * DTILE;
+  } else {
+    // eight blocks per resident slot (D64_BLOCKS per SM), so that the last wave
+    // leaves little of the chip idle, as far as a chunk keeps enough pairs
+    // (sources x images) to outweigh a block's start
+    d.width = 3;
+    const int want = nblk(8L * D64_BLOCKS * sm_count, d.bx);
+    const int least_len = bc == QV_BC_OPEN ? 128 : bc == QV_BC_OPENXY ? 64 : 32;
+    int len = max(nblk(na, want), least_len);
+    if (cap) len = max(len, nblk(na, cap / 3));
+    d.chunk_len = ((len + 31) / 32) * 32;
+  }
+  d.nchunk = nblk(na, d.chunk_len);
+  return d;
 }
 
 // Source packs of the compacted active list (c->act, c->n_act).
@@ -625,21 +775,16 @@ int qv_launch_direct(qv_ctx *c) {
   QV_LAUNCH_CHECK(c);
   QV_COUNT(c, 1);
   bool mixed = c->p.precision == QV_PREC_MIXED;
-  int bx = nblk(na, DTILE);
-  // enough chunks to fill ~4 blocks per SM, each chunk at least 4 tiles
-  int want = (4 * c->sm_count + bx - 1) / bx;
-  int maxch = max(1, na / (4 * DTILE));
-  int nchunk = max(1, min(want, maxch));
-  int chunk_len = ((nblk(na, nchunk) + DTILE - 1) / DTILE) * DTILE;
-  nchunk = nblk(na, chunk_len);
-  size_t need = sizeof(double) * 6 * (size_t)na * nchunk;
+  const DirectPlan d = direct_plan(na, c->sm_count, c->p.boundary, mixed, 0);
+  const int nchunk = d.nchunk, chunk_len = d.chunk_len;
+  size_t need = sizeof(double) * d.width * (size_t)na * nchunk;
   if (need > c->dpart_bytes) {
     int rc = qv_grow(c, (void **)&c->dpart, need);
     if (rc) return rc;
     c->dpart_bytes = need;
   }
   double *part = c->dpart;
-  dim3 grid(bx, nchunk);
+  dim3 grid(d.bx, nchunk);
   double L = c->p.box_size;
   switch (c->p.boundary) {
 #define QV_DIRECT_CASE(BCV)                                                                   \
@@ -662,9 +807,13 @@ int qv_launch_direct(qv_ctx *c) {
       return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d not supported", c->p.boundary);
   }
   QV_LAUNCH_CHECK(c);
-  double scale = mixed ? c->p.quant_circ / (4. * QV_PI) : c->p.quant_circ / (2. * QV_PI);
-  k_direct_reduce<<<tb, 256, 0, c->stream>>>(na, nchunk, c->act, part, scale, c->u_li, c->u,
-                                             c->u_bs);
+  const double scale = c->p.quant_circ / (4. * QV_PI);
+  if (mixed)
+    k_direct_reduce<<<tb, 256, 0, c->stream>>>(na, nchunk, c->act, part, scale, c->u_li, c->u,
+                                               c->u_bs);
+  else
+    k_direct_reduce64<<<nblk(3L * na, 128), 128, 0, c->stream>>>(na, nchunk, c->act, part, scale,
+                                                                 c->u_li, c->u, c->u_bs);
   QV_LAUNCH_CHECK(c);
   QV_COUNT(c, 2);
   return QV_OK;
@@ -707,13 +856,9 @@ int qv_direct_scratch(cudaStream_t s, const qv_params *p, int sm_count, int n, c
   int *stat = blk + nb + 1;
   if (cudaMemsetAsync(stat, 0, sizeof(int), s) != cudaSuccess) return QV_ERR_CUDA;
   k_pack_sources<<<tb, 256, 0, s>>>(na, act, x, gi, src64, src32);
-  int bx = nblk(na, DTILE);
-  int want = (4 * sm_count + bx - 1) / bx;
-  int maxch = max(1, na / (4 * DTILE));
-  int nchunk = max(1, min(min(want, maxch), max_chunks));
-  int chunk_len = ((nblk(na, nchunk) + DTILE - 1) / DTILE) * DTILE;
-  nchunk = nblk(na, chunk_len);
-  dim3 grid(bx, nchunk);
+  const DirectPlan d = direct_plan(na, sm_count, p->boundary, mixed, 6 * max_chunks);
+  const int nchunk = d.nchunk, chunk_len = d.chunk_len;
+  dim3 grid(d.bx, nchunk);
   double L = p->box_size;
   switch (p->boundary) {
 #define QV_DIRECT_SCRATCH_CASE(BCV)                                                      \
@@ -733,8 +878,12 @@ int qv_direct_scratch(cudaStream_t s, const qv_params *p, int sm_count, int n, c
     default:
       return QV_ERR_UNSUPPORTED;
   }
-  double scale = mixed ? p->quant_circ / (4. * QV_PI) : p->quant_circ / (2. * QV_PI);
-  k_direct_reduce_bs<<<tb, 256, 0, s>>>(na, nchunk, act, part, scale, u_bs);
+  const double scale = p->quant_circ / (4. * QV_PI);
+  if (mixed)
+    k_direct_reduce_bs<<<tb, 256, 0, s>>>(na, nchunk, act, part, scale, u_bs);
+  else
+    k_direct_reduce64<<<nblk(3L * na, 128), 128, 0, s>>>(na, nchunk, act, part, scale, nullptr,
+                                                         nullptr, u_bs);
   if (cudaGetLastError() != cudaSuccess) return QV_ERR_CUDA;
   int st = 0;
   if (cudaMemcpyAsync(&st, stat, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
