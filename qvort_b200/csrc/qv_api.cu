@@ -142,7 +142,7 @@ extern "C" int qv_destroy(qv_ctx *c) {
   if (c->d_nact) cudaFree(c->d_nact);
   {
     void *adj[] = {c->adj_xb, c->adj_gib, c->adj_gbb, c->adj_giib, c->adj_gbbb, c->adj_nb,
-                   c->line_flags, c->line_st, c->line_rec};
+                   c->field_buf, c->line_flags, c->line_st, c->line_rec};
     for (void *q : adj)
       if (q) cudaFree(q);
   }

@@ -323,107 +323,12 @@ __device__ __forceinline__ TilePipe make_pipe(const void *src, int j0, int j1, c
 // ms now = 6.2e11 pairs/s, 90 % of the FP64 rate (148 SM x 64 lanes x 1.965
 // GHz) at that operation count.
 template <int BC>
-struct Img {
-  static constexpr int PX = BC == QV_BC_PERIODIC ? 3 : 1;
-  static constexpr int PY = (BC == QV_BC_PERIODIC || BC == QV_BC_OPENX) ? 3 : 1;
-  static constexpr int PZ = BC == QV_BC_OPEN ? 1 : 3;
-};
-
-template <int P>
-__device__ __forceinline__ void axis_shifts(double d, double L, double *r) {
-  if (P == 3) {
-    r[0] = d - L;
-    r[1] = d;
-    r[2] = d + L;
-  } else {
-    r[0] = d;
-  }
-}
-template <int P>
-__device__ __forceinline__ double least(const double *v) {
-  return P == 3 ? fmin(fmin(v[0], v[1]), v[2]) : v[0];
-}
-
-// Adds the terms of one source (main image unless skip_main, and the images)
-// to (ax, ay, az).  dx, dy, dz = x_j - x_i, c = |s|^2.  fast: every image has
-// |R1| > |s|, hence R1.R2 >= |R1| (|R1| - |s|) > 0 (seg_f_pos).
-template <int BC>
-__device__ __forceinline__ void source64(double dx, double dy, double dz, double sx, double sy,
-                                         double sz, double c, double L, bool fast, bool skip_main,
-                                         const double *rx, const double *px, const double *ry,
-                                         const double *py, const double *rz, const double *pz,
-                                         double &ax, double &ay, double &az) {
-  constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
-  double fx[PX], fy[PY], fz[PZ];  // sum of f at each shift of an axis
-#pragma unroll
-  for (int k = 0; k < PX; k++) fx[k] = 0.;
-#pragma unroll
-  for (int k = 0; k < PY; k++) fy[k] = 0.;
-#pragma unroll
-  for (int k = 0; k < PZ; k++) fz[k] = 0.;
-  if (fast) {
-    // per-axis parts of A = |R1|^2 (p), d = R1.R2 = A + R1.s (g), B = |R2|^2 =
-    // d + R1.s + |s|^2 (t)
-    double gx[PX], tx[PX], gy[PY], ty[PY], gz[PZ], tz[PZ];
-#pragma unroll
-    for (int k = 0; k < PX; k++) { gx[k] = fma(rx[k], sx, px[k]); tx[k] = fma(rx[k], sx, gx[k] + c); }
-#pragma unroll
-    for (int k = 0; k < PY; k++) { gy[k] = fma(ry[k], sy, py[k]); ty[k] = fma(ry[k], sy, gy[k]); }
-#pragma unroll
-    for (int k = 0; k < PZ; k++) { gz[k] = fma(rz[k], sz, pz[k]); tz[k] = fma(rz[k], sz, gz[k]); }
-#pragma unroll
-    for (int a = 0; a < PX; a++) {
-#pragma unroll
-      for (int b = 0; b < PY; b++) {
-        const double pxy = px[a] + py[b], gxy = gx[a] + gy[b], txy = tx[a] + ty[b];
-        double row = 0.;
-#pragma unroll
-        for (int k = 0; k < PZ; k++) {
-          const double f = seg_f_pos(pxy + pz[k], txy + tz[k], gxy + gz[k]);
-          row += f;
-          fz[k] += f;
-        }
-        fx[a] += row;
-        fy[b] += row;
-      }
-    }
-  } else {
-#pragma unroll 1
-    for (int m = 0; m < PX * PY * PZ; m++) {
-      const int a = m / (PY * PZ), b = (m / PZ) % PY, k = m % PZ;
-      if (skip_main && m == PX * PY * PZ / 2) continue;  // the middle one is unshifted
-      const double X = PX == 3 ? dx + (a - 1) * L : dx, Y = PY == 3 ? dy + (b - 1) * L : dy,
-                   Z = PZ == 3 ? dz + (k - 1) * L : dz;
-      const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
-      const double cx = Y * sz - Z * sy, cy = Z * sx - X * sz, cz = X * sy - Y * sx;
-      const double ex = X + sx, ey = Y + sy, ez = Z + sz;
-      const double f = seg_f_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
-      ax += f * cx;
-      ay += f * cy;
-      az += f * cz;
-    }
-    return;
-  }
-  double gx = 0., gy = 0., gz = 0.;
-#pragma unroll
-  for (int k = 0; k < PX; k++) gx = fma(fx[k], rx[k], gx);
-#pragma unroll
-  for (int k = 0; k < PY; k++) gy = fma(fy[k], ry[k], gy);
-#pragma unroll
-  for (int k = 0; k < PZ; k++) gz = fma(fz[k], rz[k], gz);
-  ax += gy * sz - gz * sy;
-  ay += gz * sx - gx * sz;
-  az += gx * sy - gy * sx;
-}
-
-template <int BC>
 __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const int *__restrict__ act,
                                                     const double *__restrict__ x,
                                                     const int *__restrict__ beh,
                                                     const double *__restrict__ src, int chunk_len,
                                                     double L, double *part, int *status,
                                                     int stage_fail) {
-  constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
   __shared__ __align__(128) double tiles[2][DTILE * 8];
   __shared__ __align__(8) unsigned long long bars[2];
   const int q = blockIdx.x * DTILE + threadIdx.x;
@@ -447,25 +352,13 @@ __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const in
     for (int k = 0; k < m; k++) {
       const double *s = tile + 8 * k;
       const int jj = (int)s[7];
-      const double dx = s[0] - xi0, dy = s[1] - xi1, dz = s[2] - xi2, c = s[6];
-      double rx[PX], ry[PY], rz[PZ], px[PX], py[PY], pz[PZ];
-      axis_shifts<PX>(dx, L, rx);
-      axis_shifts<PY>(dy, L, ry);
-      axis_shifts<PZ>(dz, L, rz);
-#pragma unroll
-      for (int e = 0; e < PX; e++) px[e] = rx[e] * rx[e];
-#pragma unroll
-      for (int e = 0; e < PY; e++) py[e] = ry[e] * ry[e];
-#pragma unroll
-      for (int e = 0; e < PZ; e++) pz[e] = rz[e] * rz[e];
-      // the warp takes the cancellation-free form together when all its targets
-      // may; the margin covers the rounding of both sides
-      const double m1 = least<PX>(px) + least<PY>(py) + least<PZ>(pz);
+      const double c = s[6];
+      const Seg64<BC> e(s[0] - xi0, s[1] - xi1, s[2] - xi2, L);
       const bool skip = !live || jj == bi;  // src/timestep.f90:471, 496
-      const bool fast = __all_sync(0xffffffffu, skip || m1 > 1.0001 * c);
+      // one form for the whole warp
+      const bool fast = __all_sync(0xffffffffu, skip || e.far(c));
       if (skip) continue;
-      source64<BC>(dx, dy, dz, s[3], s[4], s[5], c, L, fast, jj == ii, rx, px, ry, py, rz, pz, ax,
-                   ay, az);
+      e.velocity(s[3], s[4], s[5], c, L, fast, jj == ii, ax, ay, az);
     }
     pipe.release();
   }

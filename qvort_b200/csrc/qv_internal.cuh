@@ -183,6 +183,8 @@ struct qv_ctx {
          *adj_gbbb = nullptr, *adj_nb = nullptr;
   int adj_n = 0;
   size_t adj_nb_bytes = 0;
+  double *field_buf = nullptr;  // field points: points, results, per-chunk partial sums
+  size_t field_bytes = 0;
   double *src64 = nullptr;  // direct-sum source pack (FP64)
   float *src32 = nullptr;   // direct-sum source pack (FP32 hi/lo)
   unsigned long long *evals = nullptr;  // device eval counter
