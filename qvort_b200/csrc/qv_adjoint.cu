@@ -4,8 +4,8 @@
 // 180-309) through every piece of it:
 //   * the local LIA term (forward-mode dual numbers over its 9- or 15-value
 //     ghost stencil, the same templated formula as the velocity),
-//   * the direct sum (hand-derived gradients of the straight-segment term,
-//     a target pass and a source pass, no atomics),
+//   * the direct sum (hand-derived gradients of the straight-segment term, one
+//     pass over the pairs for both ends, no atomics),
 //   * or the Barnes-Hut walk with the topology of the last build frozen
 //     (hand-derived leaf and monopole+dipole gradients; the gradients that
 //     belong to a source cell are reduced over the warp and added to a per-node
@@ -116,121 +116,124 @@ __global__ void k_lia_vjp(int n, const double *__restrict__ x, const int *__rest
 }
 
 // ------------------------------------------------------------ direct sum
-__device__ __forceinline__ double shiftv(double v, int m, double L) {
-  return m == 0 ? v : (m > 0 ? v + L : v - L);
+// One pass over all (source, target) pairs gives both ends' gradients: a thread
+// holds one source and sums its own (dL/dx_j at fixed s, dL/ds) over a chunk of
+// targets, while each target's gradient -- minus the sum over sources -- is
+// reduced over the warp (12 shuffles a target against 27 images x ~55 FP64
+// operations a lane) and over the block's warps in shared memory.  Partial
+// sums per (source block, target) and per (target chunk, source) are added in
+// a fixed order by k_dvjp_reduce, so results are deterministic, with no
+// atomics.  A two-pass split (a thread per target, then a thread per source)
+// evaluates every pair twice.  Bound: FP64 issue.  6,400 points, 27 images:
+// velocity and gradient together took 333 ms with two passes, divisions in every
+// image term and 50 blocks; 8.4 ms now, about 2 of them the velocity.
+#define VT 128  // sources per block
+#define VG 32   // targets per shared-memory tile
+#define QV_DVJP_PART ((size_t)256 << 20)  // bytes of per-target partial sums per launch
+
+// Sum of (v0, v1, v2) over the warp: lanes 0, 8 and 16 return the three sums.
+__device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
+  const bool hi = lane & 16, md = lane & 8;
+  double a = hi ? v2 : v0, b = hi ? 0. : v1;
+  a += __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 16);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v1 : 0., 16);
+  double r = md ? b : a;
+  r += __shfl_xor_sync(0xffffffffu, md ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
 }
 
-#define VT 128
-// Target pass: x_bar_i += -sum_j (grad_R1 + grad_R2) over sources j and images,
-// with the skip rules of src/timestep.f90:471, 496.
+// Targets t_lo..t_hi (positions in act); tpart: (source blocks) x (t_hi - t_lo)
+// x 3, spart: (target chunks) x na x 6.
 template <int BC>
-__global__ void __launch_bounds__(VT) k_dvjp_tgt(int na, const int *__restrict__ act,
-                                                 const double *__restrict__ x,
-                                                 const double *__restrict__ gi,
-                                                 const int *__restrict__ beh,
-                                                 const double *__restrict__ ubar, double gfac,
-                                                 double L, double *xb) {
-  constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
-  __shared__ double sx[VT][3], sg[VT][3];
-  __shared__ int sj[VT];
-  int q = blockIdx.x * VT + threadIdx.x;
-  bool live = q < na;
-  int i = live ? act[q] : 0;
-  double xi[3] = {0., 0., 0.}, g[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
-  int bi = -1, ii = i + 1;
+__global__ void __launch_bounds__(VT, 2) k_dvjp(int na, const int *__restrict__ act,
+                                                const double *__restrict__ x,
+                                                const double *__restrict__ gi,
+                                                const int *__restrict__ beh,
+                                                const double *__restrict__ ubar, double gfac,
+                                                double L, int t_lo, int t_hi, int chunk_len,
+                                                double *tpart, double *spart) {
+  __shared__ double tx[VG][3], tg[VG][3], red[VT / 32][VG][3];
+  __shared__ int tb[VG], ti[VG];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int q = blockIdx.x * VT + threadIdx.x;
+  const bool live = q < na;
+  const int j = live ? act[q] : 0, jj = j + 1;
+  double xj[3] = {0., 0., 0.}, s[3] = {0., 0., 0.}, dx[3] = {0., 0., 0.}, dg[3] = {0., 0., 0.};
+  if (live)
+#pragma unroll
+    for (int c = 0; c < 3; c++) { xj[c] = x[3 * j + c]; s[c] = gi[3 * j + c] - xj[c]; }
+  const double c2 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+  const int t0 = t_lo + blockIdx.y * chunk_len, t1 = min(t_hi, t0 + chunk_len);
+  for (int t = t0; t < t1; t += VG) {
+    const int m = min(VG, t1 - t);
+    __syncthreads();  // the last tile's sums are out
+    for (int e = threadIdx.x; e < 3 * m; e += VT) {
+      const int k = e / 3, c = e - 3 * k, i = act[t + k];
+      tx[k][c] = x[3 * i + c];
+      tg[k][c] = gfac * ubar[3 * i + c];
+      if (c == 0) {
+        tb[k] = beh[i];
+        ti[k] = i + 1;
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < m; k++) {
+      const Seg64<BC> e(xj[0] - tx[k][0], xj[1] - tx[k][1], xj[2] - tx[k][2], s[0], s[1], s[2], c2,
+                        L);
+      // src/timestep.f90:471, 496
+      const bool own = jj == ti[k], skip = !live || jj == tb[k] || (own && e.NI == 1);
+      const bool fast = __all_sync(0xffffffffu, skip || (e.far(own, L) && !e.on_line()));
+      double dR[3] = {0., 0., 0.}, dS[3];
+      if (!skip) {
+        e.gradient(tg[k][0], tg[k][1], tg[k][2], L, fast, own, dR, dS);
+#pragma unroll
+        for (int c = 0; c < 3; c++) { dx[c] += dR[c] - dS[c]; dg[c] += dS[c]; }
+      }
+      __syncwarp();
+      const double r = warp_sum3(dR[0], dR[1], dR[2], lane);
+      if ((lane & 7) == 0 && lane < 24) red[wid][k][lane >> 3] = r;
+    }
+    __syncthreads();
+    double *o = tpart + ((size_t)blockIdx.x * (t_hi - t_lo) + (t - t_lo)) * 3;
+    for (int e = threadIdx.x; e < 3 * m; e += VT) {
+      double v = 0.;
+#pragma unroll
+      for (int w = 0; w < VT / 32; w++) v += red[w][e / 3][e % 3];
+      o[e] = v;
+    }
+  }
   if (live) {
-    for (int c = 0; c < 3; c++) { xi[c] = x[3 * i + c]; g[c] = gfac * ubar[3 * i + c]; }
-    bi = beh[i];
+    double *o = spart + ((size_t)blockIdx.y * na + q) * 6;
+#pragma unroll
+    for (int c = 0; c < 3; c++) { o[c] = dx[c]; o[3 + c] = dg[c]; }
   }
-  for (int t0 = 0; t0 < na; t0 += VT) {
-    __syncthreads();
-    int k = t0 + threadIdx.x;
-    if (k < na) {
-      int j = act[k];
-      for (int c = 0; c < 3; c++) { sx[threadIdx.x][c] = x[3 * j + c]; sg[threadIdx.x][c] = gi[3 * j + c]; }
-      sj[threadIdx.x] = j + 1;
-    }
-    __syncthreads();
-    if (!live) continue;
-    int m = min(VT, na - t0);
-    for (int kk = 0; kk < m; kk++) {
-      int jj = sj[kk];
-      if (jj == bi) continue;
-      for (int im = -1; im < NIMG; im++) {
-        if (im < 0 && jj == ii) continue;
-        int ma = 0, mb = 0, mc = 0;
-        if (im >= 0) qv_img_shift(BC, im, &ma, &mb, &mc);
-        double R1[3] = {shiftv(sx[kk][0], ma, L) - xi[0], shiftv(sx[kk][1], mb, L) - xi[1],
-                        shiftv(sx[kk][2], mc, L) - xi[2]};
-        double R2[3] = {shiftv(sg[kk][0], ma, L) - xi[0], shiftv(sg[kk][1], mb, L) - xi[1],
-                        shiftv(sg[kk][2], mc, L) - xi[2]};
-        double s[3] = {sg[kk][0] - sx[kk][0], sg[kk][1] - sx[kk][1], sg[kk][2] - sx[kk][2]};
-        double cx = R1[1] * s[2] - R1[2] * s[1], cy = R1[2] * s[0] - R1[0] * s[2],
-               cz = R1[0] * s[1] - R1[1] * s[0];
-        if (cx * cx + cy * cy + cz * cz == 0.) continue;  // 4ac - b^2 == 0 (skipped forward)
-        double a1[3], a2[3];
-        seg_grad(R1, R2, g, a1, a2);
-        for (int c = 0; c < 3; c++) acc[c] -= a1[c] + a2[c];
-      }
-    }
-  }
-  if (live)
-    for (int c = 0; c < 3; c++) xb[3 * i + c] += acc[c];
 }
 
-// Source pass: x_bar_j += sum_i grad_R1, ghosti_bar_j += sum_i grad_R2.
-template <int BC>
-__global__ void __launch_bounds__(VT) k_dvjp_src(int na, const int *__restrict__ act,
-                                                 const double *__restrict__ x,
-                                                 const double *__restrict__ gi,
-                                                 const int *__restrict__ beh,
-                                                 const double *__restrict__ ubar, double gfac,
-                                                 double L, double *xb, double *gib) {
-  constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
-  __shared__ double tx[VT][3], tg[VT][3];
-  __shared__ int tb[VT], ti[VT];
-  int q = blockIdx.x * VT + threadIdx.x;
-  bool live = q < na;
-  int j = live ? act[q] : 0;
-  double xj[3] = {0., 0., 0.}, gj[3] = {0., 0., 0.}, s[3], a1s[3] = {0., 0., 0.},
-         a2s[3] = {0., 0., 0.};
-  int jj = j + 1;
-  if (live)
-    for (int c = 0; c < 3; c++) { xj[c] = x[3 * j + c]; gj[c] = gi[3 * j + c]; }
-  for (int c = 0; c < 3; c++) s[c] = gj[c] - xj[c];
-  for (int t0 = 0; t0 < na; t0 += VT) {
-    __syncthreads();
-    int k = t0 + threadIdx.x;
-    if (k < na) {
-      int i = act[k];
-      for (int c = 0; c < 3; c++) { tx[threadIdx.x][c] = x[3 * i + c]; tg[threadIdx.x][c] = gfac * ubar[3 * i + c]; }
-      tb[threadIdx.x] = beh[i];
-      ti[threadIdx.x] = i + 1;
-    }
-    __syncthreads();
-    if (!live) continue;
-    int m = min(VT, na - t0);
-    for (int kk = 0; kk < m; kk++) {
-      if (jj == tb[kk]) continue;
-      for (int im = -1; im < NIMG; im++) {
-        if (im < 0 && jj == ti[kk]) continue;
-        int ma = 0, mb = 0, mc = 0;
-        if (im >= 0) qv_img_shift(BC, im, &ma, &mb, &mc);
-        double R1[3] = {shiftv(xj[0], ma, L) - tx[kk][0], shiftv(xj[1], mb, L) - tx[kk][1],
-                        shiftv(xj[2], mc, L) - tx[kk][2]};
-        double R2[3] = {shiftv(gj[0], ma, L) - tx[kk][0], shiftv(gj[1], mb, L) - tx[kk][1],
-                        shiftv(gj[2], mc, L) - tx[kk][2]};
-        double cx = R1[1] * s[2] - R1[2] * s[1], cy = R1[2] * s[0] - R1[0] * s[2],
-               cz = R1[0] * s[1] - R1[1] * s[0];
-        if (cx * cx + cy * cy + cz * cz == 0.) continue;
-        double a1[3], a2[3];
-        seg_grad(R1, R2, tg[kk], a1, a2);
-        for (int c = 0; c < 3; c++) { a1s[c] += a1[c]; a2s[c] += a2[c]; }
-      }
-    }
+// Adds a slab's partial sums to the point adjoints: one thread per component.
+__global__ void k_dvjp_reduce(int na, const int *__restrict__ act, int t_lo, int t_hi, int nsb,
+                              int nchunk, const double *__restrict__ tpart,
+                              const double *__restrict__ spart, double *xb, double *gib) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 3 * na) return;
+  const int q = e / 3, c = e - 3 * q, o = 3 * act[q] + c;
+  double sx = 0., sg = 0., st = 0.;
+#pragma unroll 8
+  for (int k = 0; k < nchunk; k++) {
+    const double *p = spart + ((size_t)k * na + q) * 6 + c;
+    sx += p[0];
+    sg += p[3];
   }
-  if (live)
-    for (int c = 0; c < 3; c++) { xb[3 * j + c] += a1s[c]; gib[3 * j + c] += a2s[c]; }
+  if (q >= t_lo && q < t_hi) {
+    const size_t stride = 3 * (size_t)(t_hi - t_lo);
+    const double *p = tpart + (e - 3 * t_lo);
+#pragma unroll 8
+    for (int k = 0; k < nsb; k++) st += p[k * stride];
+  }
+  xb[o] += sx - st;
+  gib[o] += sg;
 }
 
 // ------------------------------------------------------------ tree walk
@@ -608,11 +611,11 @@ __global__ void __launch_bounds__(FW * 32) k_field(int m, const double *__restri
     const double2 *s = reinterpret_cast<const double2 *>(src + 8 * (size_t)(live ? j : j0));
     const double2 s0 = s[0], s1 = s[1], s2 = s[2];
     const double sx = s1.y, sy = s2.x, sz = s2.y, c = s[3].x;
-    const Seg64<BC> e(s0.x - X, s0.y - Y, s1.x - Z, L);
-    const bool fast = __all_sync(0xffffffffu, !live || e.far(c));
+    const Seg64<BC> e(s0.x - X, s0.y - Y, s1.x - Z, sx, sy, sz, c, L);
+    const bool fast = __all_sync(0xffffffffu, !live || e.far(false, L));
     if (!live) continue;
-    constexpr int NI = Img<BC>::PX * Img<BC>::PY * Img<BC>::PZ;
-    if (!GI) e.velocity(sx, sy, sz, c, L, fast, false, v[0], v[1], v[2]);
+    constexpr int NI = Seg64<BC>::NI;
+    if (!GI) e.velocity(L, fast, false, v[0], v[1], v[2]);
 #pragma unroll 1
     for (int im = GI ? 0 : NI / 2; im < (GI ? NI : NI / 2 + 1); im++) {
       double rx, ry, rz;
@@ -780,25 +783,47 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
     if ((rc = qv_compact_active(c))) return rc;
     int na = c->n_act;
     if (na > 0) {
-      int nb = nblk(na, VT);
-      switch (p.boundary) {
+      // Slabs of targets bound the partial sums: source blocks x targets x 24
+      // bytes is 2 GB at 100,000 points, so above QV_DVJP_PART bytes the
+      // targets are taken in several launches.
+      const int nsb = nblk(na, VT);
+      const size_t row = sizeof(double) * 3 * (size_t)nsb;
+      const int slab = (int)std::min<size_t>(na, std::max<size_t>(VG, QV_DVJP_PART / row / VG * VG));
+      // eight blocks per resident slot (2 per SM), each with enough pairs
+      // (targets x images) to outweigh its start and its partial sums
+      const int want = nblk(16L * c->sm_count, nsb);
+      const int least = p.boundary == QV_BC_PERIODIC ? 8 : p.boundary == QV_BC_OPENX ? 16 : VG;
+      const int chunk_len = nblk(nblk(slab, want), least) * least, nchunk = nblk(slab, chunk_len);
+      const size_t tbytes = row * slab, sbytes = sizeof(double) * 6 * (size_t)na * nchunk;
+      if (tbytes + sbytes > c->dpart_bytes) {
+        c->dpart_bytes = 0;  // the old buffer goes first
+        if ((rc = qv_grow(c, (void **)&c->dpart, tbytes + sbytes))) return rc;
+        c->dpart_bytes = tbytes + sbytes;
+      }
+      double *tpart = c->dpart, *spart = c->dpart + tbytes / sizeof(double);
+      for (int t_lo = 0; t_lo < na; t_lo += slab) {
+        const int t_hi = std::min(na, t_lo + slab), nch = nblk(t_hi - t_lo, chunk_len);
+        const dim3 grid(nsb, nch);
+        switch (p.boundary) {
 #define QV_DVJP(BCV)                                                                              \
   case BCV:                                                                                       \
-    k_dvjp_tgt<BCV><<<nb, VT, 0, c->stream>>>(na, c->act, c->x, c->gi, c->behind, ubar, gfac,     \
-                                              p.box_size, c->adj_xb);                             \
-    k_dvjp_src<BCV><<<nb, VT, 0, c->stream>>>(na, c->act, c->x, c->gi, c->behind, ubar, gfac,     \
-                                              p.box_size, c->adj_xb, c->adj_gib);                 \
+    k_dvjp<BCV><<<grid, VT, 0, c->stream>>>(na, c->act, c->x, c->gi, c->behind, ubar, gfac,       \
+                                            p.box_size, t_lo, t_hi, chunk_len, tpart, spart);     \
     break;
-        QV_DVJP(QV_BC_OPEN)
-        QV_DVJP(QV_BC_PERIODIC)
-        QV_DVJP(QV_BC_OPENX)
-        QV_DVJP(QV_BC_OPENXY)
+          QV_DVJP(QV_BC_OPEN)
+          QV_DVJP(QV_BC_PERIODIC)
+          QV_DVJP(QV_BC_OPENX)
+          QV_DVJP(QV_BC_OPENXY)
 #undef QV_DVJP
-        default:
-          return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", p.boundary);
+          default:
+            return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", p.boundary);
+        }
+        QV_LAUNCH_CHECK(c);
+        k_dvjp_reduce<<<nblk(3L * na, 128), 128, 0, c->stream>>>(
+            na, c->act, t_lo, t_hi, nsb, nch, tpart, spart, c->adj_xb, c->adj_gib);
+        QV_LAUNCH_CHECK(c);
+        QV_COUNT(c, 2);
       }
-      QV_LAUNCH_CHECK(c);
-      QV_COUNT(c, 2);
     }
   } else if (p.velocity == QV_VEL_TREE) {
     if (!c->tree.valid)

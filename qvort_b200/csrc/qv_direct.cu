@@ -310,18 +310,12 @@ __device__ __forceinline__ TilePipe make_pipe(const void *src, int j0, int j1, c
 }
 
 // ------------------------------------------------------------ FP64 kernel
-// One thread per target, each staged source summed against it in all images.
-// u = f (R1 x s) per image, and s is the same for all of them: the kernel sums
-// f and f R1 over the images and takes one cross product per source.  R1 takes,
-// per axis, one of three values (shift -L, 0, L), so |R1|^2, R1.s and |R2|^2 =
-// |R1|^2 + 2 R1.s + |s|^2 are sums of per-axis parts, and sum f R1 per axis is
-// the sum over the three shifts of (R1 component) x (sum of f at that shift).
-//
-// Bound: FP64 issue, about 27 operations a pair (two rsqrt_pos and one div_pos
-// are 14 of them).  24,700 points, 27 images: 70.3 ms with the reference's
-// formula pair by pair (library rsqrt and division, 1.3 waves of blocks), 26.4
-// ms now = 6.2e11 pairs/s, 90 % of the FP64 rate (148 SM x 64 lanes x 1.965
-// GHz) at that operation count.
+// One thread per target, each staged source summed against it in all images
+// (Seg64).  Bound: FP64 issue, about 26 operations a pair (two rsqrt_pos and
+// one div_pos are 14 of them).  24,700 points, 27 images: 70.3 ms with the
+// reference's formula pair by pair (library rsqrt and division, 1.3 waves of
+// blocks), 26.0 ms now = 6.3e11 pairs/s, 88 % of the FP64 rate (148 SM x 64
+// lanes x 1.965 GHz) at that operation count.
 template <int BC>
 __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const int *__restrict__ act,
                                                     const double *__restrict__ x,
@@ -352,13 +346,12 @@ __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const in
     for (int k = 0; k < m; k++) {
       const double *s = tile + 8 * k;
       const int jj = (int)s[7];
-      const double c = s[6];
-      const Seg64<BC> e(s[0] - xi0, s[1] - xi1, s[2] - xi2, L);
-      const bool skip = !live || jj == bi;  // src/timestep.f90:471, 496
+      const Seg64<BC> e(s[0] - xi0, s[1] - xi1, s[2] - xi2, s[3], s[4], s[5], s[6], L);
+      // src/timestep.f90:471, 496
+      const bool own = jj == ii, skip = !live || jj == bi || (own && e.NI == 1);
       // one form for the whole warp
-      const bool fast = __all_sync(0xffffffffu, skip || e.far(c));
-      if (skip) continue;
-      e.velocity(s[3], s[4], s[5], c, L, fast, jj == ii, ax, ay, az);
+      const bool fast = __all_sync(0xffffffffu, skip || e.far(own, L));
+      if (!skip) e.velocity(L, fast, own, ax, ay, az);
     }
     pipe.release();
   }

@@ -115,38 +115,56 @@ __device__ __forceinline__ double least(const double *v) {
   return P == 3 ? fmin(fmin(v[0], v[1]), v[2]) : v[0];
 }
 
-// One source segment against one target in every image: R1 = x_j + shift - x_i
-// and its square, per axis and shift.
+// One source segment against one target in every image.  Per axis and shift:
+// R1 = x_j + shift - x_i (r) and the parts of |R1|^2 (p) and R1.R2 (g); the sum
+// over the axes gives an image's value.
 template <int BC>
 struct Seg64 {
   static constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
-  double rx[PX], ry[PY], rz[PZ], px[PX], py[PY], pz[PZ];
-  __device__ __forceinline__ Seg64(double dx, double dy, double dz, double L) {
+  static constexpr int NI = PX * PY * PZ;
+  double sx, sy, sz, c;  // segment vector s and |s|^2
+  double rx[PX], ry[PY], rz[PZ], px[PX], py[PY], pz[PZ], gx[PX], gy[PY], gz[PZ];
+  __device__ __forceinline__ Seg64(double dx, double dy, double dz, double sx_, double sy_,
+                                   double sz_, double c_, double L)
+      : sx(sx_), sy(sy_), sz(sz_), c(c_) {
     axis_shifts<PX>(dx, L, rx);
     axis_shifts<PY>(dy, L, ry);
     axis_shifts<PZ>(dz, L, rz);
 #pragma unroll
-    for (int e = 0; e < PX; e++) px[e] = rx[e] * rx[e];
+    for (int e = 0; e < PX; e++) { px[e] = rx[e] * rx[e]; gx[e] = fma(rx[e], sx, px[e]); }
 #pragma unroll
-    for (int e = 0; e < PY; e++) py[e] = ry[e] * ry[e];
+    for (int e = 0; e < PY; e++) { py[e] = ry[e] * ry[e]; gy[e] = fma(ry[e], sy, py[e]); }
 #pragma unroll
-    for (int e = 0; e < PZ; e++) pz[e] = rz[e] * rz[e];
+    for (int e = 0; e < PZ; e++) { pz[e] = rz[e] * rz[e]; gz[e] = fma(rz[e], sz, pz[e]); }
   }
-  // Whether |R1| > |s| in every image, so that R1.R2 >= |R1| (|R1| - |s|) > 0
-  // (the _pos forms); the margin covers the rounding of both sides.
-  __device__ __forceinline__ bool far(double c) const {
-    return least<PX>(px) + least<PY>(py) + least<PZ>(pz) > 1.0001 * c;
+  // Whether R1.R2 > |s|^2 / 16 in every image that is summed: the _pos forms
+  // hold there, and |R2|^2 = R1.R2 + R1.s + |s|^2 keeps its digits (both ends
+  // lie well off the target).  Every point's own neighbours pass, so only
+  // points about to reconnect take the general form.  The least R1.R2 over
+  // the images is the sum of the axes' least parts.  skip_main (the point's
+  // own segment): the other images lie a box side away.
+  __device__ __forceinline__ bool far(bool skip_main, double L) const {
+    if (skip_main) return c < 0.25 * L * L;
+    return least<PX>(gx) + least<PY>(gy) + least<PZ>(gz) > 0.0625 * c;
+  }
+  // R1 of image m (m = (a PY + b) PZ + k, shifts ascending)
+  __device__ __forceinline__ void image(int m, double L, double &X, double &Y, double &Z) const {
+    const int a = m / (PY * PZ), b = (m / PZ) % PY, k = m % PZ;
+    X = PX == 3 ? rx[PX / 2] + (a - 1) * L : rx[0];
+    Y = PY == 3 ? ry[PY / 2] + (b - 1) * L : ry[0];
+    Z = PZ == 3 ? rz[PZ / 2] + (k - 1) * L : rz[0];
   }
   // Adds the velocity terms of every image (the unshifted one unless skip_main)
-  // to (ax, ay, az); s is the same in all of them, so f and f R1 are summed
-  // over the images and the cross product is taken once.
-  __device__ __forceinline__ void velocity(double sx, double sy, double sz, double c, double L,
-                                           bool fast, bool skip_main, double &ax, double &ay,
-                                           double &az) const {
+  // to (ax, ay, az).  s is the same in all of them, so f and f R1 are summed
+  // over the images -- sum f R1 per axis is the sum over its shifts of (R1
+  // component) x (sum of f at that shift) -- and the cross product is taken
+  // once.  fast: far() holds.
+  __device__ __forceinline__ void velocity(double L, bool fast, bool skip_main, double &ax,
+                                           double &ay, double &az) const {
     if (!fast) {
 #pragma unroll 1
-      for (int m = 0; m < PX * PY * PZ; m++) {
-        if (skip_main && m == PX * PY * PZ / 2) continue;  // the middle one is unshifted
+      for (int m = 0; m < NI; m++) {
+        if (skip_main && m == NI / 2) continue;  // the middle one is unshifted
         double X, Y, Z;
         image(m, L, X, Y, Z);
         const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
@@ -161,21 +179,13 @@ struct Seg64 {
       return;
     }
     double fx[PX], fy[PY], fz[PZ];  // sum of f at each shift of an axis
+    double tx[PX], ty[PY], tz[PZ];  // parts of |R2|^2 = R1.R2 + R1.s + |s|^2
 #pragma unroll
-    for (int k = 0; k < PX; k++) fx[k] = 0.;
+    for (int k = 0; k < PX; k++) { fx[k] = 0.; tx[k] = fma(rx[k], sx, gx[k] + c); }
 #pragma unroll
-    for (int k = 0; k < PY; k++) fy[k] = 0.;
+    for (int k = 0; k < PY; k++) { fy[k] = 0.; ty[k] = fma(ry[k], sy, gy[k]); }
 #pragma unroll
-    for (int k = 0; k < PZ; k++) fz[k] = 0.;
-    // per-axis parts of A = |R1|^2 (p), d = R1.R2 = A + R1.s (g), B = |R2|^2 =
-    // d + R1.s + |s|^2 (t)
-    double gx[PX], tx[PX], gy[PY], ty[PY], gz[PZ], tz[PZ];
-#pragma unroll
-    for (int k = 0; k < PX; k++) { gx[k] = fma(rx[k], sx, px[k]); tx[k] = fma(rx[k], sx, gx[k] + c); }
-#pragma unroll
-    for (int k = 0; k < PY; k++) { gy[k] = fma(ry[k], sy, py[k]); ty[k] = fma(ry[k], sy, gy[k]); }
-#pragma unroll
-    for (int k = 0; k < PZ; k++) { gz[k] = fma(rz[k], sz, pz[k]); tz[k] = fma(rz[k], sz, gz[k]); }
+    for (int k = 0; k < PZ; k++) { fz[k] = 0.; tz[k] = fma(rz[k], sz, gz[k]); }
 #pragma unroll
     for (int a = 0; a < PX; a++) {
 #pragma unroll
@@ -184,7 +194,11 @@ struct Seg64 {
         double row = 0.;
 #pragma unroll
         for (int k = 0; k < PZ; k++) {
-          const double f = seg_f_pos(pxy + pz[k], txy + tz[k], gxy + gz[k]);
+          double A = pxy + pz[k], B = txy + tz[k], d = gxy + gz[k];
+          const bool own = skip_main && (a * PY + b) * PZ + k == NI / 2;
+          if (own) A = B = d = 1.;
+          double f = seg_f_pos(A, B, d);
+          if (own) f = 0.;
           row += f;
           fz[k] += f;
         }
@@ -203,11 +217,103 @@ struct Seg64 {
     ay += hz * sx - hx * sz;
     az += hx * sy - hy * sx;
   }
-  // R1 of image m (m = (a PY + b) PZ + k, shifts ascending)
-  __device__ __forceinline__ void image(int m, double L, double &X, double &Y, double &Z) const {
-    const int a = m / (PY * PZ), b = (m / PZ) % PY, k = m % PZ;
-    X = PX == 3 ? rx[PX / 2] + (a - 1) * L : rx[0];
-    Y = PY == 3 ? ry[PY / 2] + (b - 1) * L : ry[0];
-    Z = PZ == 3 ? rz[PZ / 2] + (k - 1) * L : rz[0];
+  // Whether some image may have its target exactly on the segment's line
+  // (R1 x s = 0): those terms' gradients are left out.
+  __device__ __forceinline__ bool on_line() const {
+    bool z = false;
+#pragma unroll
+    for (int a = 0; a < PX; a++)
+#pragma unroll
+      for (int b = 0; b < PY; b++) z |= rx[a] * sy - ry[b] * sx == 0.;
+    if (!z) return false;
+    z = false;
+#pragma unroll
+    for (int b = 0; b < PY; b++)
+#pragma unroll
+      for (int k = 0; k < PZ; k++) z |= ry[b] * sz - rz[k] * sy == 0.;
+    if (!z) return false;
+    z = false;
+#pragma unroll
+    for (int a = 0; a < PX; a++)
+#pragma unroll
+      for (int k = 0; k < PZ; k++) z |= rz[k] * sx - rx[a] * sz == 0.;
+    return z;
+  }
+  // For an upstream g, the gradient of g . sum over images of f (R1 x s): dR
+  // with respect to x_j at fixed s (minus the target's), dS with respect to s.
+  // With h = s x g, Q = g.(R1 x s) = R1.h, alpha = 2 Q fA, beta = Q fw:
+  //   dR = h sum f + sum alpha R1 + s sum beta
+  //   dS = g x sum f R1 + sum beta R1 + s sum Q 2 fc
+  // fast: far() holds and on_line() does not.
+  __device__ __forceinline__ void gradient(double ux, double uy, double uz, double L, bool fast,
+                                           bool skip_main, double *dR, double *dS) const {
+    const double hx = sy * uz - sz * uy, hy = sz * ux - sx * uz, hz = sx * uy - sy * ux;
+    double f0 = 0., b0 = 0., c0 = 0.;
+    double fX = 0., fY = 0., fZ = 0., aX = 0., aY = 0., aZ = 0., bX = 0., bY = 0., bZ = 0.;
+    if (fast) {
+      double tx[PX], ty[PY], tz[PZ], qx[PX], qy[PY], qz[PZ];
+#pragma unroll
+      for (int k = 0; k < PX; k++) { tx[k] = fma(rx[k], sx, gx[k] + c); qx[k] = rx[k] * hx; }
+#pragma unroll
+      for (int k = 0; k < PY; k++) { ty[k] = fma(ry[k], sy, gy[k]); qy[k] = ry[k] * hy; }
+#pragma unroll
+      for (int k = 0; k < PZ; k++) { tz[k] = fma(rz[k], sz, gz[k]); qz[k] = rz[k] * hz; }
+#pragma unroll
+      for (int a = 0; a < PX; a++) {
+        double fa = 0., aa = 0., ba = 0.;  // sums over the shifts (b, k) of this a
+#pragma unroll
+        for (int b = 0; b < PY; b++) {
+          const double pxy = px[a] + py[b], gxy = gx[a] + gy[b], txy = tx[a] + ty[b],
+                       qxy = qx[a] + qy[b];
+          double fb = 0., ab = 0., bb = 0.;
+#pragma unroll
+          for (int k = 0; k < PZ; k++) {
+            double A = pxy + pz[k], B = txy + tz[k], d = gxy + gz[k];
+            double Q = qxy + qz[k];
+            const bool own = skip_main && (a * PY + b) * PZ + k == NI / 2;
+            if (own) A = B = d = 1.;
+            SegD t = seg_d_pos(A, B, d);
+            if (own) t.f = Q = 0.;
+            const double al = 2. * Q * t.fA, be = Q * t.fw;
+            c0 = fma(Q, t.fc2, c0);
+            fb += t.f; ab += al; bb += be;
+            fZ = fma(t.f, rz[k], fZ);
+            aZ = fma(al, rz[k], aZ);
+            bZ = fma(be, rz[k], bZ);
+          }
+          fa += fb; aa += ab; ba += bb;
+          fY = fma(fb, ry[b], fY);
+          aY = fma(ab, ry[b], aY);
+          bY = fma(bb, ry[b], bY);
+        }
+        f0 += fa; b0 += ba;
+        fX = fma(fa, rx[a], fX);
+        aX = fma(aa, rx[a], aX);
+        bX = fma(ba, rx[a], bX);
+      }
+    } else {
+#pragma unroll 1
+      for (int m = 0; m < NI; m++) {
+        if (skip_main && m == NI / 2) continue;
+        double X, Y, Z;
+        image(m, L, X, Y, Z);
+        const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
+        const double cx = Y * sz - Z * sy, cy = Z * sx - X * sz, cz = X * sy - Y * sx;
+        const double ex = X + sx, ey = Y + sy, ez = Z + sz;
+        const SegD t =
+            seg_d_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
+        const double Q = X * hx + Y * hy + Z * hz, al = 2. * Q * t.fA, be = Q * t.fw;
+        f0 += t.f; b0 += be; c0 += Q * t.fc2;
+        fX += t.f * X; fY += t.f * Y; fZ += t.f * Z;
+        aX += al * X; aY += al * Y; aZ += al * Z;
+        bX += be * X; bY += be * Y; bZ += be * Z;
+      }
+    }
+    dR[0] = fma(hx, f0, fma(sx, b0, aX));
+    dR[1] = fma(hy, f0, fma(sy, b0, aY));
+    dR[2] = fma(hz, f0, fma(sz, b0, aZ));
+    dS[0] = fma(sx, c0, bX) + (uy * fZ - uz * fY);
+    dS[1] = fma(sy, c0, bY) + (uz * fX - ux * fZ);
+    dS[2] = fma(sz, c0, bZ) + (ux * fY - uy * fX);
   }
 };

@@ -113,3 +113,99 @@ def test_field_velocity_and_jacobian_at_split_edges(n, m, bc, images):
                 oJ[:, r] += torch.autograd.grad(v[:, r].sum(), P, retain_graph=r < 2)[0].numpy()
     assert np.abs(u - ou).max() <= 1e-11 * np.abs(ou).max()
     assert np.abs(J - oJ).max() <= 1e-11 * np.abs(oJ).max()
+
+
+def _direct_vjp(w, ubar, bc):
+    """x_bar of the BS arm by torch autograd: local term (second order) and the
+    direct sum over images, without the pairs whose target lies exactly on the
+    segment's line (they are left out of the gradient)."""
+    import torch
+
+    p = O.params(**dict(w.params, boundary=bc))
+    x = torch.tensor(w.x, requires_grad=True)
+    inf, beh = torch.tensor(w.infront).long() - 1, torch.tensor(w.behind).long() - 1
+    g = O.ghosts(p, w.x, w.infront, w.behind)
+    gi = x[inf] + (torch.tensor(g[0]) - x[inf]).detach()
+    gb = x[beh] + (torch.tensor(g[1]) - x[beh]).detach()
+    i, b = (x - gi).norm(dim=1, keepdim=True), (x - gb).norm(dim=1, keepdim=True)
+    s1 = (b * gi + (i - b) * x - i * gb) / (2 * b * i)
+    s2 = 2 * (gi / (i * (i + b)) - x / (i * b) + gb / (b * (i + b)))
+    G = p.quant_circ / (4 * np.pi)
+    loss = (G * torch.log(1.21 / p.corea * torch.sqrt(i * b)) * torch.linalg.cross(s1, s2)
+            * torch.tensor(ubar)).sum()
+    n = w.n
+    ax = {"open": (0, 0, 0), "openxy": (0, 0, 1), "openx": (0, 1, 1), "periodic": (1, 1, 1)}[bc]
+    for a in range(-ax[0], ax[0] + 1):
+        for c in range(-ax[1], ax[1] + 1):
+            for d in range(-ax[2], ax[2] + 1):
+                sh = torch.tensor([a, c, d], dtype=torch.float64) * p.box_size
+                skip = torch.arange(n)[None] == beh[:, None]
+                if (a, c, d) == (0, 0, 0):
+                    skip = skip | torch.eye(n, dtype=torch.bool)
+                r1 = (x + sh)[None] - x[:, None]
+                s = (gi - x)[None].expand_as(r1)
+                skip = skip | (torch.linalg.cross(r1, s).detach() == 0).all(-1)
+                r1 = torch.where(skip[..., None], torch.ones_like(r1), r1)
+                s = torch.where(skip[..., None], torch.tensor([1.0, 0.0, 0.0]).double(), s)
+                r2, cr = r1 + s, torch.linalg.cross(r1, s)
+                A, B, D = r1.norm(dim=-1), r2.norm(dim=-1), (r1 * r2).sum(-1)
+                den = torch.where(D < 0, (cr * cr).sum(-1) / torch.where(D < 0, A * B - D, 1.0),
+                                  A * B + D)
+                f = (A + B) / (A * B * den) * (~skip)
+                loss = loss + (G * f[..., None] * cr * torch.tensor(ubar)[:, None]).sum()
+    return torch.autograd.grad(loss, x)[0].numpy()
+
+
+def _vjp(w, ubar, bc):
+    import torch
+
+    from qvort_b200 import adjoint as A
+    from qvort_b200 import lib as L
+
+    s = A.FilamentSystem(L.default_params(**dict(w.params, boundary=bc, precision="fp64")),
+                         w.infront, w.behind)
+    x = torch.tensor(w.x, device="cuda", requires_grad=True)
+    (g,) = torch.autograd.grad(A.velocity(x, s), x, torch.tensor(ubar, device="cuda"))
+    s.close()
+    return g.cpu().numpy()
+
+
+@pytest.mark.parametrize("bc", ["open", "openxy", "openx", "periodic"])
+@pytest.mark.parametrize("n", [5, 31, 33, 128, 129, 260])
+def test_direct_vjp_at_tile_and_chunk_edges(n, bc):
+    """Both ends' gradients of every pair.  Each gradient is a difference of
+    terms larger by at most |d|/|s| < 1e4 (see above): 1e-11 of the largest."""
+    w = _ring_pair(n)
+    ubar = np.random.default_rng(n).normal(0.0, 0.1, w.x.shape)
+    g, og = _vjp(w, ubar, bc), _direct_vjp(w, ubar, bc)
+    assert np.abs(g - og).max() <= 1e-11 * np.abs(og).max()
+
+
+@pytest.mark.parametrize("bc", ["open", "periodic"])
+def test_direct_vjp_near_and_on_a_segments_line(bc):
+    """A target beside the middle of another filament's segment (obtuse angle
+    between its ends), a square of axis-parallel sides whose points lie exactly
+    on one another's lines, and a planar ring."""
+    w = W.ring(24, 0.01, 0.0, seed=1)          # exactly in z = 0
+    h = 0.0078125
+    t = np.arange(4)[:, None] * h
+    o = np.zeros((4, 1))
+    sq = np.concatenate([np.hstack([t, o, o]), np.hstack([o + 4 * h, t, o]),
+                         np.hstack([4 * h - t, o + 4 * h, o]), np.hstack([o, 4 * h - t, o])])
+    sq = sq + [-0.03125, -0.03125, 0.015625]
+    k = w.n
+    mid = 0.5 * (w.x[3] + w.x[4]) + [0.0, 0.0, 2e-5]
+    near = np.array([mid, mid + [0.004, 0.001, 0.003], mid + [-0.002, 0.004, 0.005],
+                     mid + [0.001, -0.003, 0.002], mid + [0.003, 0.003, 0.006]])
+    m = len(sq)
+    x = np.concatenate([w.x, sq, near])
+    inf = np.concatenate([w.infront, k + 1 + (np.arange(m) + 1) % m,
+                          k + m + 1 + (np.arange(5) + 1) % 5]).astype(np.int32)
+    beh = np.concatenate([w.behind, k + 1 + (np.arange(m) - 1) % m,
+                          k + m + 1 + (np.arange(5) - 1) % 5]).astype(np.int32)
+    v = W.Workload("lines", x, inf, beh, w.params)
+    ubar = np.random.default_rng(3).normal(0.0, 0.1, x.shape)
+    g, og = _vjp(v, ubar, bc), _direct_vjp(v, ubar, bc)
+    assert np.isfinite(g).all()
+    # the near pair's 1 + cos is about 1e-3 of 1: its digits cost another 1e3
+    assert np.abs(g - og).max() <= 1e-9 * np.abs(og).max()
