@@ -1100,139 +1100,196 @@ int qv_launch_walk(qv_ctx *c) {
 // ------------------------------------------------------- field points (tree)
 // tree_walk_general (src/tree.f90:425-488) at m arbitrary points, as the Tree
 // arm of mesh_velocity uses it (src/timestep.f90:374-452): per point the
-// unshifted tree, then the boundary's images in the reference's loop order,
-// all into one running FP64 sum, with the reference's operations: a node
-// within epsilon of the point adds nothing (its subtree included), the
-// opening test is width/dist < tree_theta, a leaf's segment runs from its
-// centroid to centroid + circ, the leaf term is divided by 4 pi, the far term
-// is not, and neither carries quant_circ.  One warp per 32 points with the
-// warp-coherent (node, lane mask) stack of the velocity walk.
+// unshifted tree and the boundary's images: a node within epsilon of the point
+// adds nothing (its subtree included), the opening test is width/dist <
+// tree_theta, a leaf's segment runs from its point to its ghost, the leaf term
+// is divided by 4 pi, the far term is not, and neither carries quant_circ.
+//
+// The points are taken in Morton order of a grid of cells, so that the 32 of a
+// warp open the same nodes (a mesh's own order runs a line of points across
+// the box).  A warp task is (32 points, one image, and for the unshifted image
+// one root child), as in the velocity walk; its partial sums are added per
+// point in the images' order, so results do not depend on the grouping.  Bound:
+// FP64 issue and the latency of a pop.  32^3 mesh through the tangle (24.7k
+// points, 27 images, theta 0.4): 19.5 ms with one warp per 32 mesh points in
+// their own order over all images and 54 divisions per far cell (20-23 ms a
+// call), 0.82 ms a call now, copies included.
 #define GW 4
+#define QV_MESH_SLAB 65536  // points per launch (bounds the partial sums: 53 MB)
+
+// Morton cell of a point in a grid of 2^b cells a side over [-L/2, L/2);
+// points outside fall in the border cells (a NaN in cell 0).
+__device__ __forceinline__ int morton_cell(const double *p, double L, int b) {
+  const int n = 1 << b;
+  int key = 0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const int g = min(n - 1, max(0, __double2int_rd((p[c] / L + 0.5) * n)));
+    for (int k = 0; k < b; k++) key |= ((g >> k) & 1) << (3 * k + c);
+  }
+  return key;
+}
+__global__ void k_mesh_count(int m, const double *__restrict__ pts, double L, int b, int *cell) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < m) atomicAdd(&cell[morton_cell(pts + 3 * (size_t)q, L, b)], 1);
+}
+// cell: the cells' offsets, advanced past their points
+__global__ void k_mesh_scatter(int m, const double *__restrict__ pts, double L, int b, int *cell,
+                               int *perm) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < m) perm[atomicAdd(&cell[morton_cell(pts + 3 * (size_t)q, L, b)], 1)] = q;
+}
+
+struct MeshArgs {
+  int m;            // points of this slab
+  const int *perm;  // their indices
+  const double *pts;
+  const WNode64 *w64;
+  const WPay64 *p64;
+  const double *cent, *circ;
+  double L, theta;
+  double *part;  // (NSPLIT + images) x m x 3
+  unsigned long long *evals;
+  int stk_cap, *status;
+};
+
+// width/dist < tree_theta on node h (true: take it whole); skip: within epsilon
+__device__ __forceinline__ bool general_far(const double *x, const WNode64 &h, const double *s,
+                                            double theta, bool &skip) {
+  const double dist = exact_dist(x, h, s);
+  skip = dist < QV_DEPS;
+  return __ddiv_rn(h.width, dist) < theta;
+}
+
+// A leaf's term in the reference's own operations (src/tree.f90:450-467): the
+// segment from its centroid to centroid + circ, which may end on the point.
+__device__ __noinline__ void general_leaf(const double *x, const double *C0, const double *R,
+                                          const double *s, double *acc) {
+  double v1[3], v2[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    v1[c] = __dsub_rn(__dadd_rn(C0[c], s[c]), x[c]);
+    v2[c] = __dsub_rn(__dadd_rn(__dadd_rn(C0[c], R[c]), s[c]), x[c]);
+  }
+  const double a = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v1[0], v1[0]), __dmul_rn(v1[1], v1[1])), __dmul_rn(v1[2], v1[2])));
+  const double b = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v2[0], v2[0]), __dmul_rn(v2[1], v2[1])), __dmul_rn(v2[2], v2[2])));
+  const double dv = __dadd_rn(__dadd_rn(__dmul_rn(v1[0], v2[0]), __dmul_rn(v1[1], v2[1])), __dmul_rn(v1[2], v2[2]));
+  const double ab = __dmul_rn(a, b);
+  const double cc = __dmul_rn(ab, __dadd_rn(ab, dv));
+  const double f = __ddiv_rn(__dadd_rn(a, b), cc);
+  const double cr[3] = {__dsub_rn(__dmul_rn(v1[1], v2[2]), __dmul_rn(v1[2], v2[1])),
+                        __dsub_rn(__dmul_rn(v1[2], v2[0]), __dmul_rn(v1[0], v2[2])),
+                        __dsub_rn(__dmul_rn(v1[0], v2[1]), __dmul_rn(v1[1], v2[0]))};
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    acc[c] = __dadd_rn(acc[c], __ddiv_rn(__ddiv_rn(__dmul_rn(f, cr[c]), 4.), QV_PI));
+}
+
 template <int BC>
-__global__ void __launch_bounds__(GW * 32) k_walk_general(int m, const double *__restrict__ pts,
-                                                         const WNode64 *__restrict__ w64,
-                                                         const WPay64 *__restrict__ p64,
-                                                         const double *__restrict__ cent,
-                                                         const double *__restrict__ circ,
-                                                         double L, double theta, int nroots,
-                                                         double *u, unsigned long long *evals,
-                                                         int *status) {
+__global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
   constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
-  __shared__ int2 stk[GW][STK];
+  extern __shared__ StkEnt64 stk_pts[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int2 *st = stk[wid];
-  const int ngroups = (m + 31) / 32;
-  for (int g = blockIdx.x * GW + wid; g < ngroups; g += gridDim.x * GW) {
-    const int q = g * 32 + lane;
-    const bool live = q < m;
-    double x[3] = {0., 0., 0.};
-    if (live) { x[0] = pts[3 * q]; x[1] = pts[3 * q + 1]; x[2] = pts[3 * q + 2]; }
-    double acc[3] = {0., 0., 0.};
-    unsigned long long ev = 0;
+  StkEnt64 *st = stk_pts + wid * a.stk_cap;
+  const int ngroups = (a.m + 31) / 32;
+  const int items = ngroups * (NSPLIT + NIMG);
+  const double ith = 1. / a.theta;
+  for (int item = blockIdx.x * GW + wid; item < items; item += gridDim.x * GW) {
+    const int sl = item / ngroups, q = (item - sl * ngroups) * 32 + lane;
+    const bool live = q < a.m;
+    double s[3], x[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
+    slot_shift(BC, sl, a.L, s);
+    if (live) {
+      const double *p = a.pts + 3 * (size_t)a.perm[q];
+      x[0] = p[0]; x[1] = p[1]; x[2] = p[2];
+    }
+    const double t0 = x[0] - s[0], t1 = x[1] - s[1], t2 = x[2] - s[2];
+    unsigned ev = 0;
     bool bad = false;
-    const unsigned live_mask = __ballot_sync(0xffffffffu, live);
-    for (int img = -1; img < NIMG; img++) {
-      int ma = 0, mb = 0, mc = 0;
-      if (img >= 0) qv_img_shift(BC, img, &ma, &mb, &mc);
-      const double s[3] = {shift_of(ma, L), shift_of(mb, L), shift_of(mc, L)};
-      int top = 0;
-      if (lane == 0) st[0] = make_int2(0, (int)live_mask);
-      top = live_mask ? 1 : 0;
-      __syncwarp();
-      while (top > 0) {
-        top--;
-        const int2 e = st[top];
-        __syncwarp();
-        const int node = e.x;
-        const bool in = (((unsigned)e.y) >> lane) & 1u;
-        const WNode64 h = w64[node];
-        bool open = false;
-        if (in && h.count > 0) {
-          const double dist = exact_dist(x, h, s);
-          if (!(dist < QV_DEPS)) {
-            const double th = __ddiv_rn(h.width, dist);
-            const double zero3[3] = {0., 0., 0.};
-            const double *C0 = cent + 3 * node, *R = node < nroots ? zero3 : circ + 3 * node;
-            if (h.count == 1) {
-              double v1[3], v2[3];
-#pragma unroll
-              for (int c = 0; c < 3; c++) {
-                v1[c] = __dsub_rn(__dadd_rn(C0[c], s[c]), x[c]);
-                v2[c] = __dsub_rn(__dadd_rn(__dadd_rn(C0[c], R[c]), s[c]), x[c]);
-              }
-              const double a = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v1[0], v1[0]), __dmul_rn(v1[1], v1[1])), __dmul_rn(v1[2], v1[2])));
-              const double b = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v2[0], v2[0]), __dmul_rn(v2[1], v2[1])), __dmul_rn(v2[2], v2[2])));
-              const double dv = __dadd_rn(__dadd_rn(__dmul_rn(v1[0], v2[0]), __dmul_rn(v1[1], v2[1])), __dmul_rn(v1[2], v2[2]));
-              const double ab = __dmul_rn(a, b);
-              const double cc = __dmul_rn(ab, __dadd_rn(ab, dv));
-              const double f = __ddiv_rn(__dadd_rn(a, b), cc);
-              const double cr[3] = {__dsub_rn(__dmul_rn(v1[1], v2[2]), __dmul_rn(v1[2], v2[1])),
-                                    __dsub_rn(__dmul_rn(v1[2], v2[0]), __dmul_rn(v1[0], v2[2])),
-                                    __dsub_rn(__dmul_rn(v1[0], v2[1]), __dmul_rn(v1[1], v2[0]))};
-#pragma unroll
-              for (int c = 0; c < 3; c++)
-                acc[c] = __dadd_rn(acc[c], __ddiv_rn(__ddiv_rn(__dmul_rn(f, cr[c]), 4.), QV_PI));
-              ev++;
-            } else if (th < theta) {
-              const double v[3] = {__dsub_rn(x[0], __dadd_rn(C0[0], s[0])),
-                                   __dsub_rn(x[1], __dadd_rn(C0[1], s[1])),
-                                   __dsub_rn(x[2], __dadd_rn(C0[2], s[2]))};
-              const double d2 = __dmul_rn(dist, dist);
-              const double d3 = __dmul_rn(d2, dist);
-              const double d5 = __dmul_rn(__dmul_rn(d2, d2), dist);
-              const WPay64 &P = p64[node];
-              double ci[3], Cm[9];
-#pragma unroll
-              for (int c = 0; c < 3; c++) ci[c] = node < nroots ? 0. : P.a[c];
-#pragma unroll
-              for (int c = 0; c < 9; c++) Cm[c] = node < nroots ? 0. : P.C[c];
-              double ub[3] = {__ddiv_rn(__dsub_rn(__dmul_rn(ci[1], v[2]), __dmul_rn(ci[2], v[1])), d3),
-                              __ddiv_rn(__dsub_rn(__dmul_rn(ci[2], v[0]), __dmul_rn(ci[0], v[2])), d3),
-                              __ddiv_rn(__dsub_rn(__dmul_rn(ci[0], v[1]), __dmul_rn(ci[1], v[0])), d3)};
-              for (int k = 0; k < 3; k++)
-                for (int l = 0; l < 3; l++) {
-                  double vc = __dmul_rn(v[0], Cm[l]);
-                  vc = __dadd_rn(vc, __dmul_rn(v[1], Cm[3 + l]));
-                  vc = __dadd_rn(vc, __dmul_rn(v[2], Cm[6 + l]));
-#pragma unroll
-                  for (int mm = 0; mm < 3; mm++) {
-                    const double e = (mm == k || k == l || l == mm) ? 0.
-                                     : ((mm + 1) % 3 == k ? 1. : -1.);  // eps(m,k,l)
-                    ub[mm] = __dsub_rn(ub[mm], __ddiv_rn(__dmul_rn(e, Cm[3 * k + l]), d3));
-                  }
-#pragma unroll
-                  for (int mm = 0; mm < 3; mm++) {
-                    const double e = (mm == k || k == l || l == mm) ? 0.
-                                     : ((mm + 1) % 3 == k ? 1. : -1.);
-                    ub[mm] = __dadd_rn(ub[mm], __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(3., e), v[k]), vc), d5));
-                  }
-                }
-#pragma unroll
-              for (int c = 0; c < 3; c++) acc[c] = __dadd_rn(acc[c], ub[c]);
-              ev++;
-            } else {
-              open = true;
-            }
-          }
-        }
-        const unsigned om = __ballot_sync(0xffffffffu, open);
-        if (om) {
-          int nc = h.nchild;
-          if (top + nc > STK) {  // unreachable for trees within QV_MAX_DEPTH
-            bad = true;
-            nc = 0;
-          }
-          if (lane < nc) st[top + lane] = make_int2(h.child_first + nc - 1 - lane, (int)om);
-          top += nc;
-        }
-        __syncwarp();
+    // the root's own decision; the unshifted image's tasks then take one child
+    const WNode64 r = a.w64[0];
+    bool ropen = false;
+    if (live) {
+      bool skip;
+      const bool far = general_far(x, r, s, a.theta, skip);
+      if (!skip) {
+        // a lone point's root carries no segment, a far root no moments
+        if (r.count == 1 || far) ev += sl == 0 || sl >= NSPLIT;
+        else ropen = true;
       }
     }
-    if (live) { u[3 * q] = acc[0]; u[3 * q + 1] = acc[1]; u[3 * q + 2] = acc[2]; }
+    const unsigned rm = __ballot_sync(0xffffffffu, ropen);
+    const int c0 = sl < NSPLIT ? sl : 0, c1 = sl < NSPLIT ? min(r.nchild, sl + 1) : r.nchild;
+    int top = rm && c1 > c0 ? c1 - c0 : 0;
+    if (lane < top) {
+      const int ch = r.child_first + c1 - 1 - lane;
+      fill_ent64(st[lane], a.w64[ch], ch, rm, ith, false, true);
+    }
+    __syncwarp();
+    while (top > 0) {
+      top--;
+      const StkEnt64 e = st[top];
+      const bool in = (e.mask >> lane) & 1u;
+      __syncwarp();
+      const double v0 = t0 - e.cx, v1 = t1 - e.cy, v2 = t2 - e.cz;
+      const double d2 = fma(v0, v0, fma(v1, v1, v2 * v2));
+      bool skip = false;
+      if (e.nc < 0) {
+        if (in) {
+          if (d2 < 1e-28) general_far(x, a.w64[e.node], s, a.theta, skip);
+          if (!skip) {
+            const WPay64 &P = a.p64[e.node];
+            if (!leaf_term64(-v0, -v1, -v2, P.b[0] - t0, P.b[1] - t1, P.b[2] - t2, P.b[0] - e.cx,
+                             P.b[1] - e.cy, P.b[2] - e.cz, 1. / (4. * QV_PI), acc))
+              general_leaf(x, a.cent + 3 * (size_t)e.node, a.circ + 3 * (size_t)e.node, s, acc);
+            ev++;
+          }
+        }
+        continue;
+      }
+      bool far = in && d2 > e.rhi, open = in && d2 < e.rlo;
+      if (in && (!(far || open) || d2 < 1e-28)) {
+        far = general_far(x, a.w64[e.node], s, a.theta, skip);
+        open = !skip && !far;
+        far = !skip && far;
+      }
+      if (far) {
+        far_term64(v0, v1, v2, d2, a.p64[e.node], acc);
+        ev++;
+      }
+      const unsigned om = __ballot_sync(0xffffffffu, open);
+      if (om) {
+        int nc = e.nc;
+        if (top + nc > a.stk_cap) {  // unreachable: the cap follows the tree depth
+          bad = true;
+          nc = 0;
+        }
+        if (lane < nc) {
+          const int ch = e.child_first + nc - 1 - lane;
+          fill_ent64(st[top + lane], a.w64[ch], ch, om, ith, false, true);
+        }
+        top += nc;
+      }
+      __syncwarp();
+    }
+    if (live) {
+      double *o = a.part + ((size_t)sl * a.m + q) * 3;
+      o[0] = acc[0]; o[1] = acc[1]; o[2] = acc[2];
+    }
     for (int o = 16; o > 0; o >>= 1) ev += __shfl_down_sync(0xffffffffu, ev, o);
-    if (lane == 0 && ev) atomicAdd(evals, ev);
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, QV_STAT_STACK);
+    if (lane == 0 && ev) atomicAdd(a.evals, (unsigned long long)ev);
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.status, QV_STAT_STACK);
   }
+}
+
+__global__ void k_mesh_reduce(int m, int nslot, const int *__restrict__ perm,
+                              const double *__restrict__ part, double *u) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * m) return;
+  double v = 0.;
+#pragma unroll 8
+  for (int k = 0; k < nslot; k++) v += part[(size_t)k * 3 * m + t];
+  u[3 * (size_t)perm[t / 3] + t % 3] = v;
 }
 
 extern "C" int qv_field_velocity_tree(qv_ctx *c, int m, const double *pts, double *u,
@@ -1250,37 +1307,61 @@ extern "C" int qv_field_velocity_tree(qv_ctx *c, int m, const double *pts, doubl
     if ((rc = qv_launch_tree_build(c))) return rc;
   if ((rc = qv_tree_finalize_root(c))) return rc;
   TreeBuf &t = c->tree;
-  double *dp = nullptr;
-  QV_CUDA(c, cudaMalloc((void **)&dp, sizeof(double) * 6 * (size_t)m));
-  struct Free {
-    double *p;
-    ~Free() { cudaFree(p); }
-  } guard{dp};  // freed on every return path
-  double *du = dp + 3 * (size_t)m;
-  QV_CUDA(c, cudaMemcpyAsync(dp, pts, sizeof(double) * 3 * m, cudaMemcpyHostToDevice, c->stream));
+  // points, results, partial sums of a slab, the points' Morton order and cells
+  const int nslot = NSPLIT + qv_img_count(c->p.boundary);
+  const int slab = std::min(m, QV_MESH_SLAB);
+  int b = 1;
+  while (b < 5 && (16 << (3 * b)) < m) b++;  // about 16 points a cell, 32^3 cells at most
+  const int ncell = 1 << (3 * b);
+  const size_t np = 3 * (size_t)m, npart = 3 * (size_t)slab * nslot;
+  const size_t need = sizeof(double) * (2 * np + npart) + sizeof(int) * ((size_t)m + ncell + 2);
+  if (need > c->field_bytes) {
+    c->field_bytes = 0;  // the old buffer goes first
+    if ((rc = qv_grow(c, (void **)&c->field_buf, need))) return rc;
+    c->field_bytes = need;
+  }
+  double *dp = c->field_buf, *du = dp + np, *part = du + np;
+  int *perm = (int *)(part + npart), *cell = perm + m;
+  QV_CUDA(c, cudaMemcpyAsync(dp, pts, sizeof(double) * np, cudaMemcpyHostToDevice, c->stream));
   QV_CUDA(c, cudaMemsetAsync(c->evals, 0, sizeof(unsigned long long), c->stream));
   QV_CUDA(c, cudaMemsetAsync(c->dstatus, 0, sizeof(int), c->stream));
-  const int nb = std::max(1, std::min((m + 32 * GW - 1) / (32 * GW), 64 * c->sm_count));
-  switch (c->p.boundary) {
-#define QV_GW_CASE(BCV)                                                                          \
-  case BCV:                                                                                      \
-    k_walk_general<BCV><<<nb, GW * 32, 0, c->stream>>>(m, dp, t.w64, t.p64, t.cent, t.circ,     \
-                                                       c->p.box_size, c->p.tree_theta, 1, du,   \
-                                                       c->evals, c->dstatus);                   \
-    break;
-    QV_GW_CASE(QV_BC_OPEN)
-    QV_GW_CASE(QV_BC_PERIODIC)
-    QV_GW_CASE(QV_BC_OPENX)
-    QV_GW_CASE(QV_BC_OPENXY)
-#undef QV_GW_CASE
-    default:
-      return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d not supported", c->p.boundary);
-  }
+  QV_CUDA(c, cudaMemsetAsync(cell, 0, sizeof(int) * ncell, c->stream));
+  const int pb = (m + 255) / 256;
+  k_mesh_count<<<pb, 256, 0, c->stream>>>(m, dp, c->p.box_size, b, cell);
+  k_scan_small<<<1, 1024, 0, c->stream>>>(ncell, cell, cell + ncell);
+  k_mesh_scatter<<<pb, 256, 0, c->stream>>>(m, dp, c->p.box_size, b, cell, perm);
   QV_LAUNCH_CHECK(c);
-  QV_COUNT(c, 1);
+  QV_COUNT(c, 3);
+  MeshArgs a;
+  a.pts = dp; a.w64 = t.w64; a.p64 = t.p64; a.cent = t.cent; a.circ = t.circ;
+  a.L = c->p.box_size; a.theta = c->p.tree_theta;
+  a.part = part; a.evals = c->evals; a.status = c->dstatus;
+  a.stk_cap = 7 * (t.depth + 1) + 8;  // as in the velocity walk
+  const size_t smem = sizeof(StkEnt64) * a.stk_cap * GW;
+  const void *f = nullptr;
+  switch (c->p.boundary) {
+    case QV_BC_OPEN: f = (const void *)k_walk_general<QV_BC_OPEN>; break;
+    case QV_BC_PERIODIC: f = (const void *)k_walk_general<QV_BC_PERIODIC>; break;
+    case QV_BC_OPENX: f = (const void *)k_walk_general<QV_BC_OPENX>; break;
+    case QV_BC_OPENXY: f = (const void *)k_walk_general<QV_BC_OPENXY>; break;
+    default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d not supported", c->p.boundary);
+  }
+  if (smem > 48 * 1024)
+    QV_CUDA(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  for (int lo = 0; lo < m; lo += slab) {
+    a.m = std::min(slab, m - lo);
+    a.perm = perm + lo;
+    const int items = (a.m + 31) / 32 * nslot;
+    const int nb = std::max(1, std::min((items + GW - 1) / GW, 64 * c->sm_count));
+    void *args[] = {&a};
+    QV_CUDA(c, cudaLaunchKernel(f, dim3(nb), dim3(GW * 32), args, smem, c->stream));
+    k_mesh_reduce<<<(3 * a.m + 255) / 256, 256, 0, c->stream>>>(a.m, nslot, a.perm, part, du);
+    QV_LAUNCH_CHECK(c);
+    QV_COUNT(c, 2);
+  }
   unsigned long long ev = 0;
   int st = 0;
-  QV_CUDA(c, cudaMemcpyAsync(u, du, sizeof(double) * 3 * m, cudaMemcpyDeviceToHost, c->stream));
+  QV_CUDA(c, cudaMemcpyAsync(u, du, sizeof(double) * np, cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaMemcpyAsync(&ev, c->evals, sizeof(ev), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaMemcpyAsync(&st, c->dstatus, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -4,6 +4,7 @@
 // stack entry of the mixed-precision walk.
 #pragma once
 #include "qv_f32x2.cuh"
+#include "qv_f64.cuh"
 #include "qv_internal.cuh"
 
 __device__ __forceinline__ double shift_of(int m, double L) {
@@ -141,3 +142,73 @@ struct __align__(16) StkEnt {
   int pad;
 };
 
+
+// ------------------------------------------------------------ FP64 walks
+// Stack entry of the FP64 walks: the child's centroid and the squared opening
+// radius, made by the lane that pushes it, so that a pop reads shared memory
+// and the distance vector serves both the opening test and the far-field term.
+struct __align__(16) StkEnt64 {
+  double cx, cy, cz;
+  // squared distance above rhi: the node is taken whole; below rlo: opened; in
+  // between (and where no radius is valid: rhi = inf, rlo = -1) the reference's
+  // expression decides
+  double rhi, rlo;
+  int node;
+  unsigned mask;
+  int child_first, nc;  // nc: children, or -1 for a one-point leaf
+  int jb, pad;
+};
+
+// Opening test theta = width / (dist - geo) < tree_theta (geo = 0 without the
+// extra correction) as dist^2 > rc2, rc = geo + width / tree_theta.  A cell's
+// centroid lies inside it, so geo <= (sqrt 3 / 2) width, and a distance below
+// geo gives width / dist >= 2 / sqrt 3: for tree_theta < 1.15 the two agree.
+// The relative margin of 1e-11 on either side is far above the rounding of
+// both (dist - geo loses at most a factor two); the reference's rounded
+// expression decides inside it, so every decision is the reference's.
+__device__ __forceinline__ void fill_ent64(StkEnt64 &E, const WNode64 &h, int node, unsigned mask,
+                                           double inv_theta, bool extra, bool sure) {
+  E.cx = h.cx; E.cy = h.cy; E.cz = h.cz;
+  const double rc = (extra ? h.geo : 0.) + h.width * inv_theta, rc2 = rc * rc;
+  E.rhi = sure ? rc2 * (1. + 1e-11) : __longlong_as_double(0x7ff0000000000000ll);
+  E.rlo = sure ? rc2 * (1. - 1e-11) : -1.;
+  E.node = node;
+  E.mask = mask;
+  E.child_first = h.child_first;
+  E.nc = h.count == 1 ? -1 : h.nchild;
+  E.jb = h.jb;
+}
+
+// Far cell (src/tree.f90:397-411): (circ x v - w) / d^3 + 3 v x (C^T v) / d^5,
+// v = x - (cent + shift), d2 = |v|^2 > 0, added to acc.
+__device__ __forceinline__ void far_term64(double v0, double v1, double v2, double d2,
+                                           const WPay64 &P, double *acc) {
+  const double r = rsqrt_pos(d2), r2 = r * r, r3 = r2 * r, t5 = 3. * r3 * r2;
+  const double z0 = fma(v0, P.C[0], fma(v1, P.C[3], v2 * P.C[6]));
+  const double z1 = fma(v0, P.C[1], fma(v1, P.C[4], v2 * P.C[7]));
+  const double z2 = fma(v0, P.C[2], fma(v1, P.C[5], v2 * P.C[8]));
+  const double cx = fma(P.a[1], v2, fma(-P.a[2], v1, -P.b[0]));
+  const double cy = fma(P.a[2], v0, fma(-P.a[0], v2, -P.b[1]));
+  const double cz = fma(P.a[0], v1, fma(-P.a[1], v0, -P.b[2]));
+  acc[0] = fma(cx, r3, fma(fma(v1, z2, -v2 * z1), t5, acc[0]));
+  acc[1] = fma(cy, r3, fma(fma(v2, z0, -v0 * z2), t5, acc[1]));
+  acc[2] = fma(cz, r3, fma(fma(v0, z1, -v1 * z0), t5, acc[2]));
+}
+
+// One-point leaf (src/tree.f90:380-390): the straight segment from R1 to R2 =
+// R1 + s, scale times its term added to acc, where the target lies off the
+// segment (R1.R2 well above 0): the form there neither cancels nor divides by
+// a small number.  false: beside or on the segment, nothing added -- the caller
+// takes the reference's expression.
+__device__ __forceinline__ bool leaf_term64(double r1x, double r1y, double r1z, double r2x,
+                                            double r2y, double r2z, double sx, double sy, double sz,
+                                            double scale, double *acc) {
+  const double d = r1x * r2x + r1y * r2y + r1z * r2z;
+  if (!(d > 0.0625 * (sx * sx + sy * sy + sz * sz))) return false;
+  const double A = r1x * r1x + r1y * r1y + r1z * r1z, B = r2x * r2x + r2y * r2y + r2z * r2z;
+  const double f = seg_f_pos(A, B, d) * scale;
+  acc[0] = fma(f, r1y * sz - r1z * sy, acc[0]);
+  acc[1] = fma(f, r1z * sx - r1x * sz, acc[1]);
+  acc[2] = fma(f, r1x * sy - r1y * sx, acc[2]);
+  return true;
+}

@@ -209,3 +209,31 @@ def test_direct_vjp_near_and_on_a_segments_line(bc):
     assert np.isfinite(g).all()
     # the near pair's 1 + cos is about 1e-3 of 1: its digits cost another 1e3
     assert np.abs(g - og).max() <= 1e-9 * np.abs(og).max()
+
+
+@pytest.mark.parametrize("bc", ["open", "openxy", "openx", "periodic"])
+@pytest.mark.parametrize("m", [1, 31, 33, 129, 700, 66000])
+def test_field_velocity_tree_at_group_and_slab_edges(m, bc):
+    """Points per warp, cells of their Morton order and points per launch at their
+    edges, points outside the box and on a filament among them.  The sums are
+    FP64 in another order than the oracle's: its far cells and leaves agree to a
+    few ulp of each term, the terms to 1e3 of the sum: 1e-12 of the largest."""
+    w = W.random_rings(4, 0.006, 0.012, 5e-4, 0.1, seed=m)
+    rng = np.random.default_rng(m)
+    pts = rng.uniform(-0.05, 0.05, (m, 3))
+    pts[::7] = rng.uniform(-0.08, 0.08, pts[::7].shape)
+    pts[::11] = w.x[rng.integers(0, w.n, len(pts[::11]))]
+    c = _ctx(w, boundary=bc, velocity="Tree", tree_theta=0.4, precision="fp64")
+    u, ev = c.field_velocity_tree(pts)
+    pick = np.arange(m) if m < 1000 else np.unique(np.r_[rng.integers(0, m, 300), 65535, 65536])
+    p = O.params(**dict(w.params, boundary=bc, velocity="Tree", tree_theta=0.4))
+    g = O.ghosts(p, w.x, w.infront, w.behind)
+    tree = O.Tree(p, w.x, g[0], w.infront)
+    ou, oev = O.field_velocity_tree(p, tree, pts[pick])
+    tree.close()
+    if m < 1000:
+        assert ev == oev
+    assert np.array_equal(np.isnan(u[pick]), np.isnan(ou))
+    ok = ~np.isnan(ou).any(axis=1)
+    if ok.any():
+        assert np.abs(u[pick] - ou)[ok].max() <= 1e-12 * np.abs(ou[ok]).max()
