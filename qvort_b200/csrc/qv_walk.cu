@@ -19,10 +19,10 @@
 // walk would visit, in the same depth-first child order, while node headers
 // are fetched once per warp (broadcast loads) instead of once per target.
 //
-// Opening decisions are always the reference's FP64 decisions: the FP64 walk
-// computes them with round-to-nearest intrinsics; the mixed walk evaluates
-// them in FP32 with a rigorous margin and falls back to the FP64 expression
-// when a decision is within that margin, so both walks visit identical nodes.
+// Opening decisions are always the reference's FP64 decisions: the walks
+// compare squared distances (the FP64 walk in FP64, the mixed walk in FP32)
+// with a rigorous margin and fall back to the reference's FP64 expression when
+// a decision is within that margin, so both walks visit identical nodes.
 //
 // The root counts every slot and carries zero circ/Cij (src/tree.f90:51-58):
 // when an image's root passes the opening test the image adds nothing, as in
@@ -33,7 +33,6 @@
 #include "qv_walk.cuh"
 
 #define WW 4                           // warps per block
-#define STK (7 * QV_MAX_DEPTH + 16)    // stack entries per warp (FP64 walk)
 #define NSPLIT 8                       // tasks per target group for the main image
 // Active points from which the mixed walk's unshifted-image tasks carry 64
 // targets, not 32.
@@ -117,20 +116,38 @@ __device__ __forceinline__ void slot_image(int bc, int s, int &ma, int &mb, int 
 }
 
 // ---------------------------------------------------------------- FP64 walk
+// Image shift of task slot sl (FP64).
+__device__ __forceinline__ void slot_shift(int bc, int sl, double L, double *s) {
+  int ma, mb, mc;
+  slot_image(bc, sl, ma, mb, mc);
+  s[0] = shift_of(ma, L); s[1] = shift_of(mb, L); s[2] = shift_of(mc, L);
+}
+
+// The reference's arithmetic: FP64 opening decisions and terms.  A pop compares
+// the squared distance with the radius made when the node was pushed
+// (StkEnt64), and the same distance vector gives the far-field term, which
+// needs one reciprocal square root; leaves off the target's own surroundings
+// likewise.  Bound: instruction issue (a third of it FP64) and dependent FP64
+// latency.  Walk of the tangle (24.7k points, 27 images, theta 0.4): 1.01 ms
+// with a square root and a division per test and eight divisions per far cell,
+// 0.53 ms now; large tangle (803k points, theta 0.5): 24 -> 12.6 ms.  Taking 2
+// or 4 nodes at a time for 16 or 8 targets ran as fast (0.55 and 0.52 ms, 13.2
+// and 13.8), but a target's sums would then depend on its group.
 template <int BC>
 __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
   constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
-  __shared__ int2 stk[WW][STK];
+  extern __shared__ StkEnt64 stk64[];
   if (a.gate && *a.gate == 0) return;
   const double rdelta = a.root_est ? a.root_est[3] : 0.;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int2 *st = stk[wid];
+  StkEnt64 *st = stk64 + wid * a.stk_cap;
+  const double ith = 1. / a.theta;
+  const bool sure = !a.extra || a.theta < 1.15;  // see fill_ent64
   const int items = a.ngroups * (NSPLIT + NIMG);
   for (int item = blockIdx.x * WW + wid; item < items; item += gridDim.x * WW) {
-    const int sl = item / a.ngroups, g = item - sl * a.ngroups;
-    int q = g * 32 + lane;
-    bool live = q < a.n_act;
-    int i = live ? a.perm[q] : 0;
+    const int sl = item / a.ngroups, q = (item - sl * a.ngroups) * 32 + lane;
+    const bool live = q < a.n_act;
+    const int i = live ? a.perm[q] : 0;
     double xi[3] = {0., 0., 0.};
     int bi = -1, fi = -1, ii = -1;
     if (live) {
@@ -138,132 +155,106 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
       bi = a.beh[i]; fi = a.inf[i]; ii = i + 1;
     }
     double acc[3] = {0., 0., 0.};
-    unsigned long long ev = 0, evf = 0;
+    unsigned ev = 0, evf = 0;  // per task: far below 2^32
     bool bad = false, runc = false;
-    int ma, mb, mc;
-    slot_image(BC, sl, ma, mb, mc);
-    const double s[3] = {shift_of(ma, a.L), shift_of(mb, a.L), shift_of(mc, a.L)};
-    int top = 0;
-    if (sl >= NSPLIT) {
-      const unsigned live_mask = __ballot_sync(0xffffffffu, live);
-      if (lane == 0) st[0] = make_int2(0, (int)live_mask);
-      top = live_mask ? 1 : 0;
-    } else {
-      // unshifted image: the root's own decision, then only root child sl
-      const WNode64 r = a.w64[0];
-      bool ropen = false;
-      if (r.count == 1) {
-        const unsigned live_mask = __ballot_sync(0xffffffffu, live);
-        if (sl == 0 && lane == 0) st[0] = make_int2(0, (int)live_mask);
-        top = (sl == 0 && live_mask) ? 1 : 0;
-      } else {
-        if (live) {
-          ropen = root_open(xi, r, s, a.theta, a.extra, rdelta, runc);
-          if (!ropen && sl == 0) { ev++; evf++; }  // root far field: zero moments
-        }
-        const unsigned om = __ballot_sync(0xffffffffu, ropen);
-        if (om && sl < r.nchild) {
-          if (lane == 0) st[0] = make_int2(r.child_first + sl, (int)om);
-          top = 1;
-        }
-      }
+    double s[3];
+    slot_shift(BC, sl, a.L, s);
+    const double t0 = xi[0] - s[0], t1 = xi[1] - s[1], t2 = xi[2] - s[2];
+    // the root's own decision; the unshifted image's tasks then take one child
+    const WNode64 r = a.w64[0];
+    const bool lone = r.count == 1;  // the root is a leaf: the first task takes it
+    bool go = live && lone && (sl == 0 || sl >= NSPLIT);
+    if (live && !lone) {
+      go = root_open(xi, r, s, a.theta, a.extra, rdelta, runc);
+      if (!go && (sl == 0 || sl >= NSPLIT)) { ev++; evf++; }  // root far field: zero moments
+    }
+    const unsigned rm = __ballot_sync(0xffffffffu, go);
+    const int c0 = sl < NSPLIT ? sl : 0, c1 = sl < NSPLIT ? min(r.nchild, sl + 1) : r.nchild;
+    int top = !rm ? 0 : lone ? 1 : max(0, c1 - c0);
+    if (lane < top) {
+      const int ch = lone ? 0 : r.child_first + c1 - 1 - lane;
+      fill_ent64(st[lane], a.w64[ch], ch, rm, ith, a.extra, sure);
     }
     __syncwarp();
     while (top > 0) {
       top--;
-      int2 e = st[top];
+      const StkEnt64 e = st[top];
+      const bool in = (e.mask >> lane) & 1u;
       __syncwarp();
-      const int node = e.x;
-      const bool in = (((unsigned)e.y) >> lane) & 1u;
-      const WNode64 h = a.w64[node];
-      if (h.count == 1) {
-        if (in) {
-          int j = h.jb;
-          if (j != ii && j != bi && j != fi) {
-            double dist = exact_dist(xi, h, s);
-            if (dist < QV_DEPS) {
-              bad = true;
-            } else {
-              const WPay64 &P = a.p64[node];
+      const double v0 = t0 - e.cx, v1 = t1 - e.cy, v2 = t2 - e.cz;
+      const double d2 = fma(v0, v0, fma(v1, v1, v2 * v2));
+      if (e.nc < 0) {
+        const int j = e.jb;
+        if (in && j != ii && j != bi && j != fi) {
+          if (d2 < 1e-28 && exact_dist(xi, a.w64[e.node], s) < QV_DEPS) {
+            bad = true;
+          } else {
+            const WPay64 &P = a.p64[e.node];
+            if (!leaf_term64(-v0, -v1, -v2, P.b[0] - t0, P.b[1] - t1, P.b[2] - t2, P.b[0] - P.a[0],
+                             P.b[1] - P.a[1], P.b[2] - P.a[2], 1., acc)) {
+              // beside the segment: the reference's expression
               double R1[3], R2[3], cr[3];
 #pragma unroll
               for (int c = 0; c < 3; c++) {
                 R1[c] = P.a[c] + s[c] - xi[c];
                 R2[c] = P.b[c] + s[c] - xi[c];
               }
-              double ra = sqrt(R1[0] * R1[0] + R1[1] * R1[1] + R1[2] * R1[2]);
-              double rb = sqrt(R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2]);
-              double cc = ra * rb * (ra * rb + (R1[0] * R2[0] + R1[1] * R2[1] + R1[2] * R2[2]));
+              const double ra = sqrt(R1[0] * R1[0] + R1[1] * R1[1] + R1[2] * R1[2]);
+              const double rb = sqrt(R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2]);
+              const double cc =
+                  ra * rb * (ra * rb + (R1[0] * R2[0] + R1[1] * R2[1] + R1[2] * R2[2]));
               cross3(R1, R2, cr);
-              double f = (ra + rb) / cc;
+              const double f = (ra + rb) / cc;
 #pragma unroll
               for (int c = 0; c < 3; c++) acc[c] += f * cr[c];
-              ev++;
             }
-          }
-        }
-      } else {
-        bool open = false;
-        if (in) {
-          double dist = exact_dist(xi, h, s);
-          if (node == 0 ? root_open(xi, h, s, a.theta, a.extra, rdelta, runc)
-                        : exact_open(dist, h, a.theta, a.extra)) {
-            open = true;
-          } else {
             ev++;
-            evf++;
-            if (node != 0) {
-              const WPay64 &P = a.p64[node];
-              double v[3] = {__dsub_rn(xi[0], __dadd_rn(h.cx, s[0])),
-                             __dsub_rn(xi[1], __dadd_rn(h.cy, s[1])),
-                             __dsub_rn(xi[2], __dadd_rn(h.cz, s[2]))};
-              double d2 = dist * dist, d3 = d2 * dist, d5 = d2 * d2 * dist;
-              double cv[3], z[3], vz[3];
-              cross3(P.a, v, cv);
-#pragma unroll
-              for (int l = 0; l < 3; l++) z[l] = v[0] * P.C[l] + v[1] * P.C[3 + l] + v[2] * P.C[6 + l];
-              cross3(v, z, vz);
-#pragma unroll
-              for (int c = 0; c < 3; c++) acc[c] += (cv[c] - P.b[c]) / d3 + 3. * vz[c] / d5;
-            }
           }
         }
-        unsigned om = __ballot_sync(0xffffffffu, open);
-        if (om) {
-          int nc = h.nchild;
-          if (top + nc > STK) {  // unreachable for trees within QV_MAX_DEPTH
-            bad = true;
-            nc = 0;
-          }
-          if (lane < nc) st[top + lane] = make_int2(h.child_first + nc - 1 - lane, (int)om);
-          top += nc;
-        }
-        __syncwarp();
+        continue;
       }
+      bool far = in && d2 > e.rhi, open = in && d2 < e.rlo;
+      if (in && !(far || open)) {
+        const WNode64 h = a.w64[e.node];
+        open = exact_open(exact_dist(xi, h, s), h, a.theta, a.extra);
+        far = !open;
+      }
+      if (far) {
+        far_term64(v0, v1, v2, d2, a.p64[e.node], acc);
+        ev++;
+        evf++;
+      }
+      const unsigned om = __ballot_sync(0xffffffffu, open);
+      if (om) {
+        int nc = e.nc;
+        if (top + nc > a.stk_cap) {  // unreachable: the cap follows the tree depth
+          bad = true;
+          nc = 0;
+        }
+        if (lane < nc) {
+          const int ch = e.child_first + nc - 1 - lane;
+          fill_ent64(st[top + lane], a.w64[ch], ch, om, ith, a.extra, sure);
+        }
+        top += nc;
+      }
+      __syncwarp();
     }
     if (live) {
       double *o = a.part + ((size_t)sl * a.n_act + q) * 3;
       o[0] = acc[0]; o[1] = acc[1]; o[2] = acc[2];
     }
-    if (runc) note_undecided(a, q, sl, (unsigned)ev, (unsigned)evf);
+    if (runc) note_undecided(a, q, sl, ev, evf);
     for (int o = 16; o > 0; o >>= 1) {
       ev += __shfl_down_sync(0xffffffffu, ev, o);
       evf += __shfl_down_sync(0xffffffffu, evf, o);
     }
-    if (lane == 0 && ev) atomicAdd(a.evals, ev);
-    if (lane == 0 && evf) atomicAdd(a.evals_far, evf);
+    if (lane == 0 && ev) atomicAdd(a.evals, (unsigned long long)ev);
+    if (lane == 0 && evf) atomicAdd(a.evals_far, (unsigned long long)evf);
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.status, QV_STAT_SINGULAR);
   }
 }
 
 // ---------------------------------------------------------------- mixed walk
-// Image shift of task slot sl (FP64), for the rare exact tests.
-__device__ __forceinline__ void slot_shift(int bc, int sl, double L, double *s) {
-  int ma, mb, mc;
-  slot_image(bc, sl, ma, mb, mc);
-  s[0] = shift_of(ma, L); s[1] = shift_of(mb, L); s[2] = shift_of(mc, L);
-}
-
 // One target of a lane's pair: its point index and links.
 struct PairTarget {
   int i, bi, fi;  // point index (0-based), behind, infront; bi = fi = -1 if not live
@@ -820,8 +811,9 @@ __device__ __forceinline__ void walk32_body(const WalkArgs &a) {
 // The walks, and the same walks under a second name for the gated relaunch
 // after an overflowing root fix-up (it returns at once unless flagged), so
 // that a profile tells the two launches apart.
+// 5 blocks/SM: 0.53 ms on the tangle (unbounded 0.57, 8 0.59)
 template <int BC>
-__global__ void __launch_bounds__(WW * 32) k_walk64(WalkArgs a) { walk64_body<BC>(a); }
+__global__ void __launch_bounds__(WW * 32, 5) k_walk64(WalkArgs a) { walk64_body<BC>(a); }
 template <int BC>
 __global__ void __launch_bounds__(WW * 32) k_walk64_redo(WalkArgs a) { walk64_body<BC>(a); }
 // 5 blocks/SM (96 registers): faster than 4 (111 registers) on the paired tasks
@@ -985,7 +977,7 @@ int qv_launch_walk(qv_ctx *c) {
   // a depth-first stack over a tree of depth D never holds more than 7 D + 1
   // entries (each open pushes at most 8 and pops 1)
   a.stk_cap = 7 * (t.depth + 1) + 8;
-  size_t smem = sizeof(StkEnt) * a.stk_cap * WW;
+  size_t smem = (mixed ? sizeof(StkEnt) : sizeof(StkEnt64)) * a.stk_cap * WW;
   const long nnear = (long)NSPLIT * (a.pair_near ? a.ng64 : a.ngroups);
   const long items = mixed ? nnear + (long)a.ng64 * nimg : (long)a.ngroups * (NSPLIT + nimg);
   const bool dynamic = mixed && (t.n_act >= QV_WALK_DYNAMIC || l1);
@@ -1008,14 +1000,21 @@ int qv_launch_walk(qv_ctx *c) {
     QV_CUDA(c, cudaMemsetAsync(c->walk_next, 0, 4 * sizeof(int), c->stream));
     a.next = c->walk_next;
   }
-  if (mixed && smem > 48 * 1024) {
+  static_assert(sizeof(StkEnt) == sizeof(StkEnt64), "one opt-in serves both walks");
+  if (smem > 48 * 1024) {
     if (smem > c->smem_walk) {  // per context: attributes are per device
       const void *fs[] = {(const void *)k_walk32<QV_BC_OPEN>, (const void *)k_walk32<QV_BC_PERIODIC>,
                           (const void *)k_walk32<QV_BC_OPENX>, (const void *)k_walk32<QV_BC_OPENXY>,
                           (const void *)k_walk32_redo<QV_BC_OPEN>,
                           (const void *)k_walk32_redo<QV_BC_PERIODIC>,
                           (const void *)k_walk32_redo<QV_BC_OPENX>,
-                          (const void *)k_walk32_redo<QV_BC_OPENXY>};
+                          (const void *)k_walk32_redo<QV_BC_OPENXY>,
+                          (const void *)k_walk64<QV_BC_OPEN>, (const void *)k_walk64<QV_BC_PERIODIC>,
+                          (const void *)k_walk64<QV_BC_OPENX>, (const void *)k_walk64<QV_BC_OPENXY>,
+                          (const void *)k_walk64_redo<QV_BC_OPEN>,
+                          (const void *)k_walk64_redo<QV_BC_PERIODIC>,
+                          (const void *)k_walk64_redo<QV_BC_OPENX>,
+                          (const void *)k_walk64_redo<QV_BC_OPENXY>};
       for (const void *f : fs)
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       c->smem_walk = smem;
@@ -1028,8 +1027,8 @@ int qv_launch_walk(qv_ctx *c) {
   case BCV:                                                                \
     if (mixed && redo) k_walk32_redo<BCV><<<grid, WW * 32, smem, st>>>(w); \
     else if (mixed) k_walk32<BCV><<<grid, WW * 32, smem, st>>>(w);        \
-    else if (redo) k_walk64_redo<BCV><<<grid, WW * 32, 0, st>>>(w);       \
-    else k_walk64<BCV><<<grid, WW * 32, 0, st>>>(w);                      \
+    else if (redo) k_walk64_redo<BCV><<<grid, WW * 32, smem, st>>>(w);    \
+    else k_walk64<BCV><<<grid, WW * 32, smem, st>>>(w);                   \
     break;
       QV_WALK_CASE(QV_BC_OPEN)
       QV_WALK_CASE(QV_BC_PERIODIC)
