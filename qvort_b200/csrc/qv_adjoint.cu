@@ -40,6 +40,7 @@
 #include "qv_ab.cuh"
 #include "qv_f64.cuh"
 #include "qv_lia.cuh"
+#include "qv_walk.cuh"
 
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
@@ -237,186 +238,227 @@ __global__ void k_dvjp_reduce(int na, const int *__restrict__ act, int t_lo, int
 }
 
 // ------------------------------------------------------------ tree walk
+// The velocity walk again, with the opened cells held: one node at a time for 32
+// targets.  A node's adjoint (cent, circ, C: 15 values) is the sum over its
+// targets: a halving butterfly (16 exchanges where summing each value on its
+// own took 75) leaves the sums spread over the lanes, which add them to the
+// node's record (128 bytes) with one atomic instruction.  The opening test and
+// the far-field gradient need one reciprocal square root, as in the velocity
+// walk.
+//
+// Bound: instruction issue (36 % of it FP64).  50,000 points, 27 images, theta
+// 0.4: 2.28 ms with a rounded square root and division per test, 15 separate
+// warp sums and 15 atomics by one lane per node; 0.97 ms now.  Two or four
+// nodes at a time for 16 or 8 targets send two to four times the atomics,
+// which then meet on the top nodes' L2 lines (1.2 and 3.5 ms; 1.0 and 1.15 with
+// 16 copies of those nodes' records).
 #define AW 4
-#define ASTK (7 * QV_MAX_DEPTH + 16)
 #define ANSPLIT 8
+#define NBS 16  // doubles per node adjoint record: cent 3, circ 3, C 9, unused
 
 struct WalkVjpArgs {
-  int n_act, ngroups;
+  int n_act, ngroups, stk_cap;
   const int *perm, *inf, *beh;
   const double *x, *ubar;
   const WNode64 *w64;
   const WPay64 *p64;
-  const int *first;
   double L, theta, gfac;
   int extra;
-  double *xb, *gib, *nb;  // nb: per-node adjoint of (cent, circ, C) = 15 doubles
+  double *xb, *gib, *nb;  // nb: per-node adjoints (NBS doubles each)
 };
 
-__device__ __forceinline__ double sh_of(int m, double L) { return m == 0 ? 0. : (m > 0 ? L : -L); }
-
-__device__ __forceinline__ double wsum(double v, unsigned mask) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-  return v;
+// Sums the NV values of v (16 or 8) over the warp by halving: v[0] of lane l
+// becomes the sum of value l / (32 / NV).
+template <int NV>
+__device__ __forceinline__ void warp_sums(double *v, int lane) {
+  int n = NV;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < NV / 2; k++) {
+        if (k >= n) break;
+        const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
 }
 
-__device__ __forceinline__ bool open_exact(const double *xi, const WNode64 &h, const double *s,
-                                           double theta, int extra, double &dist) {
-  double d0 = __dsub_rn(xi[0], __dadd_rn(h.cx, s[0]));
-  double d1 = __dsub_rn(xi[1], __dadd_rn(h.cy, s[1]));
-  double d2 = __dsub_rn(xi[2], __dadd_rn(h.cz, s[2]));
-  dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2)));
-  double th;
-  if (extra) {
-    double r = __dsub_rn(dist, h.geo);
-    th = r > 0. ? __ddiv_rn(h.width, r) : __ddiv_rn(h.width, dist);
-  } else {
-    th = __ddiv_rn(h.width, dist);
+// Gradients of g . f (R x s) for a straight segment off the target (d = R.(R +
+// s) > 0): dR at fixed s, dS at fixed R (see Seg64::gradient).
+__device__ __forceinline__ void seg_gradient_pos(const double *R, const double *s, const double *g,
+                                                 double A, double B, double d, double *dR,
+                                                 double *dS) {
+  const SegD t = seg_d_pos(A, B, d);
+  const double h[3] = {s[1] * g[2] - s[2] * g[1], s[2] * g[0] - s[0] * g[2],
+                       s[0] * g[1] - s[1] * g[0]};
+  const double gr[3] = {g[1] * R[2] - g[2] * R[1], g[2] * R[0] - g[0] * R[2],
+                        g[0] * R[1] - g[1] * R[0]};
+  const double Q = R[0] * h[0] + R[1] * h[1] + R[2] * h[2];
+  const double al = 2. * Q * t.fA, be = Q * t.fw, ga = Q * t.fc2;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    dR[c] = fma(t.f, h[c], fma(al, R[c], be * s[c]));
+    dS[c] = fma(t.f, gr[c], fma(be, R[c], ga * s[c]));
   }
-  return !(th < theta);
 }
 
 template <int BC>
-__global__ void __launch_bounds__(AW * 32, 5) k_walk_vjp(WalkVjpArgs a) {
+__global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
   constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
-  __shared__ int2 stk[AW][ASTK];
+  extern __shared__ int2 stk_adj[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int2 *st = stk[wid];
+  int2 *st = stk_adj + wid * a.stk_cap;
+  const double ith = 1. / a.theta;
+  const bool sure = !a.extra || a.theta < 1.15;
   const int items = a.ngroups * (ANSPLIT + NIMG);
   for (int item = blockIdx.x * AW + wid; item < items; item += gridDim.x * AW) {
-    const int sl = item / a.ngroups, gg = item - sl * a.ngroups;
-    int q = gg * 32 + lane;
-    bool live = q < a.n_act;
-    int i = live ? a.perm[q] : 0;
-    double xi[3] = {0., 0., 0.}, g[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
+    const int sl = item / a.ngroups, q = (item - sl * a.ngroups) * 32 + lane;
+    const bool live = q < a.n_act;
+    const int i = live ? a.perm[q] : 0;
+    double xi[3] = {0., 0., 0.}, gu[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
     int bi = -1, fi = -1, ii = -1;
     if (live) {
-      for (int c = 0; c < 3; c++) { xi[c] = a.x[3 * i + c]; g[c] = a.gfac * a.ubar[3 * i + c]; }
+#pragma unroll
+      for (int c = 0; c < 3; c++) { xi[c] = a.x[3 * i + c]; gu[c] = a.gfac * a.ubar[3 * i + c]; }
       bi = a.beh[i]; fi = a.inf[i]; ii = i + 1;
     }
     int ma = 0, mb = 0, mc = 0;
     if (sl >= ANSPLIT) qv_img_shift(BC, sl - ANSPLIT, &ma, &mb, &mc);
-    const double s[3] = {sh_of(ma, a.L), sh_of(mb, a.L), sh_of(mc, a.L)};
-    int top = 0;
-    if (sl >= ANSPLIT) {
-      const unsigned lm = __ballot_sync(0xffffffffu, live);
-      if (lane == 0) st[0] = make_int2(0, (int)lm);
-      top = lm ? 1 : 0;
-    } else {
-      const WNode64 r = a.w64[0];
-      if (r.count == 1) {
-        const unsigned lm = __ballot_sync(0xffffffffu, live);
-        if (sl == 0 && lane == 0) st[0] = make_int2(0, (int)lm);
-        top = (sl == 0 && lm) ? 1 : 0;
-      } else {
-        bool ropen = false;
-        double dd;
-        if (live) ropen = open_exact(xi, r, s, a.theta, a.extra, dd);
-        const unsigned om = __ballot_sync(0xffffffffu, ropen);
-        if (om && sl < r.nchild) {
-          if (lane == 0) st[0] = make_int2(r.child_first + sl, (int)om);
-          top = 1;
-        }
-      }
-    }
+    const double s[3] = {shift_of(ma, a.L), shift_of(mb, a.L), shift_of(mc, a.L)};
+    const double t0 = xi[0] - s[0], t1 = xi[1] - s[1], t2 = xi[2] - s[2];
+    // the root's own decision; the unshifted image's tasks then take one child
+    const WNode64 r = a.w64[0];
+    const bool lone = r.count == 1;
+    const bool go = live && (lone ? sl == 0 || sl >= ANSPLIT
+                                  : exact_open(exact_dist(xi, r, s), r, a.theta, a.extra));
+    const unsigned rm = __ballot_sync(0xffffffffu, go);
+    const int c0 = lone ? 0 : r.child_first + (sl < ANSPLIT ? sl : 0);
+    const int c1 = lone ? 1 : r.child_first + (sl < ANSPLIT ? min(r.nchild, sl + 1) : r.nchild);
+    int top = rm ? max(0, c1 - c0) : 0;
+    if (lane < top) st[lane] = make_int2(c0 + lane, (int)rm);
     __syncwarp();
     while (top > 0) {
       top--;
-      int2 e = st[top];
+      const int2 e = st[top];
       __syncwarp();
       const int node = e.x;
       const bool in = (((unsigned)e.y) >> lane) & 1u;
       const WNode64 h = a.w64[node];
-      if (h.count == 1) {
-        bool ev = false;
-        double gR1[3] = {0., 0., 0.}, gR2[3] = {0., 0., 0.};
-        if (in) {
-          int j = h.jb;
-          if (j != ii && j != bi && j != fi) {
-            const WPay64 &P = a.p64[node];
-            double R1[3], R2[3];
+      const double v[3] = {t0 - h.cx, t1 - h.cy, t2 - h.cz};
+      const double d2 = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));
+      bool open = false, far = false, leaf = false;
+      double w[16];
+      const WPay64 &P = a.p64[node];
+      if (in && h.count == 1) {
+        const int j = h.jb;
+        leaf = j != ii && j != bi && j != fi;
+      } else if (in) {
+        const double rc = fma(h.width, ith, a.extra ? h.geo : 0.), rc2 = rc * rc;
+        // node_test as in the velocity walk: the reference's expression near rc
+        open = !sure || !(fabs(d2 - rc2) > 1e-11 * rc2)
+                   ? exact_open(exact_dist(xi, h, s), h, a.theta, a.extra)
+                   : d2 < rc2;
+        far = !open && node != 0;
+      }
+      if (__any_sync(0xffffffffu, leaf)) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) w[k] = 0.;
+        if (leaf) {
+          double dR[3], dS[3];
+          const double R[3] = {-v[0], -v[1], -v[2]};
+          double sv[3], R2[3];
+#pragma unroll
+          for (int c = 0; c < 3; c++) sv[c] = P.b[c] - P.a[c];
+          R2[0] = P.b[0] - t0; R2[1] = P.b[1] - t1; R2[2] = P.b[2] - t2;
+          const double d = R[0] * R2[0] + R[1] * R2[1] + R[2] * R2[2];
+          if (d > 0.0625 * (sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2])) {
+            seg_gradient_pos(R, sv, gu, d2, R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2], d, dR,
+                             dS);
+          } else {  // beside the segment
+            double g1[3], E1[3], E2[3];
+#pragma unroll
             for (int c = 0; c < 3; c++) {
-              R1[c] = P.a[c] + s[c] - xi[c];
-              R2[c] = P.b[c] + s[c] - xi[c];
+              E1[c] = P.a[c] + s[c] - xi[c];
+              E2[c] = P.b[c] + s[c] - xi[c];
             }
-            seg_grad(R1, R2, g, gR1, gR2);
-            for (int c = 0; c < 3; c++) acc[c] -= gR1[c] + gR2[c];
-            ev = true;
+            seg_grad(E1, E2, gu, g1, dS);
+#pragma unroll
+            for (int c = 0; c < 3; c++) dR[c] = g1[c] + dS[c];
+          }
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            acc[c] -= dR[c];
+            w[c] = dR[c] - dS[c];
+            w[3 + c] = dS[c];
           }
         }
-        if (__any_sync(0xffffffffu, ev)) {
-          double v[6];
-          for (int c = 0; c < 3; c++) { v[c] = wsum(gR1[c], 0xffffffffu); v[3 + c] = wsum(gR2[c], 0xffffffffu); }
-          if (lane == 0) {
-            int p = a.first[node];
-            for (int c = 0; c < 3; c++) {
-              atomicAdd(&a.xb[3 * p + c], v[c]);
-              atomicAdd(&a.gib[3 * p + c], v[3 + c]);
-            }
+        warp_sums<8>(w, lane);
+        const int m = lane >> 2;  // the value this lane holds
+        if ((lane & 3) == 0 && m < 6) atomicAdd(&(m < 3 ? a.xb : a.gib)[3 * h.first + m % 3], w[0]);
+        continue;
+      }
+      if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) w[k] = 0.;
+        if (far) {
+          const double r1 = rsqrt_pos(d2), r2 = r1 * r1, r3 = r2 * r1, r5 = r3 * r2;
+          const double p5 = 3. * r5;
+          double z[3], av[3], bv[3];
+#pragma unroll
+          for (int l = 0; l < 3; l++) z[l] = fma(v[0], P.C[l], fma(v[1], P.C[3 + l], v[2] * P.C[6 + l]));
+          av[0] = fma(P.a[1], v[2], fma(-P.a[2], v[1], -P.b[0]));
+          av[1] = fma(P.a[2], v[0], fma(-P.a[0], v[2], -P.b[1]));
+          av[2] = fma(P.a[0], v[1], fma(-P.a[1], v[0], -P.b[2]));
+          cross3(v, z, bv);
+          const double ga = gu[0] * av[0] + gu[1] * av[1] + gu[2] * av[2];
+          const double gb = gu[0] * bv[0] + gu[1] * bv[1] + gu[2] * bv[2];
+          double gxc[3], zxg[3], gxv[3];
+          cross3(gu, P.a, gxc);
+          cross3(z, gu, zxg);
+          cross3(gu, v, gxv);
+          const double kv = -p5 * fma(5. * r2, gb, ga);
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            const double Cg = fma(P.C[3 * c], gxv[0], fma(P.C[3 * c + 1], gxv[1], P.C[3 * c + 2] * gxv[2]));
+            const double gv = fma(kv, v[c], fma(r3, gxc[c], p5 * (zxg[c] + Cg)));
+            acc[c] += gv;
+            w[c] = -gv;               // cent
+            w[3 + c] = -r3 * gxv[c];  // circ: r3 v x g
           }
+          // C(p, l): v_p (3 r5 g x v)_l, and w_0 = C12 - C21, w_1 = C20 - C02,
+          // w_2 = C01 - C10 with adjoint -r3 g
+          const double zb[3] = {p5 * gxv[0], p5 * gxv[1], p5 * gxv[2]};
+          const double wb[3] = {-r3 * gu[0], -r3 * gu[1], -r3 * gu[2]};
+          w[6] = v[0] * zb[0];
+          w[7] = fma(v[0], zb[1], wb[2]);
+          w[8] = fma(v[0], zb[2], -wb[1]);
+          w[9] = fma(v[1], zb[0], -wb[2]);
+          w[10] = v[1] * zb[1];
+          w[11] = fma(v[1], zb[2], wb[0]);
+          w[12] = fma(v[2], zb[0], wb[1]);
+          w[13] = fma(v[2], zb[1], -wb[0]);
+          w[14] = v[2] * zb[2];
         }
-      } else {
-        bool open = false, far = false;
-        double nbv[15];
-        for (int k = 0; k < 15; k++) nbv[k] = 0.;
-        if (in) {
-          double dist;
-          open = open_exact(xi, h, s, a.theta, a.extra, dist);
-          if (!open && node != 0) {
-            far = true;
-            const WPay64 &P = a.p64[node];
-            double v[3] = {xi[0] - (h.cx + s[0]), xi[1] - (h.cy + s[1]), xi[2] - (h.cz + s[2])};
-            double d2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-            double r1 = 1. / sqrt(d2);
-            double r3 = r1 * r1 * r1, r5 = r3 / d2, r7 = r5 / d2;
-            double z[3];
-            for (int l = 0; l < 3; l++) z[l] = v[0] * P.C[l] + v[1] * P.C[3 + l] + v[2] * P.C[6 + l];
-            double av[3] = {P.a[1] * v[2] - P.a[2] * v[1] - P.b[0], P.a[2] * v[0] - P.a[0] * v[2] - P.b[1],
-                            P.a[0] * v[1] - P.a[1] * v[0] - P.b[2]};
-            double bv[3] = {v[1] * z[2] - v[2] * z[1], v[2] * z[0] - v[0] * z[2], v[0] * z[1] - v[1] * z[0]};
-            double ga = g[0] * av[0] + g[1] * av[1] + g[2] * av[2];
-            double gb = g[0] * bv[0] + g[1] * bv[1] + g[2] * bv[2];
-            double gxc[3] = {g[1] * P.a[2] - g[2] * P.a[1], g[2] * P.a[0] - g[0] * P.a[2],
-                             g[0] * P.a[1] - g[1] * P.a[0]};
-            double zxg[3] = {z[1] * g[2] - z[2] * g[1], z[2] * g[0] - z[0] * g[2], z[0] * g[1] - z[1] * g[0]};
-            double gxv[3] = {g[1] * v[2] - g[2] * v[1], g[2] * v[0] - g[0] * v[2], g[0] * v[1] - g[1] * v[0]};
-            double Cg[3];
-            for (int p = 0; p < 3; p++) Cg[p] = P.C[3 * p] * gxv[0] + P.C[3 * p + 1] * gxv[1] + P.C[3 * p + 2] * gxv[2];
-            double gv[3];
-            for (int c = 0; c < 3; c++)
-              gv[c] = -3. * r5 * ga * v[c] + r3 * gxc[c] - 15. * r7 * gb * v[c] + 3. * r5 * (zxg[c] + Cg[c]);
-            for (int c = 0; c < 3; c++) acc[c] += gv[c];
-            // node adjoint: cent (0-2), circ (3-5), C row-major (6-14)
-            for (int c = 0; c < 3; c++) nbv[c] = -gv[c];
-            double vxg[3] = {v[1] * g[2] - v[2] * g[1], v[2] * g[0] - v[0] * g[2], v[0] * g[1] - v[1] * g[0]};
-            for (int c = 0; c < 3; c++) nbv[3 + c] = r3 * vxg[c];
-            double zb[3] = {3. * r5 * gxv[0], 3. * r5 * gxv[1], 3. * r5 * gxv[2]};
-            for (int p = 0; p < 3; p++)
-              for (int l = 0; l < 3; l++) nbv[6 + 3 * p + l] = v[p] * zb[l];
-            double wb[3] = {-r3 * g[0], -r3 * g[1], -r3 * g[2]};
-            // w_0 = C12 - C21, w_1 = C20 - C02, w_2 = C01 - C10
-            nbv[6 + 5] += wb[0]; nbv[6 + 7] -= wb[0];
-            nbv[6 + 6] += wb[1]; nbv[6 + 2] -= wb[1];
-            nbv[6 + 1] += wb[2]; nbv[6 + 3] -= wb[2];
-          }
-        }
-        if (__any_sync(0xffffffffu, far)) {
-          for (int k = 0; k < 15; k++) {
-            double t = wsum(nbv[k], 0xffffffffu);
-            if (lane == 0) atomicAdd(&a.nb[15 * node + k], t);
-          }
-        }
-        unsigned om = __ballot_sync(0xffffffffu, open);
-        if (om) {
-          int nc = h.nchild;
-          if (top + nc > ASTK) nc = 0;  // unreachable within QV_MAX_DEPTH
-          if (lane < nc) st[top + lane] = make_int2(h.child_first + nc - 1 - lane, (int)om);
-          top += nc;
-        }
+        warp_sums<16>(w, lane);
+        if (!(lane & 1) && lane < 30) atomicAdd(a.nb + NBS * (size_t)node + (lane >> 1), w[0]);
+      }
+      const unsigned om = __ballot_sync(0xffffffffu, open);
+      if (om) {
+        int nc = h.nchild;
+        if (top + nc > a.stk_cap) nc = 0;  // unreachable: the cap follows the tree depth
+        if (lane < nc) st[top + lane] = make_int2(h.child_first + nc - 1 - lane, (int)om);
+        top += nc;
         __syncwarp();
       }
     }
     if (live)
+#pragma unroll
       for (int c = 0; c < 3; c++) atomicAdd(&a.xb[3 * i + c], acc[c]);
   }
 }
@@ -432,7 +474,7 @@ __global__ void k_moment_vjp(int n_nodes, const int *__restrict__ level,
   int lane = threadIdx.x & 31;
   int k = 1 + (blockIdx.x * blockDim.x + threadIdx.x) / 32;
   if (k >= n_nodes) return;
-  const double *B = nb + 15 * k;
+  const double *B = nb + NBS * (size_t)k;
   double Cb[9], cb[3], qb[3];
   bool any = false;
   for (int t = 0; t < 15; t++) any |= B[t] != 0.;
@@ -830,7 +872,7 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
       if ((rc = qv_launch_tree_build(c))) return rc;
     if ((rc = qv_tree_finalize_root(c))) return rc;
     TreeBuf &t = c->tree;
-    size_t nbytes = sizeof(double) * 15 * (size_t)t.n_nodes;
+    size_t nbytes = sizeof(double) * NBS * (size_t)t.n_nodes;
     if (nbytes > c->adj_nb_bytes) {
       if ((rc = qv_grow(c, (void **)&c->adj_nb, nbytes))) return rc;
       c->adj_nb_bytes = nbytes;
@@ -838,20 +880,27 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
     QV_CUDA(c, cudaMemsetAsync(c->adj_nb, 0, nbytes, c->stream));
     if (t.n_act > 0) {
       WalkVjpArgs a;
-      a.n_act = t.n_act; a.ngroups = (t.n_act + 31) / 32; a.perm = t.perm; a.inf = c->infront;
-      a.beh = c->behind; a.x = c->x; a.ubar = ubar; a.w64 = t.w64; a.p64 = t.p64; a.first = t.first;
+      a.n_act = t.n_act; a.ngroups = (t.n_act + 31) / 32; a.perm = t.perm;
+      a.inf = c->infront; a.beh = c->behind; a.x = c->x; a.ubar = ubar; a.w64 = t.w64; a.p64 = t.p64;
       a.L = p.box_size; a.theta = p.tree_theta; a.gfac = gfac; a.extra = p.tree_extra_correction;
       a.xb = c->adj_xb; a.gib = c->adj_gib; a.nb = c->adj_nb;
+      a.stk_cap = 7 * (t.depth + 1) + 8;  // as in the velocity walk
+      const size_t smem = sizeof(int2) * a.stk_cap * AW;
       int nimg = qv_img_count(p.boundary);
       long items = (long)a.ngroups * (ANSPLIT + nimg);
       int nb = (int)std::min<long>((items + AW - 1) / AW, 64L * c->sm_count);
+      const void *f = nullptr;
       switch (p.boundary) {
-        case QV_BC_OPEN: k_walk_vjp<QV_BC_OPEN><<<nb, AW * 32, 0, c->stream>>>(a); break;
-        case QV_BC_PERIODIC: k_walk_vjp<QV_BC_PERIODIC><<<nb, AW * 32, 0, c->stream>>>(a); break;
-        case QV_BC_OPENX: k_walk_vjp<QV_BC_OPENX><<<nb, AW * 32, 0, c->stream>>>(a); break;
-        case QV_BC_OPENXY: k_walk_vjp<QV_BC_OPENXY><<<nb, AW * 32, 0, c->stream>>>(a); break;
+        case QV_BC_OPEN: f = (const void *)k_walk_vjp<QV_BC_OPEN>; break;
+        case QV_BC_PERIODIC: f = (const void *)k_walk_vjp<QV_BC_PERIODIC>; break;
+        case QV_BC_OPENX: f = (const void *)k_walk_vjp<QV_BC_OPENX>; break;
+        case QV_BC_OPENXY: f = (const void *)k_walk_vjp<QV_BC_OPENXY>; break;
         default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", p.boundary);
       }
+      if (smem > 48 * 1024)
+        QV_CUDA(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      void *args[] = {&a};
+      QV_CUDA(c, cudaLaunchKernel(f, dim3(nb), dim3(AW * 32), args, smem, c->stream));
       QV_LAUNCH_CHECK(c);
       if (t.n_nodes > 1) {
         k_moment_vjp<<<nblk((long)(t.n_nodes - 1) * 32, 256), 256, 0, c->stream>>>(

@@ -237,3 +237,29 @@ def test_field_velocity_tree_at_group_and_slab_edges(m, bc):
     ok = ~np.isnan(ou).any(axis=1)
     if ok.any():
         assert np.abs(u[pick] - ou)[ok].max() <= 1e-12 * np.abs(ou[ok]).max()
+
+
+@pytest.mark.parametrize("bc", ["open", "openxy", "openx", "periodic"])
+@pytest.mark.parametrize("n", [5, 31, 33, 64, 129, 260])
+def test_tree_velocity_and_vjp_at_group_edges(n, bc):
+    """FP64 Barnes-Hut velocity and its gradient with the opened cells held, at
+    the edges of the walks' target groups, against torch autograd over the same
+    cells (perf/cases.py): both in FP64, 1e-11 of the largest as above."""
+    import torch
+
+    from perf import cases as P
+    from qvort_b200 import adjoint as A
+    from qvort_b200 import lib as L
+
+    w = _ring_pair(n)
+    w.params = dict(w.params, boundary=bc, velocity="Tree", tree_theta=0.45, precision="fp64",
+                    deriv_order=2)
+    ubar = np.random.default_rng(n).normal(0.0, 0.1, w.x.shape)
+    ou, og = (t.detach().cpu().numpy() for t in P._tree_u(w, torch.tensor(ubar, device=P._dev())))
+    s = A.FilamentSystem(L.default_params(**w.params), w.infront, w.behind)
+    x = torch.tensor(w.x, device="cuda", requires_grad=True)
+    u = A.velocity(x, s)
+    (g,) = torch.autograd.grad(u, x, torch.tensor(ubar, device="cuda"))
+    s.close()
+    assert np.abs(u.detach().cpu().numpy() - ou).max() <= 1e-11 * np.abs(ou).max()
+    assert np.abs(g.cpu().numpy() - og).max() <= 1e-11 * np.abs(og).max()
