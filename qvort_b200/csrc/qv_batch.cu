@@ -466,8 +466,10 @@ struct qv_batch {
   std::vector<int4> items, items_cost;  // natural and cost-descending orders
   int cap_nodes = 0, stk_cap = 0, depth = 0;
   bool points_set = false;
-  // launch configuration of the work kernel (qv_batch_tune)
-  int wpb = 4, bps = 2, order = 1;
+  // launch configuration of the work kernel: default_shape's, until qv_batch_tune
+  // or qv_batch_set_config fixes another (shape_fixed)
+  int wpb = 4, bps = 1, order = 0;
+  bool shape_fixed = false;
   cudaGraphExec_t gexec = nullptr;
   bool graph_tried = false, graph_ok = false;
   long long steps_done = 0;
@@ -665,7 +667,7 @@ extern "C" int qv_batch_create(const qv_params *p, int nsys, const int *offsets,
       (rc = upload(c, &b->d_dsrc, dsrc)) || (rc = upload(c, &b->d_dt, b->dt)) ||
       (rc = upload(c, &b->d_dact, dact)) || (rc = upload(c, &b->d_fact, fact)) ||
       (rc = upload(c, &b->d_froot, froot)) || (rc = upload(c, &b->d_roots, roots)) ||
-      (rc = upload(c, &b->d_groups, groups)) || (rc = upload(c, &b->d_items, b->items_cost)) ||
+      (rc = upload(c, &b->d_groups, groups)) || (rc = upload(c, &b->d_items, b->items)) ||
       (rc = upload(c, &b->d_nfact, one))) {
     free_batch_tables(b);
     qv_destroy(c);
@@ -704,13 +706,33 @@ extern "C" void qv_batch_destroy(qv_batch *b) {
 
 extern "C" const char *qv_batch_last_error(qv_batch *b) { return b ? b->c->err : "null batch"; }
 
+// The launch shape of a batch that nothing has tuned: four warps per block, as
+// many blocks per SM as are resident at once, up to six, while every warp finds
+// an item; items in their natural order (neighbouring groups share their nodes
+// in L1).  Two blocks per SM, largest items first, the shape before, left
+// the walks' latency uncovered: 512 systems (924k points) 7.40 ms a step, 3.92
+// with six; 64 systems (68k points) 0.67 and 0.46; 16 systems with 203 items
+// in all 0.195, and 0.19 with one.
+static int default_shape(qv_batch *b) {
+  if (b->shape_fixed) return QV_OK;
+  qv_ctx *c = b->c;
+  int per = 0;
+  QV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step, b->wpb * 32,
+                                                           work_smem_per_warp(b) * b->wpb));
+  const int want = nblk((long)b->items.size(), b->wpb * c->sm_count);
+  const int bps = std::max(1, std::min({per, 6, want}));
+  if (bps != b->bps) drop_graph(b);
+  b->bps = bps;
+  return QV_OK;
+}
+
 // Tree depth of the current positions (an eager build read back on the host)
 // and the walk stack that covers it with four levels to spare.
 static int size_stack(qv_batch *b) {
   qv_ctx *c = b->c;
   if (b->nroots == 0) {
     b->stk_cap = 8;
-    return QV_OK;
+    return default_shape(b);
   }
   int rc;
   for (int attempt = 0; attempt < 8; attempt++) {
@@ -740,7 +762,7 @@ static int size_stack(qv_batch *b) {
     size_t smem = work_smem_per_warp(b) * 8;
     QV_CUDA(c, cudaFuncSetAttribute(k_batch_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)std::min<size_t>(smem, 227 * 1024)));
-    return QV_OK;
+    return default_shape(b);
   }
   return qv_fail(c, QV_ERR_NOMEM, "forest did not fit after repeated growth");
 }
@@ -943,6 +965,7 @@ extern "C" int qv_batch_tune(qv_batch *b, int reps, int *best_cfg, float *best_m
   b->wpb = bw;
   b->bps = bb;
   b->order = bo;
+  b->shape_fixed = true;
   if (cur_order != bo) {
     const std::vector<int4> &it = bo ? b->items_cost : b->items;
     QV_CUDA(c, cudaMemcpy(b->d_items, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice));
@@ -971,6 +994,7 @@ extern "C" int qv_batch_set_config(qv_batch *b, int warps_per_block, int blocks_
   }
   b->wpb = warps_per_block;
   b->bps = blocks_per_sm;
+  b->shape_fixed = true;
   if (order != b->order) {
     const std::vector<int4> &it = order ? b->items_cost : b->items;
     QV_CUDA(c, cudaMemcpy(b->d_items, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice));
