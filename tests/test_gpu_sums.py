@@ -263,3 +263,28 @@ def test_tree_velocity_and_vjp_at_group_edges(n, bc):
     s.close()
     assert np.abs(u.detach().cpu().numpy() - ou).max() <= 1e-11 * np.abs(ou).max()
     assert np.abs(g.cpu().numpy() - og).max() <= 1e-11 * np.abs(og).max()
+
+
+@pytest.mark.parametrize("n", [1, 5, 31, 33, 64, 130, 4095, 4096, 4097, 4101])
+def test_pclose_at_split_edges_with_ties_and_empty_slots(n):
+    """The all-pairs search on either side of its split (one target per warp, four
+    beyond 4096 slots), on points of a coarse lattice -- most least distances
+    are ties, decided by the slot order -- with empty slots: bit for bit."""
+    rng = np.random.default_rng(n)
+    x = rng.integers(-6, 7, (n, 3)) * 0.0078125
+    inf, beh = (np.arange(n) + 1) % n + 1, (np.arange(n) - 1) % n + 1
+    if n > 40:  # drop a few points from the chain
+        for i in range(7, n - 3, 11):
+            inf[beh[i] - 1], beh[inf[i] - 1] = inf[i], beh[i]
+            inf[i] = beh[i] = 0
+    w = W.Workload("lattice", x, inf.astype(np.int32), beh.astype(np.int32),
+                   dict(boundary="open", velocity="LIA", tree_theta=0.0, box_size=0.1, dt=1e-7,
+                        delta=5e-4))
+    seed = rng.integers(0, n + 1, n).astype(np.int32)
+    c = _ctx(w)
+    c.set_closest(seed)
+    cl, cd = c.closest()
+    ocl, ocd = O.pclose(x, w.infront, w.behind, seed)
+    act = inf != 0
+    assert np.array_equal(cl, ocl)
+    assert np.array_equal(cd[act], ocd[act])
