@@ -159,7 +159,6 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
     bool bad = false, runc = false;
     double s[3];
     slot_shift(BC, sl, a.L, s);
-    const double t0 = xi[0] - s[0], t1 = xi[1] - s[1], t2 = xi[2] - s[2];
     // the root's own decision; the unshifted image's tasks then take one child
     const WNode64 r = a.w64[0];
     const bool lone = r.count == 1;  // the root is a leaf: the first task takes it
@@ -173,7 +172,7 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
     int top = !rm ? 0 : lone ? 1 : max(0, c1 - c0);
     if (lane < top) {
       const int ch = lone ? 0 : r.child_first + c1 - 1 - lane;
-      fill_ent64(st[lane], a.w64[ch], ch, rm, ith, a.extra, sure);
+      fill_ent64(st[lane], a.w64[ch], ch, rm, s, ith, a.extra, sure);
     }
     __syncwarp();
     while (top > 0) {
@@ -181,7 +180,7 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
       const StkEnt64 e = st[top];
       const bool in = (e.mask >> lane) & 1u;
       __syncwarp();
-      const double v0 = t0 - e.cx, v1 = t1 - e.cy, v2 = t2 - e.cz;
+      const double v0 = xi[0] - e.cx, v1 = xi[1] - e.cy, v2 = xi[2] - e.cz;
       const double d2 = fma(v0, v0, fma(v1, v1, v2 * v2));
       if (e.nc < 0) {
         const int j = e.jb;
@@ -190,8 +189,9 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
             bad = true;
           } else {
             const WPay64 &P = a.p64[e.node];
-            if (!leaf_term64(-v0, -v1, -v2, P.b[0] - t0, P.b[1] - t1, P.b[2] - t2, P.b[0] - P.a[0],
-                             P.b[1] - P.a[1], P.b[2] - P.a[2], 1., acc)) {
+            if (!leaf_term64(-v0, -v1, -v2, P.b[0] + s[0] - xi[0], P.b[1] + s[1] - xi[1],
+                             P.b[2] + s[2] - xi[2], P.b[0] - P.a[0], P.b[1] - P.a[1],
+                             P.b[2] - P.a[2], 1., acc)) {
               // beside the segment: the reference's expression
               double R1[3], R2[3], cr[3];
 #pragma unroll
@@ -233,7 +233,7 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
         }
         if (lane < nc) {
           const int ch = e.child_first + nc - 1 - lane;
-          fill_ent64(st[top + lane], a.w64[ch], ch, om, ith, a.extra, sure);
+          fill_ent64(st[top + lane], a.w64[ch], ch, om, s, ith, a.extra, sure);
         }
         top += nc;
       }
@@ -1202,7 +1202,6 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
       const double *p = a.pts + 3 * (size_t)a.perm[q];
       x[0] = p[0]; x[1] = p[1]; x[2] = p[2];
     }
-    const double t0 = x[0] - s[0], t1 = x[1] - s[1], t2 = x[2] - s[2];
     unsigned ev = 0;
     bool bad = false;
     // the root's own decision; the unshifted image's tasks then take one child
@@ -1222,7 +1221,7 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
     int top = rm && c1 > c0 ? c1 - c0 : 0;
     if (lane < top) {
       const int ch = r.child_first + c1 - 1 - lane;
-      fill_ent64(st[lane], a.w64[ch], ch, rm, ith, false, true);
+      fill_ent64(st[lane], a.w64[ch], ch, rm, s, ith, false, true);
     }
     __syncwarp();
     while (top > 0) {
@@ -1230,7 +1229,7 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
       const StkEnt64 e = st[top];
       const bool in = (e.mask >> lane) & 1u;
       __syncwarp();
-      const double v0 = t0 - e.cx, v1 = t1 - e.cy, v2 = t2 - e.cz;
+      const double v0 = x[0] - e.cx, v1 = x[1] - e.cy, v2 = x[2] - e.cz;
       const double d2 = fma(v0, v0, fma(v1, v1, v2 * v2));
       bool skip = false;
       if (e.nc < 0) {
@@ -1238,8 +1237,9 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
           if (d2 < 1e-28) general_far(x, a.w64[e.node], s, a.theta, skip);
           if (!skip) {
             const WPay64 &P = a.p64[e.node];
-            if (!leaf_term64(-v0, -v1, -v2, P.b[0] - t0, P.b[1] - t1, P.b[2] - t2, P.b[0] - e.cx,
-                             P.b[1] - e.cy, P.b[2] - e.cz, 1. / (4. * QV_PI), acc))
+            if (!leaf_term64(-v0, -v1, -v2, P.b[0] + s[0] - x[0], P.b[1] + s[1] - x[1],
+                             P.b[2] + s[2] - x[2], P.b[0] - P.a[0], P.b[1] - P.a[1],
+                             P.b[2] - P.a[2], 1. / (4. * QV_PI), acc))
               general_leaf(x, a.cent + 3 * (size_t)e.node, a.circ + 3 * (size_t)e.node, s, acc);
             ev++;
           }
@@ -1265,7 +1265,7 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
         }
         if (lane < nc) {
           const int ch = e.child_first + nc - 1 - lane;
-          fill_ent64(st[top + lane], a.w64[ch], ch, om, ith, false, true);
+          fill_ent64(st[top + lane], a.w64[ch], ch, om, s, ith, false, true);
         }
         top += nc;
       }

@@ -144,9 +144,10 @@ struct __align__(16) StkEnt {
 
 
 // ------------------------------------------------------------ FP64 walks
-// Stack entry of the FP64 walks: the child's centroid and the squared opening
-// radius, made by the lane that pushes it, so that a pop reads shared memory
-// and the distance vector serves both the opening test and the far-field term.
+// Stack entry of the FP64 walks: the child's centroid shifted to the task's
+// image and the squared opening radius, made by the lane that pushes it, so
+// that a pop reads shared memory and the distance vector -- x_i - (cent + shift),
+// rounded as the reference's -- serves both the opening test and the far term.
 struct __align__(16) StkEnt64 {
   double cx, cy, cz;
   // squared distance above rhi: the node is taken whole; below rlo: opened; in
@@ -167,8 +168,9 @@ struct __align__(16) StkEnt64 {
 // both (dist - geo loses at most a factor two); the reference's rounded
 // expression decides inside it, so every decision is the reference's.
 __device__ __forceinline__ void fill_ent64(StkEnt64 &E, const WNode64 &h, int node, unsigned mask,
-                                           double inv_theta, bool extra, bool sure) {
-  E.cx = h.cx; E.cy = h.cy; E.cz = h.cz;
+                                           const double *s, double inv_theta, bool extra,
+                                           bool sure) {
+  E.cx = h.cx + s[0]; E.cy = h.cy + s[1]; E.cz = h.cz + s[2];
   const double rc = (extra ? h.geo : 0.) + h.width * inv_theta, rc2 = rc * rc;
   E.rhi = sure ? rc2 * (1. + 1e-11) : __longlong_as_double(0x7ff0000000000000ll);
   E.rlo = sure ? rc2 * (1. - 1e-11) : -1.;
