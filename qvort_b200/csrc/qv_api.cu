@@ -649,8 +649,11 @@ static int velocity_launch(qv_ctx *c) {
   qv_phase_begin(c, PH_LIA);
   if ((rc = qv_launch_lia(c))) return rc;
   qv_phase_end(c, PH_LIA);
+  c->nact_pending = false;
   if (c->p.velocity == QV_VEL_BS) {
-    if ((rc = qv_compact_active(c))) return rc;
+    // the small sum needs no active list: its count is read with the status
+    c->nact_pending = qv_direct_small(&c->p, c->n);
+    if ((rc = c->nact_pending ? qv_compact_active_async(c) : qv_compact_active(c))) return rc;
     qv_phase_begin(c, PH_NONLOCAL);
     if ((rc = qv_launch_direct(c))) return rc;
     qv_phase_end(c, PH_NONLOCAL);
@@ -678,7 +681,11 @@ static int velocity_collect(qv_ctx *c, long long *eval_count) {
   QV_CUDA(c, cudaMemcpyAsync(hs, c->evals, sizeof(*hs), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaMemcpyAsync(hs + 1, c->evals_far, sizeof(*hs), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaMemcpyAsync(hs + 2, c->dstatus, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (c->nact_pending)
+    QV_CUDA(c, cudaMemcpyAsync(hs + 3, c->d_nact, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (c->nact_pending) memcpy(&c->n_act, hs + 3, sizeof(int));
+  c->nact_pending = false;
   const unsigned long long dev_ev = hs[0], dev_far = hs[1];
   int st = 0;
   memcpy(&st, hs + 2, sizeof(int));

@@ -361,6 +361,90 @@ __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const in
   }
 }
 
+// Few points: one block per target slot, its threads sharing out the source
+// slots, straight from the point arrays -- no active list, source pack or
+// partial sums, and one launch instead of three.  A thread per target leaves a
+// small system's threads with all sources one after another: 200 points on two
+// blocks took 26 us however little there is to sum.  Up to QV_D64_SMALL slots
+// (see there); u may be null (the allocation-free entry point wants u_bs alone).
+#define D64S 128
+template <int BC>
+__global__ void __launch_bounds__(D64S) k_direct64_small(int n, const double *__restrict__ x,
+                                                         const double *__restrict__ gi,
+                                                         const int *__restrict__ inf,
+                                                         const int *__restrict__ beh, double L,
+                                                         double scale,
+                                                         const double *__restrict__ u_li, double *u,
+                                                         double *u_bs) {
+  __shared__ double red[D64S / 32][3];
+  const int i = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (inf[i] == 0) return;
+  const double x0 = x[3 * i], x1 = x[3 * i + 1], x2 = x[3 * i + 2];
+  const int bi = beh[i];
+  double a[3] = {0., 0., 0.};
+#pragma unroll 1
+  for (int j0 = wid * 32; j0 < n; j0 += D64S) {
+    const int j = j0 + lane;
+    const bool live = j < n && inf[j] != 0;
+    const int k = live ? j : i;
+    const double y0 = x[3 * k], y1 = x[3 * k + 1], y2 = x[3 * k + 2];
+    const double s0 = gi[3 * k] - y0, s1 = gi[3 * k + 1] - y1, s2 = gi[3 * k + 2] - y2;
+    const Seg64<BC> e(y0 - x0, y1 - x1, y2 - x2, s0, s1, s2, s0 * s0 + s1 * s1 + s2 * s2, L);
+    // src/timestep.f90:471, 496
+    const bool own = j == i, skip = !live || j + 1 == bi || (own && e.NI == 1);
+    const bool fast = __all_sync(0xffffffffu, skip || e.far(own, L));
+    if (!skip) e.velocity(L, fast, own, a[0], a[1], a[2]);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    if (lane == 0) red[wid][c] = a[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    const int c = threadIdx.x;
+    double v = 0.;
+#pragma unroll
+    for (int w = 0; w < D64S / 32; w++) v += red[w][c];
+    v *= scale;
+    u_bs[3 * i + c] = v;
+    if (u) u[3 * i + c] = u_li[3 * i + c] + v;
+  }
+}
+
+// Slots up to which the FP64 sum takes a block per target.  Whole velocity call,
+// tiles and block per target: open, 200 slots 96 and 53 us, 1,000 98 and 63,
+// 4,000 145 and 130, 6,000 218 and 230; periodic 120 and 56, 143 and 105, 885 and
+// 838, 1,805 and 1,791.  Above, the tile kernel reads each source once for 128
+// targets and the call no longer hangs on its launches.  The test hook of the
+// tile kernels' waits keeps them in use.
+#define QV_D64_SMALL 4096
+bool qv_direct_small(const qv_params *p, int n) {
+  return p->precision == QV_PREC_FP64 && n <= QV_D64_SMALL && !g_stage_fail;
+}
+
+static int launch_direct_small(cudaStream_t st, const qv_params *p, int n, const double *x,
+                               const double *gi, const int *inf, const int *beh,
+                               const double *u_li, double *u, double *u_bs) {
+  const double scale = p->quant_circ / (4. * QV_PI), L = p->box_size;
+  switch (p->boundary) {
+#define QV_SMALL_CASE(BCV)                                                                       \
+  case BCV:                                                                                      \
+    k_direct64_small<BCV><<<n, D64S, 0, st>>>(n, x, gi, inf, beh, L, scale, u_li, u, u_bs);      \
+    break;
+    QV_SMALL_CASE(QV_BC_OPEN)
+    QV_SMALL_CASE(QV_BC_PERIODIC)
+    QV_SMALL_CASE(QV_BC_OPENX)
+    QV_SMALL_CASE(QV_BC_OPENXY)
+#undef QV_SMALL_CASE
+    default:
+      return QV_ERR_UNSUPPORTED;
+  }
+  return cudaGetLastError() == cudaSuccess ? QV_OK : QV_ERR_CUDA;
+}
+
 // ------------------------------------------------------------ mixed kernel
 // Every staged source is read from shared memory once and summed against the
 // thread's NT targets in all images.  An image (a, b, c) shifts the source by
@@ -654,6 +738,13 @@ int qv_pack_sources64(qv_ctx *c) {
 }
 
 int qv_launch_direct(qv_ctx *c) {
+  if (c->n > 0 && qv_direct_small(&c->p, c->n)) {
+    const int rc = launch_direct_small(c->stream, &c->p, c->n, c->x, c->gi, c->infront, c->behind,
+                                       c->u_li, c->u, c->u_bs);
+    if (rc) return qv_fail(c, rc, "direct sum of %d slots: launch failed", c->n);
+    QV_COUNT(c, 1);
+    return QV_OK;
+  }
   int na = c->n_act;
   if (na == 0) return QV_OK;
   int tb = nblk(c->n_act, 256);
@@ -727,6 +818,11 @@ __global__ void k_direct_reduce_bs(int na, int nchunk, const int *__restrict__ a
 int qv_direct_scratch(cudaStream_t s, const qv_params *p, int sm_count, int n, const double *x,
                       const int *inf, const int *beh, const double *gi, int *act, int *blk,
                       double *src64, float *src32, double *part, int max_chunks, double *u_bs) {
+  if (qv_direct_small(p, n)) {
+    if (cudaMemsetAsync(u_bs, 0, sizeof(double) * 3 * (size_t)n, s) != cudaSuccess)
+      return QV_ERR_CUDA;
+    return launch_direct_small(s, p, n, x, gi, inf, beh, nullptr, nullptr, u_bs);
+  }
   int nb = nblk(n, 256);
   k_count_active<<<nb, 256, 0, s>>>(n, inf, blk);
   k_scan_small<<<1, 1024, 0, s>>>(nb, blk, blk + nb);

@@ -174,6 +174,7 @@ struct qv_ctx {
   int *act = nullptr;  // compacted active slots (direct sums)
   int n_act = 0;
   int *d_nact = nullptr;  // device copy of n_act (tree path)
+  bool nact_pending = false;  // n_act is still on the device alone (velocity_collect reads it)
   int *blkcnt = nullptr;  // per-256-slot block counts of the compaction (n/256+2)
   double *dpart = nullptr;  // direct-sum partial sums, grown on demand
   size_t dpart_bytes = 0;
@@ -251,6 +252,8 @@ void qv_phase_collect(qv_ctx *c);
 int qv_launch_ghosts(qv_ctx *c);
 int qv_launch_lia(qv_ctx *c);
 int qv_launch_direct(qv_ctx *c);
+// whether the direct sum of n slots takes a block per target (no active list)
+bool qv_direct_small(const qv_params *p, int n);
 int qv_launch_tree_build(qv_ctx *c);
 // Join the exact root centroid and re-pack the root with it, and join the late
 // level-1 moments and payloads (no-op when both are in already).  Every reader

@@ -288,3 +288,19 @@ def test_pclose_at_split_edges_with_ties_and_empty_slots(n):
     act = inf != 0
     assert np.array_equal(cl, ocl)
     assert np.array_equal(cd[act], ocd[act])
+
+
+@pytest.mark.parametrize("bc", ["open", "periodic"])
+@pytest.mark.parametrize("n", [4095, 4096, 4097])
+def test_direct_fp64_either_side_of_the_small_sum(n, bc):
+    """The last sizes with a block per target and the first with tiles, on 64 of
+    the targets (1e-11 as above); the evaluation count needs the active count."""
+    w = _ring_pair(n)
+    u, _, _, ev = _ctx(w, boundary=bc, precision="fp64").velocity()
+    assert ev == n * n * (27 if bc == "periodic" else 1)
+    at = np.unique(np.random.default_rng(n).integers(0, n, 64))
+    x = w.x[at]
+    p = O.params(**dict(w.params, boundary=bc))
+    g = O.ghosts(p, w.x, w.infront, w.behind)
+    ou = O.velocity(p, w.x, w.infront, w.behind, g, nthreads=8)[0]
+    assert len(x) and np.abs(u - ou)[at].max() <= 1e-11 * np.abs(ou[at]).max()
