@@ -120,14 +120,16 @@ __global__ void k_lia_vjp(int n, const double *__restrict__ x, const int *__rest
 // One pass over all (source, target) pairs gives both ends' gradients: a thread
 // holds one source and sums its own (dL/dx_j at fixed s, dL/ds) over a chunk of
 // targets, while each target's gradient -- minus the sum over sources -- is
-// reduced over the warp (12 shuffles a target against 27 images x ~55 FP64
+// reduced over the warp (12 shuffles a target against 27 images x ~45 FP64
 // operations a lane) and over the block's warps in shared memory.  Partial
 // sums per (source block, target) and per (target chunk, source) are added in
 // a fixed order by k_dvjp_reduce, so results are deterministic, with no
 // atomics.  A two-pass split (a thread per target, then a thread per source)
 // evaluates every pair twice.  Bound: FP64 issue.  6,400 points, 27 images:
 // velocity and gradient together took 333 ms with two passes, divisions in every
-// image term and 50 blocks; 8.4 ms now, about 2 of them the velocity.
+// image term and 50 blocks; 7.2 ms now, 2 of them the velocity (78 % of the FP64
+// rate at about 55 operations a pair; the x shifts unrolled took 255 registers,
+// two blocks per SM and 0.4 ms more).
 #define VT 128  // sources per block
 #define VG 32   // targets per shared-memory tile
 #define QV_DVJP_PART ((size_t)256 << 20)  // bytes of per-target partial sums per launch
@@ -148,7 +150,7 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 // Targets t_lo..t_hi (positions in act); tpart: (source blocks) x (t_hi - t_lo)
 // x 3, spart: (target chunks) x na x 6.
 template <int BC>
-__global__ void __launch_bounds__(VT, 2) k_dvjp(int na, const int *__restrict__ act,
+__global__ void __launch_bounds__(VT, 3) k_dvjp(int na, const int *__restrict__ act,
                                                 const double *__restrict__ x,
                                                 const double *__restrict__ gi,
                                                 const int *__restrict__ beh,
@@ -300,7 +302,7 @@ __device__ __forceinline__ void seg_gradient_pos(const double *R, const double *
   const double gr[3] = {g[1] * R[2] - g[2] * R[1], g[2] * R[0] - g[0] * R[2],
                         g[0] * R[1] - g[1] * R[0]};
   const double Q = R[0] * h[0] + R[1] * h[1] + R[2] * h[2];
-  const double al = 2. * Q * t.fA, be = Q * t.fw, ga = Q * t.fc2;
+  const double al = Q * t.fA2, be = Q * t.fw, ga = Q * t.fc2;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     dR[c] = fma(t.f, h[c], fma(al, R[c], be * s[c]));
@@ -621,8 +623,8 @@ __global__ void k_energy_grad(int n, const double *__restrict__ x, const double 
 __device__ __forceinline__ void add_jacobian(const SegD &t, double X, double Y, double Z, double sx,
                                              double sy, double sz, double cx, double cy, double cz,
                                              double *J) {
-  const double h = 2. * t.fA;
-  const double vx = fma(h, X, t.fw * sx), vy = fma(h, Y, t.fw * sy), vz = fma(h, Z, t.fw * sz);
+  const double vx = fma(t.fA2, X, t.fw * sx), vy = fma(t.fA2, Y, t.fw * sy),
+               vz = fma(t.fA2, Z, t.fw * sz);
   J[0] -= cx * vx;
   J[1] -= fma(cx, vy, t.f * sz);
   J[2] -= fma(cx, vz, -t.f * sy);
@@ -831,9 +833,10 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
       const int nsb = nblk(na, VT);
       const size_t row = sizeof(double) * 3 * (size_t)nsb;
       const int slab = (int)std::min<size_t>(na, std::max<size_t>(VG, QV_DVJP_PART / row / VG * VG));
-      // eight blocks per resident slot (2 per SM), each with enough pairs
-      // (targets x images) to outweigh its start and its partial sums
-      const int want = nblk(16L * c->sm_count, nsb);
+      // ten blocks per resident slot (3 per SM; with five the last wave cost 5 %),
+      // each with enough pairs (targets x images) to outweigh its start and its
+      // partial sums
+      const int want = nblk(30L * c->sm_count, nsb);
       const int least = p.boundary == QV_BC_PERIODIC ? 8 : p.boundary == QV_BC_OPENX ? 16 : VG;
       const int chunk_len = nblk(nblk(slab, want), least) * least, nchunk = nblk(slab, chunk_len);
       const size_t tbytes = row * slab, sbytes = sizeof(double) * 6 * (size_t)na * nchunk;

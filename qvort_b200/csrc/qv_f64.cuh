@@ -53,31 +53,30 @@ __device__ __forceinline__ double seg_f_any(double A, double B, double d, double
 }
 
 // f and its partial derivatives as a function of A = |R1|^2, w = R1.s and
-// c = |s|^2 (B = A + 2 w + c, d = A + w): with m = |R1||R2|, e = m + d, S =
-// |R1| + |R2|, f = S / (m e) and
-//   fA = f (-((1/|R1| - 1/|R2|)^2 + 1/m) / 2 - ((A + B) / (2 m) + 1) / e)
-//   fw = f (k - (A / m + 1) / e),   2 fc = f (k - (A / m) / e),
-//   k  = 1 / (m + B) - 1 / B = -|R1| / (B S).
+// c = |s|^2 (B = A + 2 w + c, d = A + w): with a = |R1|, b = |R2|, m = a b, q =
+// 1 / m, e = m + d and g = f / e (1 / m + 1 / B and the like written through the
+// reciprocals at hand; the sum a + b in f = (a + b) / (m e) cancels from the
+// derivatives of its logarithm)
+//   2 fA = -(f ((1/a - 1/b)^2 + q) + g ((A + B) q + 2))
+//   2 fc = -(1/b^3 + f A q) / e,   fw = 2 fc - g.
 // The gradients of u = f (R1 x s) follow by the chain rule.
 struct SegD {
-  double f, fA, fw, fc2;  // fc2 = 2 df/dc
+  double f, fA2, fw, fc2;  // f, 2 df/dA, df/dw, 2 df/dc
 };
 __device__ __forceinline__ SegD seg_d_of(double A, double B, double ra, double rb, double q,
-                                         double ie, double iS) {
+                                         double ie) {
   SegD r;
   r.f = (ra + rb) * ie;
-  const double k = -(A * ra) * (rb * rb) * iS;
-  const double aq = A * q * ie, dr = ra - rb;
-  r.fc2 = k - aq;
-  r.fw = r.f * (r.fc2 - ie);
-  r.fc2 *= r.f;
-  r.fA = r.f * -fma(0.5, fma(dr, dr, q), fma(0.5 * (A + B), q, 1.) * ie);
+  const double g = r.f * ie, dr = ra - rb;
+  r.fc2 = -ie * fma(rb * rb, rb, r.f * (A * q));
+  r.fw = r.fc2 - g;
+  r.fA2 = -fma(r.f, fma(dr, dr, q), g * fma(A + B, q, 2.));
   return r;
 }
 // d > 0
 __device__ __forceinline__ SegD seg_d_pos(double A, double B, double d) {
   const double ra = rsqrt_pos(A), rb = rsqrt_pos(B), q = ra * rb;
-  return seg_d_of(A, B, ra, rb, q, div_pos(q, fma(d, q, 1.)), div_pos(1., fma(A, ra, B * rb)));
+  return seg_d_of(A, B, ra, rb, q, div_pos(q, fma(d, q, 1.)));
 }
 // any d; c2 = |R1 x s|^2 (0: a point on the segment's line, no term)
 __device__ __forceinline__ SegD seg_d_any(double A, double B, double d, double c2) {
@@ -87,7 +86,7 @@ __device__ __forceinline__ SegD seg_d_any(double A, double B, double d, double c
   }
   const double a = sqrt(A), b = sqrt(B), m = a * b;
   const double e = d < 0. ? c2 / (m - d) : m + d;
-  return seg_d_of(A, B, 1. / a, 1. / b, 1. / m, 1. / e, 1. / (a + b));
+  return seg_d_of(A, B, 1. / a, 1. / b, 1. / m, 1. / e);
 }
 
 // ------------------------------------------------------------ image sums
@@ -251,20 +250,20 @@ struct Seg64 {
     double f0 = 0., b0 = 0., c0 = 0.;
     double fX = 0., fY = 0., fZ = 0., aX = 0., aY = 0., aZ = 0., bX = 0., bY = 0., bZ = 0.;
     if (fast) {
-      double tx[PX], ty[PY], tz[PZ], qx[PX], qy[PY], qz[PZ];
-#pragma unroll
-      for (int k = 0; k < PX; k++) { tx[k] = fma(rx[k], sx, gx[k] + c); qx[k] = rx[k] * hx; }
+      double ty[PY], tz[PZ], qy[PY], qz[PZ];
 #pragma unroll
       for (int k = 0; k < PY; k++) { ty[k] = fma(ry[k], sy, gy[k]); qy[k] = ry[k] * hy; }
 #pragma unroll
       for (int k = 0; k < PZ; k++) { tz[k] = fma(rz[k], sz, gz[k]); qz[k] = rz[k] * hz; }
-#pragma unroll
+#pragma unroll 1  // a third of the code and registers: three blocks per SM
       for (int a = 0; a < PX; a++) {
+        const double xa = PX == 3 ? rx[PX / 2] + (a - 1) * L : rx[0], pa = xa * xa,
+                     ga = fma(xa, sx, pa), ta = fma(xa, sx, ga + c), qa = xa * hx;
         double fa = 0., aa = 0., ba = 0.;  // sums over the shifts (b, k) of this a
 #pragma unroll
         for (int b = 0; b < PY; b++) {
-          const double pxy = px[a] + py[b], gxy = gx[a] + gy[b], txy = tx[a] + ty[b],
-                       qxy = qx[a] + qy[b];
+          const double pxy = pa + py[b], gxy = ga + gy[b], txy = ta + ty[b],
+                       qxy = qa + qy[b];
           double fb = 0., ab = 0., bb = 0.;
 #pragma unroll
           for (int k = 0; k < PZ; k++) {
@@ -274,7 +273,7 @@ struct Seg64 {
             if (own) A = B = d = 1.;
             SegD t = seg_d_pos(A, B, d);
             if (own) t.f = Q = 0.;
-            const double al = 2. * Q * t.fA, be = Q * t.fw;
+            const double al = Q * t.fA2, be = Q * t.fw;
             c0 = fma(Q, t.fc2, c0);
             fb += t.f; ab += al; bb += be;
             fZ = fma(t.f, rz[k], fZ);
@@ -287,9 +286,9 @@ struct Seg64 {
           bY = fma(bb, ry[b], bY);
         }
         f0 += fa; b0 += ba;
-        fX = fma(fa, rx[a], fX);
-        aX = fma(aa, rx[a], aX);
-        bX = fma(ba, rx[a], bX);
+        fX = fma(fa, xa, fX);
+        aX = fma(aa, xa, aX);
+        bX = fma(ba, xa, bX);
       }
     } else {
 #pragma unroll 1
@@ -302,7 +301,7 @@ struct Seg64 {
         const double ex = X + sx, ey = Y + sy, ez = Z + sz;
         const SegD t =
             seg_d_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
-        const double Q = X * hx + Y * hy + Z * hz, al = 2. * Q * t.fA, be = Q * t.fw;
+        const double Q = X * hx + Y * hy + Z * hz, al = Q * t.fA2, be = Q * t.fw;
         f0 += t.f; b0 += be; c0 += Q * t.fc2;
         fX += t.f * X; fY += t.f * Y; fZ += t.f * Z;
         aX += al * X; aY += al * Y; aZ += al * Z;
