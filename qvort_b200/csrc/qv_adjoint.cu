@@ -466,45 +466,60 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
 }
 
 // Node adjoint -> point adjoints through cent = sum x / n, circ = sum (gi - x),
-// C = sum x (gi - x)^T - cent circ^T (src/tree.f90:154-179).  One warp per node.
-__global__ void k_moment_vjp(int n_nodes, const int *__restrict__ level,
-                             const int *__restrict__ start, const int *__restrict__ count,
-                             const int *__restrict__ ord, int cap_pts, const double *__restrict__ x,
-                             const double *__restrict__ gi, const double *__restrict__ cent,
-                             const double *__restrict__ circ, const double *__restrict__ nb,
-                             double *xb, double *gib) {
-  int lane = threadIdx.x & 31;
-  int k = 1 + (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (k >= n_nodes) return;
-  const double *B = nb + NBS * (size_t)k;
+// C = sum x (gi - x)^T - cent circ^T (src/tree.f90:154-179): the points t0, t0 +
+// step, ... of node k.
+struct MomentArgs {
+  const int *level, *start, *count, *ord;
+  int cap_pts;
+  const double *x, *gi, *cent, *circ, *nb;
+  double *xb, *gib;
+};
+__device__ __forceinline__ void moment_vjp(const MomentArgs &a, int k, int t0, int step) {
+  const int n = a.count[k];
+  if (n == 1) return;  // a leaf's gradients went to its point
+  const double *B = a.nb + NBS * (size_t)k;
   double Cb[9], cb[3], qb[3];
   bool any = false;
   for (int t = 0; t < 15; t++) any |= B[t] != 0.;
   if (!any) return;
   for (int t = 0; t < 9; t++) Cb[t] = B[6 + t];
+  const double *cent = a.cent + 3 * (size_t)k, *circ = a.circ + 3 * (size_t)k;
   // C = C_raw - cent circ^T
   for (int r = 0; r < 3; r++) {
-    cb[r] = B[r] - (Cb[3 * r] * circ[3 * k] + Cb[3 * r + 1] * circ[3 * k + 1] + Cb[3 * r + 2] * circ[3 * k + 2]);
-    qb[r] = B[3 + r] - (Cb[r] * cent[3 * k] + Cb[3 + r] * cent[3 * k + 1] + Cb[6 + r] * cent[3 * k + 2]);
+    cb[r] = B[r] - (Cb[3 * r] * circ[0] + Cb[3 * r + 1] * circ[1] + Cb[3 * r + 2] * circ[2]);
+    qb[r] = B[3 + r] - (Cb[r] * cent[0] + Cb[3 + r] * cent[1] + Cb[6 + r] * cent[2]);
   }
-  int n = count[k];
-  const int *o = ord + (size_t)level[k] * cap_pts + start[k];
-  for (int t = lane; t < n; t += 32) {
-    int p = o[t];
-    double X[3], GI[3], s[3];
-    for (int c = 0; c < 3; c++) { X[c] = x[3 * p + c]; GI[c] = gi[3 * p + c]; s[c] = GI[c] - X[c]; }
-    double dx[3], dg[3];
+  for (int c = 0; c < 3; c++) cb[c] /= n;
+  const int *o = a.ord + (size_t)a.level[k] * a.cap_pts + a.start[k];
+  for (int t = t0; t < n; t += step) {
+    const int p = o[t];
+    double X[3], s[3];
+    for (int c = 0; c < 3; c++) { X[c] = a.x[3 * p + c]; s[c] = a.gi[3 * p + c] - X[c]; }
     for (int c = 0; c < 3; c++) {
-      double Cs = Cb[3 * c] * s[0] + Cb[3 * c + 1] * s[1] + Cb[3 * c + 2] * s[2];   // (C_b s)_c
-      double CtX = Cb[c] * X[0] + Cb[3 + c] * X[1] + Cb[6 + c] * X[2];           // (C_b^T x)_c
-      dx[c] = cb[c] / n - qb[c] + Cs - CtX;
-      dg[c] = qb[c] + CtX;
-    }
-    for (int c = 0; c < 3; c++) {
-      atomicAdd(&xb[3 * p + c], dx[c]);
-      atomicAdd(&gib[3 * p + c], dg[c]);
+      const double Cs = Cb[3 * c] * s[0] + Cb[3 * c + 1] * s[1] + Cb[3 * c + 2] * s[2];  // (C_b s)_c
+      const double CtX = Cb[c] * X[0] + Cb[3 + c] * X[1] + Cb[6 + c] * X[2];          // (C_b^T x)_c
+      atomicAdd(&a.xb[3 * p + c], cb[c] - qb[c] + Cs - CtX);
+      atomicAdd(&a.gib[3 * p + c], qb[c] + CtX);
     }
   }
+}
+// Nodes k0 .. n_nodes - 1, eight to a block: a warp each, and the block's warps
+// together where a node holds more than MV_BIG points.
+#define MV_BIG 128
+__global__ void __launch_bounds__(256) k_moment_vjp(MomentArgs a, int k0, int n_nodes) {
+  const int b0 = k0 + blockIdx.x * 8, k = b0 + (threadIdx.x >> 5);
+  if (k < n_nodes && a.count[k] <= MV_BIG) moment_vjp(a, k, threadIdx.x & 31, 32);
+  for (int e = b0; e < min(b0 + 8, n_nodes); e++)
+    if (a.count[e] > MV_BIG) moment_vjp(a, e, threadIdx.x, 256);
+}
+// The nodes of the first levels (1 .. n - 1) hold most of the points each: MV_SPLIT
+// blocks per node.  A warp for a root child of 6,000 points was a chain of 200
+// gathers and atomics, 285 us at 50,000 points; MV_NOW.
+#define MV_TOP 585  // levels 0 to 3 of a full octree
+#define MV_SPLIT 16
+__global__ void __launch_bounds__(256) k_moment_vjp_top(MomentArgs a, int n) {
+  const int k = 1 + blockIdx.x;
+  if (k < n) moment_vjp(a, k, blockIdx.y * 256 + threadIdx.x, 256 * MV_SPLIT);
 }
 
 // Ghost adjoint: gi_i = x_infront(i), gb_i = x_behind(i), gii_i = x_infront(infront(i)),
@@ -906,10 +921,16 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
       QV_CUDA(c, cudaLaunchKernel(f, dim3(nb), dim3(AW * 32), args, smem, c->stream));
       QV_LAUNCH_CHECK(c);
       if (t.n_nodes > 1) {
-        k_moment_vjp<<<nblk((long)(t.n_nodes - 1) * 32, 256), 256, 0, c->stream>>>(
-            t.n_nodes, t.level, t.start, t.count, t.ord, t.cap_pts, c->x, c->gi, t.cent, t.circ,
-            c->adj_nb, c->adj_xb, c->adj_gib);
+        MomentArgs m;
+        m.level = t.level; m.start = t.start; m.count = t.count; m.ord = t.ord;
+        m.cap_pts = t.cap_pts; m.x = c->x; m.gi = c->gi; m.cent = t.cent; m.circ = t.circ;
+        m.nb = c->adj_nb; m.xb = c->adj_xb; m.gib = c->adj_gib;
+        const int ntop = std::min(t.n_nodes, MV_TOP);
+        k_moment_vjp_top<<<dim3(ntop - 1, MV_SPLIT), 256, 0, c->stream>>>(m, ntop);
+        if (t.n_nodes > ntop)
+          k_moment_vjp<<<nblk(t.n_nodes - ntop, 8), 256, 0, c->stream>>>(m, ntop, t.n_nodes);
         QV_LAUNCH_CHECK(c);
+        QV_COUNT(c, 1);
       }
       QV_COUNT(c, 2);
     }

@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(512) k_root_cent(const int *__restrict__ d_nac
 // (which also covers the rounding of sum|x| itself).  The same pass copies the
 // active positions, in active order, to xc for the exact chain, so that the
 // chain reads nothing another kernel may write before it is joined.  The last
-// block to finish (ticket ctl[3]) reduces the block sums in block order and
+// block to finish (ticket ctl[3]) reduces the block sums in a fixed order and
 // clears the counters of the walk's fix-up.
 __global__ void __launch_bounds__(256) k_root_est(const int *__restrict__ d_nact,
                                                   const int *__restrict__ act,
@@ -1112,10 +1112,18 @@ __global__ void __launch_bounds__(256) k_root_est(const int *__restrict__ d_nact
   __syncthreads();
   if (!last) return;
   __threadfence();
+  // one warp per sum: the blocks' partial sums one after another by one thread
+  // held the build up for 35 us (any order keeps the bound)
+  if (w < 6) {
+    double t = 0.;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += part[6 * b + w];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) red[w][0] = t;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double S[6] = {0., 0., 0., 0., 0., 0.};
-    for (int b = 0; b < (int)gridDim.x; b++)
-      for (int k = 0; k < 6; k++) S[k] += part[6 * b + k];
+    double S[6];
+    for (int k = 0; k < 6; k++) S[k] = red[k][0];
     const double u = 1.1102230246251565e-16, nu = n * u;
     const double gam = nu / (1. - nu);
     double e2 = 0.;
