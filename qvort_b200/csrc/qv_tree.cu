@@ -1595,6 +1595,21 @@ int qv_launch_tree_build(qv_ctx *c) {
     QV_CUDA(c, cudaEventRecord(c->ev_join[1], c->aux[1]));
   }
   bool chain_started = !spec;
+  // blocks of the cooperative build, two per SM at most
+  const int grid = std::max(1, std::min(build_grid(c), std::max(1, nblk(n, CH)) * 4));
+  if (spec && grid <= build_grid(c) - build_grid(c) / c->sm_count) {
+    // the build leaves an SM free: the chain starts here, not behind the
+    // cooperative kernel (120 us earlier at 50,000 slots)
+    QV_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
+    QV_CUDA(c, cudaStreamWaitEvent(c->aux[1], c->ev_fork, 0));
+    k_root_cent<<<1, 512, 2 * RC * 3 * sizeof(double), c->aux[1]>>>(c->d_nact, nullptr, t.root_xc,
+                                                                     t.root_est + 4);
+    QV_LAUNCH_CHECK(c);
+    QV_COUNT(c, 1);
+    QV_CUDA(c, cudaEventRecord(c->ev_join[1], c->aux[1]));
+    t.root_pending = true;
+    chain_started = true;
+  }
   if (!t.h_ctl) {
     QV_CUDA(c, cudaMallocHost((void **)&t.h_ctl, sizeof(int) * CTL_SIZE));
     QV_CUDA(c, cudaEventCreateWithFlags(&t.ev_ctl, cudaEventDisableTiming));
@@ -1617,8 +1632,6 @@ int qv_launch_tree_build(qv_ctx *c) {
     a.level = t.level; a.digit = t.digit; a.cmask = t.cmask; a.ord = t.ord; a.nodeA = t.nodeA;
     a.nodeB = t.nodeB; a.rnk = t.rnk; a.cnt9A = t.cnt9; a.cnt9B = t.cnt9 + 9 * (size_t)(t.cap_pts + 1);
     a.rs9 = t.rs9; a.chunk9 = t.chunk9; a.ctl = t.ctl; a.dig = t.dig; a.perm = t.permb;
-    int grid = std::min(build_grid(c), std::max(1, a.nchunks) * 4);
-    grid = std::max(grid, 1);
     void *args[] = {&a};
     QV_CUDA(c, cudaLaunchCooperativeKernel((void *)k_build, grid, BT, args, 0, c->stream));
     QV_COUNT(c, 2);
