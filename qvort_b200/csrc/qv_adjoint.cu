@@ -320,7 +320,8 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
   const bool sure = !a.extra || a.theta < 1.15;
   const int items = a.ngroups * (ANSPLIT + NIMG);
   for (int item = blockIdx.x * AW + wid; item < items; item += gridDim.x * AW) {
-    const int sl = item / a.ngroups, q = (item - sl * a.ngroups) * 32 + lane;
+    const int k = item / a.ngroups, q = (item - k * a.ngroups) * 32 + lane;
+    const int sl = k < ANSPLIT ? k : ANSPLIT + image_at<BC>(k - ANSPLIT);
     const bool live = q < a.n_act;
     const int i = live ? a.perm[q] : 0;
     double xi[3] = {0., 0., 0.}, gu[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};

@@ -145,7 +145,8 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
   const bool sure = !a.extra || a.theta < 1.15;  // see fill_ent64
   const int items = a.ngroups * (NSPLIT + NIMG);
   for (int item = blockIdx.x * WW + wid; item < items; item += gridDim.x * WW) {
-    const int sl = item / a.ngroups, q = (item - sl * a.ngroups) * 32 + lane;
+    const int k = item / a.ngroups, q = (item - k * a.ngroups) * 32 + lane;
+    const int sl = k < NSPLIT ? k : NSPLIT + image_at<BC>(k - NSPLIT);
     const bool live = q < a.n_act;
     const int i = live ? a.perm[q] : 0;
     double xi[3] = {0., 0., 0.};
@@ -730,7 +731,8 @@ __device__ __forceinline__ void walk_task2(const WalkArgs &a, StkEnt *st, int la
 }
 
 // Task order: the unshifted image's tasks (the heaviest: they carry the near
-// field), slot by slot, then the periodic images'.  Large systems hand the
+// field), slot by slot, then the periodic images', those across a face first
+// (image_at).  Large systems hand the
 // tasks out one at a time from a counter, so that a warp which finishes early
 // takes the next task instead of idling until its block's slowest warp is
 // done.  Small ones (a few tasks per warp) keep a fixed task per warp, whose
@@ -802,7 +804,7 @@ __device__ __forceinline__ void walk32_body(const WalkArgs &a) {
       else walk_task1<BC>(a, st, lane, sl, g, rdelta);
     } else {
       const int j = item - nnear, k = j / a.ng64;
-      walk_task2<BC>(a, st, lane, NSPLIT + k, j - k * a.ng64, rdelta);
+      walk_task2<BC>(a, st, lane, NSPLIT + image_at<BC>(k), j - k * a.ng64, rdelta);
     }
     item += gridDim.x * WW;
   }
@@ -1194,7 +1196,8 @@ __global__ void __launch_bounds__(GW * 32) k_walk_general(MeshArgs a) {
   const int items = ngroups * (NSPLIT + NIMG);
   const double ith = 1. / a.theta;
   for (int item = blockIdx.x * GW + wid; item < items; item += gridDim.x * GW) {
-    const int sl = item / ngroups, q = (item - sl * ngroups) * 32 + lane;
+    const int k = item / ngroups, q = (item - k * ngroups) * 32 + lane;
+    const int sl = k < NSPLIT ? k : NSPLIT + image_at<BC>(k - NSPLIT);
     const bool live = q < a.m;
     double s[3], x[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
     slot_shift(BC, sl, a.L, s);

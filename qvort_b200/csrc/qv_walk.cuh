@@ -11,6 +11,21 @@ __device__ __forceinline__ double shift_of(int m, double L) {
   return m == 0 ? 0. : (m > 0 ? L : -L);
 }
 
+// The k-th image to walk: the images across a face first, then those across an
+// edge, then a corner.  A face's image holds the near field of the groups beside
+// that face, whose tasks are the longest of all the images'; taken in the
+// reference's loop order the last of them started when most of the walk was done
+// and set its end.  Only the order of independent tasks: every task keeps its
+// slot, and the sums are added in the reference's order.
+static __constant__ unsigned char QV_IMG_ORDER26[26] = {4,  10, 12, 13, 15, 21, 1,  3,  5,
+                                                        7,  9,  11, 14, 16, 18, 20, 22, 24,
+                                                        0,  2,  6,  8,  17, 19, 23, 25};
+static __constant__ unsigned char QV_IMG_ORDER8[8] = {1, 3, 4, 6, 0, 2, 5, 7};
+template <int BC>
+__device__ __forceinline__ int image_at(int k) {
+  return BC == QV_BC_PERIODIC ? QV_IMG_ORDER26[k] : BC == QV_BC_OPENX ? QV_IMG_ORDER8[k] : k;
+}
+
 // dist = |x_i - (cent + shift)| in the reference's operation order.
 __device__ __forceinline__ double exact_dist(const double *xi, const WNode64 &h, const double *s) {
   double d0 = __dsub_rn(xi[0], __dadd_rn(h.cx, s[0]));
