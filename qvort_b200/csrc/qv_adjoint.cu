@@ -320,8 +320,9 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
   const bool sure = !a.extra || a.theta < 1.15;
   const int items = a.ngroups * (ANSPLIT + NIMG);
   for (int item = blockIdx.x * AW + wid; item < items; item += gridDim.x * AW) {
-    const int k = item / a.ngroups, q = (item - k * a.ngroups) * 32 + lane;
-    const int sl = k < ANSPLIT ? k : ANSPLIT + image_at<BC>(k - ANSPLIT);
+    const WNode64 r = a.w64[0];
+    const int row = item / a.ngroups, q0 = (item - row * a.ngroups) * 32, q = q0 + lane;
+    const int sl = task_slot<BC, ANSPLIT>(row, q0, r, a.w64);
     const bool live = q < a.n_act;
     const int i = live ? a.perm[q] : 0;
     double xi[3] = {0., 0., 0.}, gu[3] = {0., 0., 0.}, acc[3] = {0., 0., 0.};
@@ -336,7 +337,6 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
     const double s[3] = {shift_of(ma, a.L), shift_of(mb, a.L), shift_of(mc, a.L)};
     const double t0 = xi[0] - s[0], t1 = xi[1] - s[1], t2 = xi[2] - s[2];
     // the root's own decision; the unshifted image's tasks then take one child
-    const WNode64 r = a.w64[0];
     const bool lone = r.count == 1;
     const bool go = live && (lone ? sl == 0 || sl >= ANSPLIT
                                   : exact_open(exact_dist(xi, r, s), r, a.theta, a.extra));

@@ -145,8 +145,9 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
   const bool sure = !a.extra || a.theta < 1.15;  // see fill_ent64
   const int items = a.ngroups * (NSPLIT + NIMG);
   for (int item = blockIdx.x * WW + wid; item < items; item += gridDim.x * WW) {
-    const int k = item / a.ngroups, q = (item - k * a.ngroups) * 32 + lane;
-    const int sl = k < NSPLIT ? k : NSPLIT + image_at<BC>(k - NSPLIT);
+    const WNode64 r = a.w64[0];
+    const int row = item / a.ngroups, q0 = (item - row * a.ngroups) * 32, q = q0 + lane;
+    const int sl = task_slot<BC, NSPLIT>(row, q0, r, a.w64);
     const bool live = q < a.n_act;
     const int i = live ? a.perm[q] : 0;
     double xi[3] = {0., 0., 0.};
@@ -161,7 +162,6 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
     double s[3];
     slot_shift(BC, sl, a.L, s);
     // the root's own decision; the unshifted image's tasks then take one child
-    const WNode64 r = a.w64[0];
     const bool lone = r.count == 1;  // the root is a leaf: the first task takes it
     bool go = live && lone && (sl == 0 || sl >= NSPLIT);
     if (live && !lone) {

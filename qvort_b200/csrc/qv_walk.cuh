@@ -26,6 +26,29 @@ __device__ __forceinline__ int image_at(int k) {
   return BC == QV_BC_PERIODIC ? QV_IMG_ORDER26[k] : BC == QV_BC_OPENX ? QV_IMG_ORDER8[k] : k;
 }
 
+// The order of the FP64 walks' tasks: the longest first.  Rows of one task per
+// target group: row 0 the unshifted image's root child that holds the group (its
+// near field), then the images across a face, the other root children, the
+// other images.  The slot of the group that starts at target q in row `row`; r =
+// the root's header.  Tangle, FP64 velocity: 0.759 -> 0.740 ms (the mixed walk's
+// tasks in this order: no change).
+template <int BC, int NS>
+__device__ __forceinline__ int task_slot(int row, int q, const WNode64 &r, const WNode64 *w64) {
+  constexpr int NF = BC == QV_BC_PERIODIC ? 6 : BC == QV_BC_OPENX ? 4 : BC == QV_BC_OPENXY ? 2 : 0;
+  if (row >= 1 && row <= NF) return NS + image_at<BC>(row - 1);
+  if (row >= NF + NS) return NS + image_at<BC>(row - NS);
+  // targets lie in the order of the root's children
+  int home = 0;
+  for (int c = 0, end = 0; c < r.nchild; c++) {
+    end += w64[r.child_first + c].count;
+    if (q < end) {
+      home = c;
+      break;
+    }
+  }
+  return row == 0 ? home : (home + row - NF) % NS;
+}
+
 // dist = |x_i - (cent + shift)| in the reference's operation order.
 __device__ __forceinline__ double exact_dist(const double *xi, const WNode64 &h, const double *s) {
   double d0 = __dsub_rn(xi[0], __dadd_rn(h.cx, s[0]));
