@@ -82,15 +82,15 @@ extern "C" int qv_create(const qv_params *p, void *stream, qv_ctx **out) {
     }
     c->own_stream = true;
   }
-  if (cudaMalloc(&c->evals, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->evals_far, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&c->dstatus, sizeof(int)) != cudaSuccess ||
+  if (cudaMalloc(&c->evals, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&c->dscalar, 16 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->d_nact, 4 * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     delete c;
     return QV_ERR_NOMEM;
   }
+  c->evals_far = c->evals + 1;
+  c->dstatus = (int *)(c->evals + 2);
   *out = c;
   return QV_OK;
 }
@@ -132,12 +132,10 @@ extern "C" int qv_destroy(qv_ctx *c) {
   free_tree(c->tree);
   free_points(c);
   if (c->evals) cudaFree(c->evals);
-  if (c->evals_far) cudaFree(c->evals_far);
   for (int k = 0; k < PH_N; k++) {
     if (c->ev_beg[k]) cudaEventDestroy(c->ev_beg[k]);
     if (c->ev_end[k]) cudaEventDestroy(c->ev_end[k]);
   }
-  if (c->dstatus) cudaFree(c->dstatus);
   if (c->dscalar) cudaFree(c->dscalar);
   if (c->d_nact) cudaFree(c->d_nact);
   {
@@ -639,16 +637,15 @@ extern "C" int qv_tree_export(qv_ctx *c, int cap, int *parent, int *digit, int *
 // Launch the local term and the non-local sum (calc_velocity for every active
 // point).  The tree path issues no host synchronisation here; the counters
 // and the status word are read by velocity_collect.
-static int velocity_launch(qv_ctx *c) {
+// lia_done: the caller launched the ghosts and the local term together.
+static int velocity_launch(qv_ctx *c, bool lia_done = false) {
   int rc;
-  if (!c->ghosts_valid)
-    if ((rc = qv_launch_ghosts(c))) return rc;
-  QV_CUDA(c, cudaMemsetAsync(c->evals, 0, sizeof(unsigned long long), c->stream));
-  QV_CUDA(c, cudaMemsetAsync(c->evals_far, 0, sizeof(unsigned long long), c->stream));
-  QV_CUDA(c, cudaMemsetAsync(c->dstatus, 0, sizeof(int), c->stream));
-  qv_phase_begin(c, PH_LIA);
-  if ((rc = qv_launch_lia(c))) return rc;
-  qv_phase_end(c, PH_LIA);
+  QV_CUDA(c, cudaMemsetAsync(c->evals, 0, 3 * sizeof(*c->evals), c->stream));  // and the status
+  if (!lia_done) {
+    qv_phase_begin(c, PH_LIA);
+    if ((rc = c->ghosts_valid ? qv_launch_lia(c) : qv_launch_ghosts_lia(c))) return rc;
+    qv_phase_end(c, PH_LIA);
+  }
   c->nact_pending = false;
   if (c->p.velocity == QV_VEL_BS) {
     // the small sum needs no active list: its count is read with the status
@@ -674,13 +671,11 @@ static int velocity_launch(qv_ctx *c) {
 
 // Wait for the stream, read the evaluation counters and the status word.
 static int velocity_collect(qv_ctx *c, long long *eval_count) {
-  // the two counters and the status word land in one pinned buffer: three
-  // asynchronous copies and a single wait
+  // the two counters and the status word land in one pinned buffer: one
+  // asynchronous copy and a single wait
   if (!c->h_stat) QV_CUDA(c, cudaMallocHost((void **)&c->h_stat, 4 * sizeof(unsigned long long)));
   unsigned long long *hs = c->h_stat;
-  QV_CUDA(c, cudaMemcpyAsync(hs, c->evals, sizeof(*hs), cudaMemcpyDeviceToHost, c->stream));
-  QV_CUDA(c, cudaMemcpyAsync(hs + 1, c->evals_far, sizeof(*hs), cudaMemcpyDeviceToHost, c->stream));
-  QV_CUDA(c, cudaMemcpyAsync(hs + 2, c->dstatus, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  QV_CUDA(c, cudaMemcpyAsync(hs, c->evals, 3 * sizeof(*hs), cudaMemcpyDeviceToHost, c->stream));
   if (c->nact_pending)
     QV_CUDA(c, cudaMemcpyAsync(hs + 3, c->d_nact, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -737,15 +732,15 @@ extern "C" int qv_step_ab(qv_ctx *c) {
   return QV_OK;
 }
 
-static int rk3_stages(qv_ctx *c) {
+static int rk3_stages(qv_ctx *c, bool lia_done = false) {
   int rc;
   for (int stage = 0; stage < 3; stage++) {
     if (stage > 0) {
-      if ((rc = qv_launch_ghosts(c))) return rc;
+      if ((rc = qv_launch_ghosts_lia(c))) return rc;
       if (c->p.tree_theta > 0)
         if ((rc = qv_launch_tree_build(c))) return rc;
     }
-    if ((rc = velocity_launch(c))) return rc;
+    if ((rc = velocity_launch(c, stage > 0 || lia_done))) return rc;
     if ((rc = velocity_collect(c, nullptr))) return rc;
     qv_phase_begin(c, PH_UPDATE);
     if ((rc = qv_launch_rk3_stage(c, stage))) return rc;
@@ -815,8 +810,8 @@ typedef int (*step_hook)(qv_ctx *c, void *arg);
 static int step_body(qv_ctx *c, int itime, step_hook after_lines, void *arg,
                      step_hook after_insert = nullptr) {
   int rc;
-  qv_phase_begin(c, PH_GHOSTS);
-  if ((rc = qv_launch_ghosts(c))) return rc;                     // run.f90:41
+  qv_phase_begin(c, PH_GHOSTS);  // and the local term, timestep.f90:196-225
+  if ((rc = qv_launch_ghosts_lia(c))) return rc;                 // run.f90:41
   qv_phase_end(c, PH_GHOSTS);
   if (c->p.tree_theta > 0) {
     qv_phase_begin(c, PH_BUILD);
@@ -825,9 +820,9 @@ static int step_body(qv_ctx *c, int itime, step_hook after_lines, void *arg,
   }
   if (c->p.runge_kutta) {                                        // run.f90:50-54
     if ((rc = wait_pending_inputs(c))) return rc;
-    if ((rc = rk3_stages(c))) return rc;
+    if ((rc = rk3_stages(c, true))) return rc;
   } else {
-    if ((rc = velocity_launch(c))) return rc;
+    if ((rc = velocity_launch(c, true))) return rc;
     qv_phase_begin(c, PH_UPDATE);
     if ((rc = wait_pending_inputs(c))) return rc;
     if ((rc = qv_launch_ab(c))) return rc;
@@ -875,8 +870,7 @@ static int step_body(qv_ctx *c, int itime, step_hook after_lines, void *arg,
   if (after_lines)
     if ((rc = after_lines(c, arg))) return rc;
   qv_phase_begin(c, PH_WRAP);
-  if ((rc = qv_launch_ghosts(c))) return rc;                     // run.f90:75
-  if ((rc = qv_launch_wrap(c))) return rc;                       // run.f90:82-93
+  if ((rc = qv_launch_ghosts_wrap(c))) return rc;                // run.f90:75, 82-93
   qv_phase_end(c, PH_WRAP);
   c->ghosts_valid = false;
   return QV_OK;
@@ -1043,15 +1037,13 @@ extern "C" int qv_step_exchange(qv_ctx *c, int itime, int n, const qv_state *in,
 // that set them up.
 static int enqueue_fixed_step(qv_ctx *c, bool search) {
   int rc;
-  if ((rc = qv_launch_ghosts(c))) return rc;                     // run.f90:41
-  if ((rc = qv_launch_lia(c))) return rc;                        // timestep.f90:196-225
+  if ((rc = qv_launch_ghosts_lia(c))) return rc;                 // run.f90:41, timestep.f90:196-225
   if (c->p.velocity == QV_VEL_BS)
     if ((rc = qv_launch_direct(c))) return rc;                   // timestep.f90:226-258
   if ((rc = qv_launch_ab(c))) return rc;                         // timestep.f90:48-71
   if (search)
     if ((rc = qv_launch_closest(c))) return rc;                  // run.f90:63-69
-  if ((rc = qv_launch_ghosts(c))) return rc;                     // run.f90:75
-  if ((rc = qv_launch_wrap(c))) return rc;                       // run.f90:82-93
+  if ((rc = qv_launch_ghosts_wrap(c))) return rc;                // run.f90:75, 82-93
   return QV_OK;
 }
 

@@ -562,8 +562,7 @@ static int launch_step(qv_batch *b, int do_ab) {
 static int enqueue_step(qv_batch *b, int do_ab) {
   qv_ctx *c = b->c;
   int rc;
-  if ((rc = qv_launch_ghosts(c))) return rc;
-  if ((rc = qv_launch_lia(c))) return rc;
+  if ((rc = qv_launch_ghosts_lia(c))) return rc;
   if (b->nroots > 0) {
     ForestArgs f;
     f.nroots = b->nroots; f.n_fact = b->n_fact; f.roots = b->d_roots; f.fact = b->d_fact;

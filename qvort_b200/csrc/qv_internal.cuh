@@ -188,6 +188,8 @@ struct qv_ctx {
   size_t field_bytes = 0;
   double *src64 = nullptr;  // direct-sum source pack (FP64)
   float *src32 = nullptr;   // direct-sum source pack (FP32 hi/lo)
+  // One device block: the evaluation counters and, behind them, the status word
+  // (cleared and read together; evals_far and dstatus point into it).
   unsigned long long *evals = nullptr;  // device eval counter
   int *dstatus = nullptr;               // device status word
   double *dscalar = nullptr;            // device scalar scratch
@@ -251,6 +253,8 @@ void qv_phase_collect(qv_ctx *c);
 // ---------------------------------------------------------------- kernels
 int qv_launch_ghosts(qv_ctx *c);
 int qv_launch_lia(qv_ctx *c);
+int qv_launch_ghosts_lia(qv_ctx *c);   // both, in one launch
+int qv_launch_ghosts_wrap(qv_ctx *c);  // ghostp, wrap and NaN test at the end of a step
 int qv_launch_direct(qv_ctx *c);
 // whether the direct sum of n slots takes a block per target (no active list)
 bool qv_direct_small(const qv_params *p, int n);

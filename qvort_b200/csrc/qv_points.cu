@@ -37,10 +37,32 @@ static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 // get_ghost_p, src/periodic.f90:23-165: positions of the +-1 and +-2
 // neighbours, shifted by +-L on every periodic axis where they differ from
 // x_i by more than L/2 (strict comparisons).
+__device__ __forceinline__ void ghost_point(const double *__restrict__ x, const double *xi, int j,
+                                            int lo_axis, double L, double *g) {
+  const double h = L / 2.;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    g[c] = x[3 * j + c];
+    if (c >= lo_axis) {
+      if ((xi[c] - g[c]) > h)
+        g[c] = g[c] + L;
+      else if ((xi[c] - g[c]) < (-h))
+        g[c] = g[c] - L;
+    }
+  }
+}
+
+// NANS: also the end-of-step NaN test (see k_wrap), for open boundaries, which
+// have nothing else to do there.
+template <bool NANS>
 __global__ void k_ghosts(int n, const double *__restrict__ x, const int *__restrict__ inf,
                          const int *__restrict__ beh, double *gi, double *gb, double *gii,
-                         double *gbb, int lo_axis, double L) {
+                         double *gbb, int lo_axis, double L, int *status) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (NANS) {
+    const bool nan = i < n && (isnan(x[3 * i]) || isnan(x[3 * i + 1]) || isnan(x[3 * i + 2]));
+    if (__any_sync(0xffffffffu, nan) && (threadIdx.x & 31) == 0) atomicOr(status, QV_STAT_NAN);
+  }
   if (i >= n) return;
   int a = inf[i];
   if (a == 0) return;
@@ -48,21 +70,12 @@ __global__ void k_ghosts(int n, const double *__restrict__ x, const int *__restr
   int aa = inf[a - 1], bb = beh[b - 1];
   int src[4] = {a - 1, b - 1, aa - 1, bb - 1};
   double *dst[4] = {gi, gb, gii, gbb};
-  double xi[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
-  double h = L / 2.;
+  double xi[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]}, g[3];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
+    ghost_point(x, xi, src[k], lo_axis, L, g);
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      double g = x[3 * src[k] + c];
-      if (c >= lo_axis) {
-        if ((xi[c] - g) > h)
-          g = g + L;
-        else if ((xi[c] - g) < (-h))
-          g = g - L;
-      }
-      dst[k][3 * i + c] = g;
-    }
+    for (int c = 0; c < 3; c++) dst[k][3 * i + c] = g[c];
   }
 }
 
@@ -72,9 +85,9 @@ static int lo_axis_of(int bc) {
 
 int qv_launch_ghosts(qv_ctx *c) {
   if (c->n == 0) return QV_OK;
-  k_ghosts<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->x, c->infront, c->behind, c->gi,
-                                                   c->gb, c->gii, c->gbb,
-                                                   lo_axis_of(c->p.boundary), c->p.box_size);
+  k_ghosts<false><<<nblk(c->n, 256), 256, 0, c->stream>>>(
+      c->n, c->x, c->infront, c->behind, c->gi, c->gb, c->gii, c->gbb, lo_axis_of(c->p.boundary),
+      c->p.box_size, nullptr);
   QV_LAUNCH_CHECK(c);
   QV_COUNT(c, 1);
   c->ghosts_valid = true;
@@ -115,6 +128,54 @@ __global__ void k_lia(int n, const double *__restrict__ x, const int *__restrict
   if (velocity == QV_VEL_LIA || velocity == QV_VEL_OFF)
 #pragma unroll
     for (int c = 0; c < 3; c++) u[3 * i + c] = out[c];
+}
+
+// ghostp and the local term of every point in one launch: the ghosts a point's
+// term needs are its own, just gathered.  The same operations as k_ghosts and
+// k_lia one after the other.  With the closing ghosts and NaN test of open
+// systems together, and the counters and status cleared and read at once: 20
+// steps of 200 points 783 -> 721 us, a 1000-point velocity 108 -> 94 us.
+__global__ void __launch_bounds__(128) k_ghosts_lia(int n, const double *__restrict__ x,
+                                                    const int *__restrict__ inf,
+                                                    const int *__restrict__ beh, double *gi,
+                                                    double *gb, double *gii, double *gbb,
+                                                    int lo_axis, double L, double *u_li, double *u,
+                                                    int velocity, int order, int fixed_beta,
+                                                    double quant_circ, double corea) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int a = inf[i];
+  if (a == 0) return;
+  const int b = beh[i];
+  const int src[4] = {a - 1, b - 1, inf[a - 1] - 1, beh[b - 1] - 1};
+  double *dst[4] = {gi, gb, gii, gbb};
+  const double X[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
+  double g[4][3], out[3];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    ghost_point(x, X, src[k], lo_axis, L, g[k]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) dst[k][3 * i + c] = g[k][c];
+  }
+  lia_term(velocity, order, fixed_beta, quant_circ, corea, X, g[0], g[1], g[2], g[3], out);
+#pragma unroll
+  for (int c = 0; c < 3; c++) u_li[3 * i + c] = out[c];
+  if (velocity == QV_VEL_LIA || velocity == QV_VEL_OFF)
+#pragma unroll
+    for (int c = 0; c < 3; c++) u[3 * i + c] = out[c];
+}
+
+int qv_launch_ghosts_lia(qv_ctx *c) {
+  if (c->n == 0) return QV_OK;
+  k_ghosts_lia<<<nblk(c->n, 128), 128, 0, c->stream>>>(
+      c->n, c->x, c->infront, c->behind, c->gi, c->gb, c->gii, c->gbb, lo_axis_of(c->p.boundary),
+      c->p.box_size, c->u_li, c->u, c->p.velocity, c->p.deriv_order, c->p.fixed_lia_beta,
+      c->p.quant_circ, c->p.corea);
+  QV_LAUNCH_CHECK(c);
+  QV_COUNT(c, 1);
+  c->ghosts_valid = true;
+  c->ghosts_stored = true;
+  return QV_OK;
 }
 
 int qv_launch_lia(qv_ctx *c) {
@@ -226,6 +287,25 @@ int qv_launch_wrap(qv_ctx *c) {
                                                  c->p.box_size, c->dstatus);
   QV_LAUNCH_CHECK(c);
   QV_COUNT(c, 1);
+  return QV_OK;
+}
+
+// The end of a step: ghostp (src/run.f90:75), then the wrap and the NaN test.  An
+// open system wraps nothing, so one launch does both there.
+int qv_launch_ghosts_wrap(qv_ctx *c) {
+  int rc;
+  if (c->p.boundary != QV_BC_OPEN) {
+    if ((rc = qv_launch_ghosts(c))) return rc;
+    return qv_launch_wrap(c);
+  }
+  if (c->n == 0) return QV_OK;
+  k_ghosts<true><<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->x, c->infront, c->behind, c->gi,
+                                                         c->gb, c->gii, c->gbb, 3, c->p.box_size,
+                                                         c->dstatus);
+  QV_LAUNCH_CHECK(c);
+  QV_COUNT(c, 1);
+  c->ghosts_valid = true;
+  c->ghosts_stored = true;
   return QV_OK;
 }
 

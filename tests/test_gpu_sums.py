@@ -304,3 +304,21 @@ def test_direct_fp64_either_side_of_the_small_sum(n, bc):
     g = O.ghosts(p, w.x, w.infront, w.behind)
     ou = O.velocity(p, w.x, w.infront, w.behind, g, nthreads=8)[0]
     assert len(x) and np.abs(u - ou)[at].max() <= 1e-11 * np.abs(ou[at]).max()
+
+
+@pytest.mark.parametrize("bc", ["open", "openx", "periodic"])
+@pytest.mark.parametrize("velocity,order", [("BS", 2), ("BS", 4), ("LIA", 4), ("Off", 2)])
+def test_ghosts_and_local_term_in_one_launch_equal_two(velocity, order, bc):
+    """A velocity that gathers its own ghosts takes them and the local term in one
+    kernel, one on given ghosts the local term alone: the same bits, and the
+    oracle's ghosts."""
+    w = _ring_pair(301)
+    kw = dict(velocity=velocity, deriv_order=order, boundary=bc, precision="fp64")
+    a, b = _ctx(w, **kw), _ctx(w, **kw)
+    b.ghosts()
+    ua, la, *_ = a.velocity()
+    ub, lb, *_ = b.velocity()
+    assert np.array_equal(ua, ub) and np.array_equal(la, lb)
+    og = O.ghosts(O.params(**dict(w.params, boundary=bc)), w.x, w.infront, w.behind)
+    for g, h, o in zip(a.get_ghosts(), b.get_ghosts(), og):
+        assert np.array_equal(g, h) and np.array_equal(g, o)
