@@ -1045,14 +1045,3 @@ extern "C" int qv_field_velocity(qv_ctx *c, int m, const double *pts, int grad_i
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
   return QV_OK;
 }
-
-extern "C" int qv_velocity_device(qv_ctx *c, double *u_out) {
-  if (!c || !u_out) return QV_ERR_ARG;
-  int rc = qv_velocity(c, nullptr, nullptr, nullptr, nullptr);
-  if (rc) return rc;
-  if (c->n)
-    QV_CUDA(c, cudaMemcpyAsync(u_out, c->u, sizeof(double) * 3 * (size_t)c->n,
-                               cudaMemcpyDeviceToDevice, c->stream));
-  QV_CUDA(c, cudaStreamSynchronize(c->stream));
-  return QV_OK;
-}

@@ -311,6 +311,42 @@ static int stage_links(qv_ctx *c, int n, const int *inf, const int *beh, const i
   return QV_OK;
 }
 
+// What a new point set starts from, in one launch: the checked links taken from
+// their staging buffer (and closest, where given), everything else zeroed.  As
+// up to eleven copies and fills this took longer than a small system's velocity.
+// A caller's device arrays are still copied by the runtime, which refuses a
+// pointer that is none.
+struct LoadArgs {
+  int n, nz;     // slots; vector arrays to zero
+  double *z[6];
+  const int *inf_s, *beh_s, *closest_s;  // staged links or nullptr; nullptr closest_s: zeros
+  int *inf, *beh, *closest;              // closest nullptr: left alone
+  double *closestd;
+};
+__global__ void k_load_points(LoadArgs a) {
+  const size_t n3 = 3 * (size_t)a.n, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n3; e += step) {
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      if (k < a.nz) a.z[k][e] = 0.;
+    if (e < (size_t)a.n) {
+      if (a.inf_s) {
+        a.inf[e] = a.inf_s[e];
+        a.beh[e] = a.beh_s[e];
+      }
+      a.closestd[e] = 0.;
+      if (a.closest) a.closest[e] = a.closest_s ? a.closest_s[e] : 0;
+    }
+  }
+}
+static int load_points(qv_ctx *c, const LoadArgs &a) {
+  const int grid = (int)std::min<long>((3L * a.n + 255) / 256, 8L * c->sm_count);
+  k_load_points<<<grid, 256, 0, c->stream>>>(a);
+  QV_LAUNCH_CHECK(c);
+  QV_COUNT(c, 1);
+  return QV_OK;
+}
+
 static int set_points_impl(qv_ctx *c, int n, const double *x, const int *inf, const int *beh,
                            cudaMemcpyKind kind) {
   if (n < 0 || (n > 0 && (!x || !inf || !beh))) return qv_fail(c, QV_ERR_ARG, "bad points");
@@ -323,15 +359,15 @@ static int set_points_impl(qv_ctx *c, int n, const double *x, const int *inf, co
   if (rc) return rc;
   c->n = n;
   if (n > 0) {
-    size_t v = sizeof(double) * 3 * (size_t)n;
-    QV_CUDA(c, cudaMemcpyAsync(c->x, x, v, kind, c->stream));
-    const cudaMemcpyKind lk = host ? cudaMemcpyDeviceToDevice : kind;
-    QV_CUDA(c, cudaMemcpyAsync(c->infront, host ? c->lk : inf, sizeof(int) * n, lk, c->stream));
-    QV_CUDA(c, cudaMemcpyAsync(c->behind, host ? c->lk + n : beh, sizeof(int) * n, lk, c->stream));
-    double *zv[] = {c->u, c->u1, c->u2, c->u3, c->u_li, c->u_bs};
-    for (double *q : zv) QV_CUDA(c, cudaMemsetAsync(q, 0, v, c->stream));
-    QV_CUDA(c, cudaMemsetAsync(c->closest, 0, sizeof(int) * n, c->stream));
-    QV_CUDA(c, cudaMemsetAsync(c->closestd, 0, sizeof(double) * n, c->stream));
+    QV_CUDA(c, cudaMemcpyAsync(c->x, x, sizeof(double) * 3 * (size_t)n, kind, c->stream));
+    if (!host) {
+      QV_CUDA(c, cudaMemcpyAsync(c->infront, inf, sizeof(int) * n, kind, c->stream));
+      QV_CUDA(c, cudaMemcpyAsync(c->behind, beh, sizeof(int) * n, kind, c->stream));
+    }
+    const LoadArgs a = {n, 6, {c->u, c->u1, c->u2, c->u3, c->u_li, c->u_bs},
+                        host ? c->lk : nullptr, c->lk + n, nullptr, c->infront, c->behind,
+                        c->closest, c->closestd};
+    if ((rc = load_points(c, a))) return rc;
   }
   c->ghosts_valid = false;
   c->ghosts_stored = false;
@@ -417,22 +453,17 @@ extern "C" int qv_set_state(qv_ctx *c, int n, const qv_state *s) {
   if (n > 0) {
     const size_t v = sizeof(double) * 3 * (size_t)n;
     const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
-    const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
     QV_CUDA(c, cudaMemcpyAsync(c->x, s->x, v, h2d, c->stream));
-    QV_CUDA(c, cudaMemcpyAsync(c->infront, c->lk, sizeof(int) * n, d2d, c->stream));
-    QV_CUDA(c, cudaMemcpyAsync(c->behind, c->lk + n, sizeof(int) * n, d2d, c->stream));
     const double *hs[] = {s->u1, s->u2, s->u3};
     double *hd[] = {c->u1, c->u2, c->u3};
+    LoadArgs a = {n, 3, {c->u, c->u_li, c->u_bs}, c->lk, c->lk + n,
+                  s->closest ? c->lk + 2 * (size_t)n : nullptr, c->infront, c->behind, c->closest,
+                  c->closestd};
     for (int k = 0; k < 3; k++) {
       if (hs[k]) QV_CUDA(c, cudaMemcpyAsync(hd[k], hs[k], v, h2d, c->stream));
-      else QV_CUDA(c, cudaMemsetAsync(hd[k], 0, v, c->stream));
+      else a.z[a.nz++] = hd[k];
     }
-    if (s->closest)
-      QV_CUDA(c, cudaMemcpyAsync(c->closest, c->lk + 2 * (size_t)n, sizeof(int) * n, d2d, c->stream));
-    else QV_CUDA(c, cudaMemsetAsync(c->closest, 0, sizeof(int) * n, c->stream));
-    double *zv[] = {c->u, c->u_li, c->u_bs};
-    for (double *q : zv) QV_CUDA(c, cudaMemsetAsync(q, 0, v, c->stream));
-    QV_CUDA(c, cudaMemsetAsync(c->closestd, 0, sizeof(double) * n, c->stream));
+    if ((rc = load_points(c, a))) return rc;
   }
   c->ghosts_valid = false;
   c->ghosts_stored = false;
@@ -723,6 +754,17 @@ extern "C" int qv_velocity(qv_ctx *c, double *u, double *u_li, double *u_bs, lon
   return velocity_collect(c, eval_count);
 }
 
+// The velocities into a device array, in one wait.
+extern "C" int qv_velocity_device(qv_ctx *c, double *u_out) {
+  if (!c || !u_out) return QV_ERR_ARG;
+  if (c->n == 0) return QV_OK;
+  int rc = velocity_launch(c);
+  if (rc) return rc;
+  QV_CUDA(c, cudaMemcpyAsync(u_out, c->u, sizeof(double) * 3 * (size_t)c->n,
+                             cudaMemcpyDeviceToDevice, c->stream));
+  return velocity_collect(c, nullptr);
+}
+
 extern "C" int qv_step_ab(qv_ctx *c) {
   QV_CHECK_CTX(c);
   int rc = qv_launch_ab(c);
@@ -961,13 +1003,10 @@ extern "C" int qv_step_exchange(qv_ctx *c, int itime, int n, const qv_state *in,
     const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
     // what the step reads first, here; the AB history and closest on a side
     // stream, awaited by the update
-    const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
     QV_CUDA(c, cudaMemcpyAsync(c->x, in->x, v, h2d, c->stream));
-    QV_CUDA(c, cudaMemcpyAsync(c->infront, c->lk, sizeof(int) * n, d2d, c->stream));
-    QV_CUDA(c, cudaMemcpyAsync(c->behind, c->lk + n, sizeof(int) * n, d2d, c->stream));
-    double *zv[] = {c->u, c->u_li, c->u_bs};
-    for (double *q : zv) QV_CUDA(c, cudaMemsetAsync(q, 0, v, c->stream));
-    QV_CUDA(c, cudaMemsetAsync(c->closestd, 0, sizeof(double) * n, c->stream));
+    const LoadArgs a = {n, 3, {c->u, c->u_li, c->u_bs}, c->lk, c->lk + n, nullptr,
+                        c->infront, c->behind, nullptr, c->closestd};
+    if ((rc = load_points(c, a))) return rc;
     cudaStream_t sa = c->aux[2];
     QV_CUDA(c, cudaEventRecord(c->ev_fork2, c->stream));
     QV_CUDA(c, cudaStreamWaitEvent(sa, c->ev_fork2, 0));
