@@ -170,7 +170,7 @@ __device__ __forceinline__ void walk_item(const BatchArgs &a, StkEnt *st, int g,
       evf += far ? 1u : 0u;
       if (far && node >= a.nroots) {  // a root's moments are zero
         const WPay32 &P = a.p32[node];
-        float rd = rsqrtf(d2);
+        float rd = rsqrt_normal(d2);  // as in the single walk
         float rd2 = rd * rd, rd3 = rd2 * rd, rd5 = rd3 * rd2;
         float z0 = fmaf(v0, P.C[0], fmaf(v1, P.C[3], v2 * P.C[6]));
         float z1 = fmaf(v0, P.C[1], fmaf(v1, P.C[4], v2 * P.C[7]));

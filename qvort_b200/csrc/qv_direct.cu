@@ -481,14 +481,17 @@ __device__ __forceinline__ void seg_terms(float r1s, float r2s, float dd, float 
   oz = g * cz;
 }
 
-// seg_terms where cos is known to be positive: f / (1 + cos).
+// seg_terms where cos is known to be positive and the squared distances are
+// normal numbers: f / (1 + cos).  With the square roots' and the division's
+// handling of subnormal operands left out, 24,700 points and 27 images take 13.0
+// ms, not 15.1; the MUFU pipe (three of them a pair) would take 10.6.
 __device__ __forceinline__ void seg_terms_pos(float r1s, float r2s, float dd, float cx, float cy,
                                               float cz, float &ox, float &oy, float &oz) {
-  const float ra = rsqrtf(r1s), rb = rsqrtf(r2s);
+  const float ra = rsqrt_normal(r1s), rb = rsqrt_normal(r2s);
   const float q = ra * rb;
   const float cs = dd * q;
   const float f = (ra + rb) * q;
-  const float g = __fdividef(f, 1.f + cs);
+  const float g = f * rcp_normal(1.f + cs);
   ox = g * cx;
   oy = g * cy;
   oz = g * cz;
@@ -602,7 +605,8 @@ __global__ void __launch_bounds__(DTILE) k_direct32(int na, const int *__restric
         m1 += PY == 3 ? fminf(fminf(a1y[0], a1y[1]), a1y[2]) : a1y[1];
         m1 += PZ == 3 ? fminf(fminf(a1z[0], a1z[1]), a1z[2]) : a1z[1];
         const float ss = fmaf(sx, sx, fmaf(sy, sy, sz * sz));
-        const bool fast = __all_sync(0xffffffffu, skip_src || m1 > 1.0001f * ss);
+        // the lower bound keeps |R1|^2 and, at least 2.5e-9 of it, |R2|^2 normal
+        const bool fast = __all_sync(0xffffffffu, skip_src || (m1 > 1.0001f * ss && m1 > 1e-25f));
         if (skip_src) continue;
         float ix = 0.f, iy = 0.f, iz = 0.f;
         auto images = [&](auto term) {

@@ -315,6 +315,20 @@ int qv_forest_build(qv_ctx *c, const ForestArgs &f);
 #define QV_CTL_NNODES 0
 
 // ---------------------------------------------------------------- helpers
+// 1/sqrt(a) and 1/a of a normal number: what rsqrtf and the fast division give
+// there, without their handling of subnormal operands (three instructions of a
+// square root's four).  A subnormal a gives infinity.
+__device__ __forceinline__ float rsqrt_normal(float a) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float rcp_normal(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
 // Straight-segment Biot-Savart term in FP32, without the G/(4 pi) factor:
 //   (|R1|+|R2|) / (|R1||R2| (|R1||R2| + R1.R2)) * (R1 x R2)
 // (src/tree.f90:380-390), written with q = 1/(|R1||R2|) as

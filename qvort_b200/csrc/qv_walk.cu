@@ -462,7 +462,8 @@ __device__ __forceinline__ void walk_task1(const WalkArgs &a, StkEnt *st, int la
       evf += far ? 1u : 0u;
       if (far && node != 0) {  // the root's moments are zero
         const WPay32 &P = a.p32[node];
-        float rd = rsqrtf(d2);
+        // below 1e-25 the powers overflow either way
+        float rd = rsqrt_normal(d2);
         float rd2 = rd * rd, rd3 = rd2 * rd, rd5 = rd3 * rd2;
         float z0 = fmaf(v0, P.C[0], fmaf(v1, P.C[3], v2 * P.C[6]));
         float z1 = fmaf(v0, P.C[1], fmaf(v1, P.C[4], v2 * P.C[7]));
@@ -675,7 +676,8 @@ __device__ __forceinline__ void walk_task2(const WalkArgs &a, StkEnt *st, int la
       evfb += fb ? 1u : 0u;
       if ((fa || fb) && node != 0) {  // the root's moments are zero
         const WPay32 &P = a.p32[node];
-        const float2 rd = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+        // below 1e-25 the powers overflow either way
+        const float2 rd = make_float2(rsqrt_normal(d2.x), rsqrt_normal(d2.y));
         const float2 rd2 = mul2(rd, rd), rd3 = mul2(rd2, rd), rd5 = mul2(rd3, rd2);
         const float2 z0 = fma2(v0, bc2(P.C[0]), fma2(v1, bc2(P.C[3]), mul2(v2, bc2(P.C[6]))));
         const float2 z1 = fma2(v0, bc2(P.C[1]), fma2(v1, bc2(P.C[4]), mul2(v2, bc2(P.C[7]))));
