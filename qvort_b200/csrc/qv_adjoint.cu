@@ -712,18 +712,21 @@ __global__ void __launch_bounds__(FW * 32) k_field(int m, const double *__restri
     if (lane == k) o[k] = v[k];
 }
 
-// Sum of the chunks' partial values in chunk order: out = u (3m), du/dx (9m).
+// Sum of the chunks' partial values, a warp per value (lanes stride over the
+// chunks, in a fixed order): out = u (3m), du/dx (9m).
 __global__ void k_field_reduce(int m, int nchunk, const double *__restrict__ part, double scale,
                                double *out) {
-  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long e = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   const long tot = (long)m * FV;
   if (e >= tot) return;
   double s = 0.;
-#pragma unroll 8
-  for (int k = 0; k < nchunk; k++) s += part[k * tot + e];
+  for (int k = lane; k < nchunk; k += 32) s += part[k * tot + e];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   const long t = e / FV;
   const int k = (int)(e - t * FV);
-  out[k < 3 ? 3 * t + k : 3L * m + 9 * t + (k - 3)] = s * scale;
+  if (lane == 0) out[k < 3 ? 3 * t + k : 3L * m + 9 * t + (k - 3)] = s * scale;
 }
 
 // ------------------------------------------------------------------ host side
@@ -1035,7 +1038,7 @@ extern "C" int qv_field_velocity(qv_ctx *c, int m, const double *pts, int grad_i
     default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", c->p.boundary);
   }
   QV_LAUNCH_CHECK(c);
-  k_field_reduce<<<nblk((long)nv, 128), 128, 0, c->stream>>>(
+  k_field_reduce<<<(unsigned)((nv * 32 + 255) / 256), 256, 0, c->stream>>>(
       m, nchunk, part, c->p.quant_circ / (4. * QV_PI), du);
   QV_LAUNCH_CHECK(c);
   QV_COUNT(c, 2);

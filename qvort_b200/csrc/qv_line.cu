@@ -449,7 +449,8 @@ __global__ void __launch_bounds__(PC_T) k_precon_scan(LineArgs a, const RecEval 
 // --------------------------------------------------------------- host
 // Flag and list arrays for n slots (the slot count at the start of a scan).
 static int line_reserve(qv_ctx *c) {
-  size_t n = (size_t)std::max(c->n, 1);
+  // a multiple of four, so that every flag array starts 16-byte aligned (k_compact1)
+  size_t n = ((size_t)std::max(c->n, 1) + 3) / 4 * 4;
   if (c->line_cap >= n && c->line_st) return QV_OK;
   int rc;
   if ((rc = qv_grow(c, (void **)&c->line_flags, sizeof(int) * 4 * n))) return rc;

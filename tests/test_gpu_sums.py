@@ -322,3 +322,32 @@ def test_ghosts_and_local_term_in_one_launch_equal_two(velocity, order, bc):
     og = O.ghosts(O.params(**dict(w.params, boundary=bc)), w.x, w.infront, w.behind)
     for g, h, o in zip(a.get_ghosts(), b.get_ghosts(), og):
         assert np.array_equal(g, h) and np.array_equal(g, o)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 127, 128, 129, 4095, 4097, 8190, 65535, 65536, 65537])
+def test_active_list_at_its_edges(n):
+    """The ordered list of the active slots (one block up to 65,536 slots): points
+    with empty slots among them keep their order -- a mixed direct sum over the
+    list gives each filament's own velocity wherever its slots lie."""
+    from qvort_b200 import lib as L
+
+    m = min(n, 12)
+    w = W.ring(m, 0.01, 1e-5, seed=2) if m > 4 else None
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-0.04, 0.04, (n, 3))
+    inf, beh = np.zeros(n, np.int32), np.zeros(n, np.int32)
+    at = np.sort(rng.choice(n, m, replace=False))
+    at[-1] = n - 1
+    if m > 4:
+        x[at] = w.x
+        inf[at], beh[at] = at[w.infront - 1] + 1, at[w.behind - 1] + 1
+    kw = dict(boundary="open", velocity="BS", tree_theta=0.0, box_size=0.1, precision="mixed",
+              quant_circ=W.GAMMA_HE4, corea=W.CORE_A)
+    c = L.Context(L.default_params(**kw))
+    c.set_points(x, inf, beh)
+    u, _, _, ev = c.velocity()
+    assert ev == (m * m if m > 4 else 0)
+    if m > 4:
+        d = L.Context(L.default_params(**kw))
+        d.set_points(w.x, w.infront, w.behind)
+        assert np.array_equal(u[at], d.velocity()[0])
