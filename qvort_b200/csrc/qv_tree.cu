@@ -42,7 +42,6 @@ static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 #define CTL_NGLOB 1     // nodes made by the grid-wide levels (all nodes of > LCH points)
 #define CTL_LOCALD 2    // first block-local level, -1 if none
 #define CTL_OVERFLOW 3  // 1 = node capacity, 2 = level capacity
-#define CTL_NMID 7      // number of nodes handled by the second k_moments_big
 #define CTL_DEPTH 4
 #define CTL_NBIG 5      // number of nodes handled by k_moments_big
 #define CTL_NACT 6      // active points of this build
@@ -694,7 +693,6 @@ __global__ void __launch_bounds__(BT) k_build_local(BuildArgs a) {
 // chain lanes fed from shared memory while other warps gather and precompute.
 #define MW 8      // warps per block (small nodes: one warp per node)
 #define BIGN LCH  // nodes with more points: a block each, early (all made grid-wide)
-#define MIDN 128  // nodes with more points (up to BIGN): a block each, after the tree
 #define TN 8      // nodes with at most this many points: a thread each
 #define MC 256    // points per shared-memory chunk in the block kernel
 #define MBT 512   // threads of the block kernel: warp 0 runs the chains, the rest gather
@@ -736,7 +734,8 @@ __device__ __forceinline__ double chain15(double acc, const double *rows, int st
   return acc;
 }
 
-// One thread per node of at most TN points, then one warp per node of at most MIDN points.
+// One thread per node of at most TN points, then one warp per node of at most
+// BIGN points.
 __global__ void __launch_bounds__(MW * 32) k_moments(const int *__restrict__ ctl, int cap_nodes, int k0,
                                                      const int *__restrict__ level,
                                                      const int *__restrict__ start,
@@ -801,48 +800,61 @@ __global__ void __launch_bounds__(MW * 32) k_moments(const int *__restrict__ ctl
         C[9 * kl + 3 * mm + kk] = __dsub_rn(aC[3 * mm + kk], __dmul_rn(cm[mm], ai[kk]));
     first[kl] = idx0;
   }
-  // nodes of TN+1..MIDN points: one warp per node, the next 32 points' gather
-  // in flight while the chains run over the current 32
-  for (int k = k0 + blockIdx.x * MW + wid; k < n_nodes; k += gridDim.x * MW) {
-    int s = start[k], n = count[k];
-    if (n <= TN || n > MIDN) continue;
-    const int *o = ord + (size_t)level[k] * cap_pts + s;
-    double acc = 0.;
-    double X[3] = {0., 0., 0.}, G[3] = {0., 0., 0.};
-    if (lane < n) {
-      const int idx = o[lane];
-#pragma unroll
-      for (int c = 0; c < 3; c++) { X[c] = x[3 * idx + c]; G[c] = gi[3 * idx + c]; }
-    }
-    for (int base = 0; base < n; base += 32) {
-      const int m = min(32, n - base);
-      if (lane < m) {
-        double *b = buf[wid][lane];
-#pragma unroll
-        for (int c = 0; c < 3; c++) { b[c] = X[c]; b[3 + c] = G[c]; }
-#pragma unroll
-        for (int mm = 0; mm < 3; mm++)
-#pragma unroll
-          for (int kk = 0; kk < 3; kk++) b[6 + 3 * mm + kk] = __dmul_rn(X[mm], __dsub_rn(G[kk], X[kk]));
-      }
-      __syncwarp();
-      if (base + 32 + lane < n) {
-        const int idx = o[base + 32 + lane];
+  // nodes of TN+1..BIGN points: one warp per node, the next 32 points' gather
+  // in flight while the chains run over the current 32.  A warp reads the counts
+  // of its next 32 nodes at once, one a lane: read one at a time, the latency of
+  // the many that fall to the threads above was a third of this kernel (162 trees
+  // of 0.7M points together: 287 -> 182 us).  A warp has its chain as fast as a
+  // block of the big-chain kernel has, and 24 of them share an SM where two
+  // blocks did: with the nodes of 129 to 512 points here and not in a launch of
+  // blocks of their own, a step of those trees took 3.68 ms, not 3.77.
+  const long stride = gridDim.x * MW;
+  for (long kb = k0 + blockIdx.x * MW + wid; kb < n_nodes; kb += 32 * stride) {
+    const long kl = kb + stride * lane;
+    const int nl = kl < n_nodes ? count[kl] : 0;
+    unsigned todo = __ballot_sync(0xffffffffu, nl > TN && nl <= BIGN);
+    for (; todo; todo &= todo - 1) {
+      const int t = __ffs(todo) - 1;
+      const int k = (int)(kb + stride * t), n = __shfl_sync(0xffffffffu, nl, t);
+      const int s = start[k];
+      const int *o = ord + (size_t)level[k] * cap_pts + s;
+      double acc = 0.;
+      double X[3] = {0., 0., 0.}, G[3] = {0., 0., 0.};
+      if (lane < n) {
+        const int idx = o[lane];
 #pragma unroll
         for (int c = 0; c < 3; c++) { X[c] = x[3 * idx + c]; G[c] = gi[3 * idx + c]; }
       }
-      if (lane < 15) acc = chain15(acc, &buf[wid][0][0], 15, m, lane);
-      __syncwarp();
+      for (int base = 0; base < n; base += 32) {
+        const int m = min(32, n - base);
+        if (lane < m) {
+          double *b = buf[wid][lane];
+#pragma unroll
+          for (int c = 0; c < 3; c++) { b[c] = X[c]; b[3 + c] = G[c]; }
+#pragma unroll
+          for (int mm = 0; mm < 3; mm++)
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) b[6 + 3 * mm + kk] = __dmul_rn(X[mm], __dsub_rn(G[kk], X[kk]));
+        }
+        __syncwarp();
+        if (base + 32 + lane < n) {
+          const int idx = o[base + 32 + lane];
+#pragma unroll
+          for (int c = 0; c < 3; c++) { X[c] = x[3 * idx + c]; G[c] = gi[3 * idx + c]; }
+        }
+        if (lane < 15) acc = chain15(acc, &buf[wid][0][0], 15, m, lane);
+        __syncwarp();
+      }
+      double cm = lane < 3 ? __ddiv_rn(acc, (double)n) : 0.;
+      // C(i,k) -= cent_i circ_k  (lane 6+3i+k)
+      int ci = (lane - 6) / 3, ck = (lane - 6) % 3;
+      double cen = __shfl_sync(0xffffffffu, cm, lane >= 6 && lane < 15 ? ci : 0);
+      double cir = __shfl_sync(0xffffffffu, acc, lane >= 6 && lane < 15 ? 3 + ck : 0);
+      if (lane < 3) cent[3 * k + lane] = cm;
+      else if (lane < 6) circ[3 * k + lane - 3] = acc;
+      else if (lane < 15) C[9 * k + 3 * ci + ck] = __dsub_rn(acc, __dmul_rn(cen, cir));
+      if (lane == 0) first[k] = o[0];
     }
-    double cm = lane < 3 ? __ddiv_rn(acc, (double)n) : 0.;
-    // C(i,k) -= cent_i circ_k  (lane 6+3i+k)
-    int ci = (lane - 6) / 3, ck = (lane - 6) % 3;
-    double cen = __shfl_sync(0xffffffffu, cm, lane >= 6 && lane < 15 ? ci : 0);
-    double cir = __shfl_sync(0xffffffffu, acc, lane >= 6 && lane < 15 ? 3 + ck : 0);
-    if (lane < 3) cent[3 * k + lane] = cm;
-    else if (lane < 6) circ[3 * k + lane - 3] = acc;
-    else if (lane < 15) C[9 * k + 3 * ci + ck] = __dsub_rn(acc, __dmul_rn(cen, cir));
-    if (lane == 0) first[k] = o[0];
   }
 }
 
@@ -1693,39 +1705,30 @@ int qv_launch_tree_build(qv_ctx *c) {
     QV_COUNT(c, 1);
     qv_phase_end_async(c, PH_BUILD_LEVELS);
     qv_phase_begin(c, PH_BUILD_MOMENTS);
-    // After the local levels, on a third stream: the control block to the host
-    // and the moments of the nodes of MIDN..BIGN points (a block each); here,
-    // the warp-per-node moments.  Every moment kernel packs the nodes it
-    // finishes; the root is packed once its centroid (second stream) is in.
+    // After the local levels, on a third stream, the control block to the host;
+    // here, the moments of the nodes of at most BIGN points and their packs.  The
+    // root is packed once its centroid (second stream) is in.
     QV_CUDA(c, cudaEventRecord(c->ev_fork2, c->stream));
     QV_CUDA(c, cudaStreamWaitEvent(c->aux[2], c->ev_fork2, 0));
     QV_CUDA(c, cudaMemcpyAsync(t.h_ctl, t.ctl, sizeof(int) * CTL_SIZE, cudaMemcpyDeviceToHost,
                                c->aux[2]));
     QV_CUDA(c, cudaEventRecord(t.ev_ctl, c->aux[2]));
-    QV_CUDA(c, cudaMemsetAsync(t.ctl + CTL_NMID, 0, sizeof(int), c->aux[2]));
-    k_list_big<<<4 * c->sm_count, 256, 0, c->aux[2]>>>(t.ctl, t.cap_nodes, 1, t.count, t.rs9,
-                                                        t.ctl + CTL_NMID, MIDN, BIGN, 0, 0);
-    k_moments_big<<<2 * c->sm_count, MBT, 2 * MC * 15 * sizeof(double), c->aux[2]>>>(
-        t.rs9, t.ctl + CTL_NMID, t.level, t.start, t.count, t.ord, t.cap_pts, c->x, c->gi,
-        t.cent, t.circ, t.C, t.first, 0, pk, 1);
-    QV_CUDA(c, cudaEventRecord(c->ev_join[2], c->aux[2]));
-    QV_COUNT(c, 2);
     k_moments<<<16 * c->sm_count, MW * 32, 0, c->stream>>>(t.ctl, t.cap_nodes, 1, t.level, t.start,
                                                            t.count, t.ord, t.cap_pts, c->x, c->gi,
                                                            t.cent, t.circ, t.C, t.first);
     QV_LAUNCH_CHECK(c);
-    // the packs of those nodes (of at most MIDN points) here, while the longer
-    // chains run on; the chain kernels pack the nodes they finish.  Four times
+    // the packs of those nodes here, while the longer chains run on; the
+    // big-chain kernel packs the nodes it finishes.  Four times
     // the blocks of a full pack: each thread's few nodes are dependent loads
     // (first point, its links), and more of them in flight shortened this pass
     // by 0.13 ms at 0.8M points.
     k_pack_nodes<<<16 * c->sm_count, 128, 0, c->stream>>>(t.ctl, t.cap_nodes, pk, nullptr, t.cent,
-                                                           MIDN);
+                                                           BIGN);
     QV_LAUNCH_CHECK(c);
     QV_COUNT(c, 2);
     QV_CUDA(c, cudaEventRecord(c->ev_join[0], c->aux[0]));
     QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[0], 0));
-    QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[2], 0));
+    QV_CUDA(c, cudaStreamWaitEvent(c->stream, t.ev_ctl, 0));
     if (!spec) QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[1], 0));
     if (late) QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[4], 0));
     // every other node was packed by the kernel that summed its moments
@@ -1858,20 +1861,14 @@ int qv_forest_build(qv_ctx *c, const ForestArgs &f) {
   QV_CUDA(c, cudaEventRecord(c->ev_join[0], c->aux[0]));
   k_build_local<<<std::max(1, std::min(nblk(f.n_fact, LCH), 2 * c->sm_count)), BT, LOCAL_SMEM,
                   c->stream>>>(a);
-  QV_CUDA(c, cudaMemsetAsync(t.ctl + CTL_NMID, 0, sizeof(int), c->stream));
-  k_list_big<<<4 * c->sm_count, 256, 0, c->stream>>>(t.ctl, t.cap_nodes, f.nroots, t.count, t.rs9,
-                                                      t.ctl + CTL_NMID, MIDN, BIGN, 0, 0);
-  k_moments_big<<<2 * c->sm_count, MBT, 2 * MC * 15 * sizeof(double), c->stream>>>(
-      t.rs9, t.ctl + CTL_NMID, t.level, t.start, t.count, t.ord, t.cap_pts, c->x, c->gi, t.cent,
-      t.circ, t.C, t.first, 0, pk, 0);
   k_moments<<<16 * c->sm_count, MW * 32, 0, c->stream>>>(t.ctl, t.cap_nodes, f.nroots, t.level,
                                                          t.start, t.count, t.ord, t.cap_pts, c->x,
                                                          c->gi, t.cent, t.circ, t.C, t.first);
   QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[0], 0));
   QV_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join[1], 0));
-  k_pack_nodes<<<4 * c->sm_count, 128, 0, c->stream>>>(t.ctl, t.cap_nodes, pk, nullptr, t.cent,
-                                                        INT_MAX);
+  k_pack_nodes<<<16 * c->sm_count, 128, 0, c->stream>>>(t.ctl, t.cap_nodes, pk, nullptr, t.cent,
+                                                         INT_MAX);
   QV_LAUNCH_CHECK(c);
-  QV_COUNT(c, 10);
+  QV_COUNT(c, 8);
   return QV_OK;
 }

@@ -351,3 +351,34 @@ def test_active_list_at_its_edges(n):
         d = L.Context(L.default_params(**kw))
         d.set_points(w.x, w.infront, w.behind)
         assert np.array_equal(u[at], d.velocity()[0])
+
+
+def test_tree_moments_at_the_kernels_node_sizes():
+    """Nodes of the sizes where one moment kernel hands over to the next (8 | 9
+    points, 32 | 33, 512 | 513) and around a warp's 32-point pieces: every node's
+    moments bit for bit the oracle's."""
+    from qvort_b200 import lib as L
+
+    sizes = [1, 2, 8, 9, 31, 32, 33, 64, 65, 127, 128, 129, 511, 512, 513, 640]
+    rng = np.random.default_rng(9)
+    cells = rng.permutation(64)[:len(sizes)]  # one of the 4^3 cells of level 2 each
+    x = []
+    for m, q in zip(sizes, cells):
+        corner = np.array([q % 4, q // 4 % 4, q // 16]) * 0.025 - 0.05
+        x.append(corner + rng.uniform(0.001, 0.024, (m, 3)))
+    x = np.concatenate(x)[rng.permutation(sum(sizes))]
+    n = len(x)
+    k = np.arange(n)
+    inf, beh = ((k + 1) % n + 1).astype(np.int32), ((k - 1) % n + 1).astype(np.int32)
+    kw = dict(boundary="open", velocity="Tree", tree_theta=0.4, box_size=0.1)
+    c = L.Context(L.default_params(**kw))
+    c.set_points(x, inf, beh)
+    c.ghosts()
+    c.build_tree()
+    got = c.tree_export()
+    p = O.params(**kw)
+    want = O.Tree(p, x, O.ghosts(p, x, inf, beh)[0], inf).export()
+    assert set(sizes) <= set(got["pcount"][got["depth"] == 2])
+    assert set(got) == set(want)
+    for name in want:
+        np.testing.assert_array_equal(got[name], want[name], err_msg=name)
