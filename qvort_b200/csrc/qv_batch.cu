@@ -249,6 +249,7 @@ __device__ __forceinline__ void direct_item(const BatchArgs &a, float4 *tile, in
     }
     __syncwarp();
     if (live) {
+#pragma unroll 4
       for (int k = 0; k < m; k++) {
         float4 A = tile[4 * k], B = tile[4 * k + 1], Cc = tile[4 * k + 2], Dd = tile[4 * k + 3];
         int jj = __float_as_int(Dd.x);
@@ -261,7 +262,7 @@ __device__ __forceinline__ void direct_item(const BatchArgs &a, float4 *tile, in
         float r2z = (Cc.x - th[2]) + (Cc.w - tl[2]);
         float ox, oy, oz;
         float r1s = fmaf(r1x, r1x, fmaf(r1y, r1y, r1z * r1z));
-        qv_seg32(r1x, r1y, r1z, r2x, r2y, r2z, Dd.y, Dd.z, Dd.w, r1s, ox, oy, oz);
+        qv_seg32_direct(r1x, r1y, r1z, r2x, r2y, r2z, Dd.y, Dd.z, Dd.w, r1s, ox, oy, oz);
         k0.add(ox, oy, oz);
       }
     }

@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(DTILE) k_direct32(int na, const int *__restric
           const float r2z = (Cc.x - th[k][2][1]) + (Cc.w - tl[k][2][1]);
           const float r1s = fmaf(r1x, r1x, fmaf(r1y, r1y, r1z * r1z));
           float ox, oy, oz;
-          qv_seg32(r1x, r1y, r1z, r2x, r2y, r2z, sx, sy, sz, r1s, ox, oy, oz);
+          qv_seg32_direct(r1x, r1y, r1z, r2x, r2y, r2z, sx, sy, sz, r1s, ox, oy, oz);
           k0[k].add(ox, oy, oz);
           continue;
         }

@@ -382,3 +382,33 @@ def test_tree_moments_at_the_kernels_node_sizes():
     assert set(got) == set(want)
     for name in want:
         np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_mixed_direct_pairs_equal_the_walks_leaf_pairs(seed):
+    """The direct sum's pair term (one branch for cos >= 0) has the bits of the
+    walk's leaf pair (no branch): a point and a triangle whose corners the tree
+    visits in slot order, seen under every angle, near its ends and from afar."""
+    from qvort_b200 import lib as L
+
+    rng = np.random.default_rng(seed)
+    A, B, C = np.array([[0.005, 0.006, 0.004], [0.03, 0.011, 0.02], [0.04, 0.03, 0.045]])
+    far = rng.uniform(-0.045, 0.045, (60, 3))
+    near = A + rng.uniform(-1.0, 1.0, (30, 3)) * 10.0 ** rng.uniform(-7, -3, (30, 1))
+    line = A + rng.uniform(-0.1, 1.1, (30, 1)) * (B - A) + rng.uniform(-1e-5, 1e-5, (30, 3))
+    P = np.concatenate([far, near, line])
+    cos = np.einsum("ij,ij->i", A - P, B - P)
+    assert (cos > 0).any() and (cos < 0).any()
+    inf, beh = np.array([2, 1, 4, 5, 3], np.int32), np.array([2, 1, 5, 3, 4], np.int32)
+    ws = [(np.array([p, [-0.04, -0.03, 0.02], A, B, C]), inf, beh) for p in P]
+    kw = dict(boundary="open", box_size=0.1, precision="mixed", quant_circ=W.GAMMA_HE4,
+              corea=W.CORE_A, tree_theta=1e-3)
+    n = len(ws)
+    u = {v: L.Batch(L.default_params(**kw, velocity="Tree"), ws, [v] * n, [1e-7] * n).velocity()
+         for v in ("BS", "Tree")}
+    assert np.array_equal(u["BS"][::5], u["Tree"][::5])
+    for k in range(0, n, 17):
+        c = L.Context(L.default_params(**dict(kw, velocity="BS", tree_theta=0.0)))
+        c.set_points(*ws[k])
+        assert np.array_equal(c.velocity()[0][0], u["BS"][5 * k])
+        c.close()
