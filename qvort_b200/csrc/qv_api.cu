@@ -423,6 +423,8 @@ extern "C" int qv_set_closest(qv_ctx *c, const int *closest) {
 extern "C" int qv_get_points(qv_ctx *c, double *x, double *u) {
   QV_CHECK_CTX(c);
   size_t v = sizeof(double) * 3 * (size_t)c->n;
+  qv_populate(x, v);
+  qv_populate(u, v);
   if (x && v) QV_CUDA(c, cudaMemcpyAsync(x, c->x, v, cudaMemcpyDeviceToHost, c->stream));
   if (u && v) QV_CUDA(c, cudaMemcpyAsync(u, c->u, v, cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -748,6 +750,7 @@ extern "C" int qv_velocity(qv_ctx *c, double *u, double *u_li, double *u_bs, lon
   int rc = velocity_launch(c);
   if (rc) return rc;
   size_t v = sizeof(double) * 3 * (size_t)c->n;
+  for (double *r : {u, u_li, u_bs}) qv_populate(r, v);  // while the kernels run
   if (u) QV_CUDA(c, cudaMemcpyAsync(u, c->u, v, cudaMemcpyDeviceToHost, c->stream));
   if (u_li) QV_CUDA(c, cudaMemcpyAsync(u_li, c->u_li, v, cudaMemcpyDeviceToHost, c->stream));
   if (u_bs) QV_CUDA(c, cudaMemcpyAsync(u_bs, c->u_bs, v, cudaMemcpyDeviceToHost, c->stream));

@@ -882,6 +882,8 @@ extern "C" int qv_batch_get_points(qv_batch *b, double *x, double *u) {
   if (!b) return QV_ERR_ARG;
   qv_ctx *c = b->c;
   size_t v = sizeof(double) * 3 * (size_t)b->ntot;
+  qv_populate(x, v);
+  qv_populate(u, v);
   if (x) QV_CUDA(c, cudaMemcpyAsync(x, c->x, v, cudaMemcpyDeviceToHost, c->stream));
   if (u) QV_CUDA(c, cudaMemcpyAsync(u, c->u, v, cudaMemcpyDeviceToHost, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -5,6 +5,7 @@
 // benchmark configurations (setup_single_loop / setup_leap_frog,
 // src/initial_loop.f90:11-38, 206-245).
 #include <cctype>
+#include <cerrno>
 #include <cstdint>
 #include <cmath>
 #include <cstdio>
@@ -12,6 +13,8 @@
 #include <cstring>
 #include <string>
 #include <vector>
+
+#include <sys/mman.h>
 
 #include "../../include/qv.h"
 
@@ -350,4 +353,25 @@ extern "C" int qv_read_restart_file(const char *path, int cap, int *n, int *reco
     if (s->closestd) std::memcpy(s->closestd + i, e + F_CLOSESTD, 8);
   }
   return QV_OK;
+}
+
+// A large result array that the caller has just allocated has no pages yet, and a
+// copy into it takes a fault a page: 13 ms for 43 MB, of which the copy is 3.
+// Populating the whole pages of the array in one call (the kernel uses huge pages
+// where the allocator asked for them) brings that to 7.7; where it is not
+// supported, or the range is not ordinary memory, it fails without effect and the
+// copy does as before.  Below 1 MB allocators hand out memory that is in use.
+void qv_populate(void *p, size_t bytes) {
+#ifdef __linux__
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  const uintptr_t page = 4096;
+  if (!p || bytes < (1u << 20)) return;
+  const uintptr_t lo = ((uintptr_t)p + page - 1) / page * page;
+  const uintptr_t hi = ((uintptr_t)p + bytes) / page * page;
+  const int e = errno;
+  madvise((void *)lo, hi - lo, MADV_POPULATE_WRITE);
+  errno = e;
+#endif
 }

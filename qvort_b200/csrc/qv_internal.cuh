@@ -314,6 +314,9 @@ int qv_forest_build(qv_ctx *c, const ForestArgs &f);
 #define QV_CTL_DEPTH 4
 #define QV_CTL_NNODES 0
 
+// the pages of a large result array, ahead of the copy into it (qv_host.cpp)
+void qv_populate(void *p, size_t bytes);
+
 // ---------------------------------------------------------------- helpers
 // 1/sqrt(a) and 1/a of a normal number: what rsqrtf and the fast division give
 // there, without their handling of subnormal operands (three instructions of a

@@ -412,3 +412,30 @@ def test_mixed_direct_pairs_equal_the_walks_leaf_pairs(seed):
         c.set_points(*ws[k])
         assert np.array_equal(c.velocity()[0][0], u["BS"][5 * k])
         c.close()
+
+
+@pytest.mark.parametrize("n", [43_690, 43_691, 60_000])
+def test_large_results_into_fresh_and_offset_arrays(n):
+    """Results around and above 1 MB (the pages of larger arrays are made before the
+    copy): a new array, a used one and an unaligned slice get the same values, and
+    nothing outside the slice is written."""
+    from qvort_b200 import lib as L
+
+    w = W.ring(n, 0.01, 0.0)
+    c = L.Context(L.default_params(**dict(w.params, velocity="LIA", precision="fp64")))
+    c.set_points(w.x, w.infront, w.behind)
+    u = c.velocity()[0]
+    x0, u0 = c.get_points()
+    assert np.array_equal(x0, w.x) and np.array_equal(u0, u)
+    pad = np.full(2 * 3 * n + 1111, 7.0)
+    xs, us = pad[5:5 + 3 * n].reshape(n, 3), pad[1000 + 3 * n:1000 + 6 * n].reshape(n, 3)
+    c.get_points(xs, us)
+    assert np.array_equal(xs, x0) and np.array_equal(us, u0)
+    assert (pad[:5] == 7).all() and (pad[5 + 3 * n:1000 + 3 * n] == 7).all()
+    assert (pad[1000 + 6 * n:] == 7).all()
+    b = L.Batch(L.default_params(**dict(w.params, precision="mixed", velocity="Tree",
+                                        tree_theta=0.4)),
+                [(w.x, w.infront, w.behind)], ["Tree"], [1e-9])
+    assert np.array_equal(b.get_points()[0], w.x)
+    v = b.velocity()
+    assert np.array_equal(b.get_points()[1], v)
