@@ -12,7 +12,7 @@
 //   the octrees of all Barnes-Hut systems as one forest (qv_forest_build)
 //   the FP32 source pack of the direct systems
 //   ONE persistent work kernel over a cost-ordered list of warp items:
-//     walk items   (32 targets of a Barnes-Hut system x one root child)
+//     walk items   (32 or 64 targets of a Barnes-Hut system x one root child)
 //     direct items (32 targets of a direct system x one source chunk)
 //   one kernel that adds each point's partial sums in a fixed order and
 //   applies the AB update with the system's own dt
@@ -40,6 +40,14 @@ static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 #define BSPLIT 8   // walk items per target group: the root's children
 #define BDT 128    // source tile of the single-system direct kernel (chunk rounding)
+
+// Walk items carry 64 targets, two a lane, when there are at least this many of 32
+// targets per SM (20 for each of its 24 resident warps), and 32 otherwise, where
+// fewer and longer items leave warps idle at the end.  32 and 64 targets: 512
+// systems (175k items) 3.59 and 3.35 ms a step, 512 of 2000 to 8000 points (556k)
+// 8.85 and 7.92, 128 systems (44k) 1.11 both, 64 (22k) 0.71 and 0.73, one of 8000
+// points 0.31 and 0.36.
+#define QV_BATCH_PAIR 480
 
 // status bits
 #define BST_SINGULAR 1
@@ -209,6 +217,159 @@ __device__ __forceinline__ void walk_item(const BatchArgs &a, StkEnt *st, int g,
   }
 }
 
+// Two targets per lane: 64 targets of one system (q and q + 32) against the same
+// root child, their FP32 state as pairs, as in the single-system mixed walk's
+// 64-target tasks: one node pop serves 64 targets, the recentring and the
+// far-field term run on the packed FP32 pipe, and each target's operations and
+// their order are walk_item's.
+template <int H>
+__device__ __forceinline__ void leaf_half(const BatchArgs &a, const PairTarget &t, int node,
+                                          const WNode32 &h, const float2 *th, const float2 *tl,
+                                          float2 v0, float2 v1, float2 v2, float2 d2, Kahan3x2 &k,
+                                          unsigned &ev, bool &bad) {
+  const int j = h.jb;
+  if (j == t.i + 1 || j == t.bi || j == t.fi) return;
+  const float d2h = pick(d2, H);
+  if (d2h < 1e-20f) {
+    const double s[3] = {0., 0., 0.};
+    const double xi[3] = {a.x[3 * t.i], a.x[3 * t.i + 1], a.x[3 * t.i + 2]};
+    if (exact_dist(xi, a.w64[node], s) < QV_DEPS) {
+      bad = true;
+      return;
+    }
+  }
+  const WPay32 &P = a.p32[node];
+  const float r2x = (P.a[0] - pick(th[0], H)) + (P.b[0] - pick(tl[0], H));
+  const float r2y = (P.a[1] - pick(th[1], H)) + (P.b[1] - pick(tl[1], H));
+  const float r2z = (P.a[2] - pick(th[2], H)) + (P.b[2] - pick(tl[2], H));
+  float ox, oy, oz;
+  qv_seg32(-pick(v0, H), -pick(v1, H), -pick(v2, H), r2x, r2y, r2z, P.C[0], P.C[1], P.C[2], d2h,
+           ox, oy, oz);
+  k.add1<H>(ox, oy, oz);
+  ev++;
+}
+
+// The reference's opening test of target i against a node.
+__device__ __forceinline__ bool exact_test(const BatchArgs &a, int node, int i) {
+  const double s[3] = {0., 0., 0.};
+  const double xi[3] = {a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2]};
+  const WNode64 h64 = a.w64[node];
+  return exact_open(exact_dist(xi, h64, s), h64, a.theta, a.extra);
+}
+
+__device__ __forceinline__ void walk_item2(const BatchArgs &a, StkEnt *st, int g, int sl,
+                                           const int *perm, unsigned &ev, unsigned &evf,
+                                           bool &bad) {
+  const int lane = threadIdx.x & 31;
+  const int4 G = a.groups[g];
+  const bool la = lane < G.y, lb = lane + 32 < G.y;
+  PairTarget ta = {0, -1, -1}, tb = {0, -1, -1};
+  float2 th[3], tl[3];
+  {
+    double xa[3] = {0., 0., 0.}, xb[3] = {0., 0., 0.};
+    if (la) {
+      ta.i = perm[G.x + lane];
+      ta.bi = a.beh[ta.i]; ta.fi = a.inf[ta.i];
+      xa[0] = a.x[3 * ta.i]; xa[1] = a.x[3 * ta.i + 1]; xa[2] = a.x[3 * ta.i + 2];
+    }
+    if (lb) {
+      tb.i = perm[G.x + lane + 32];
+      tb.bi = a.beh[tb.i]; tb.fi = a.inf[tb.i];
+      xb[0] = a.x[3 * tb.i]; xb[1] = a.x[3 * tb.i + 1]; xb[2] = a.x[3 * tb.i + 2];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      th[c].x = __double2float_rn(xa[c]);
+      tl[c].x = __double2float_rn(xa[c] - (double)th[c].x);
+      th[c].y = __double2float_rn(xb[c]);
+      tl[c].y = __double2float_rn(xb[c] - (double)th[c].y);
+    }
+  }
+  Kahan3x2 k0;
+  k0.zero();
+  int top = 0;
+  {
+    const int root = G.z;
+    const WNode64 r = a.w64[root];
+    bool oa = la, ob = lb;
+    if (r.count != 1) {
+      if (la) oa = exact_test(a, root, ta.i);
+      if (lb) ob = exact_test(a, root, tb.i);
+      if (sl == 0) {  // root far field: zero moments
+        const unsigned far = (la && !oa ? 1u : 0u) + (lb && !ob ? 1u : 0u);
+        ev += far;
+        evf += far;
+      }
+    }
+    const unsigned ma = __ballot_sync(0xffffffffu, oa), mb = __ballot_sync(0xffffffffu, ob);
+    const int first = r.count == 1 ? root : r.child_first + sl;
+    if ((ma | mb) && (r.count == 1 ? sl == 0 : sl < r.nchild)) {
+      if (lane == 0) {
+        st[0].h = a.w32[first];
+        st[0].node = first;
+        st[0].mask = ma;
+        st[0].mask2 = mb;
+      }
+      top = 1;
+    }
+  }
+  __syncwarp();
+  while (top > 0) {
+    top--;
+    const WNode32 h = st[top].h;
+    const int node = st[top].node;
+    const bool ina = (st[top].mask >> lane) & 1u, inb = (st[top].mask2 >> lane) & 1u;
+    __syncwarp();
+    const float2 v0 = add2(sub2(th[0], bc2(h.ch[0])), sub2(tl[0], bc2(h.cl[0])));
+    const float2 v1 = add2(sub2(th[1], bc2(h.ch[1])), sub2(tl[1], bc2(h.cl[1])));
+    const float2 v2 = add2(sub2(th[2], bc2(h.ch[2])), sub2(tl[2], bc2(h.cl[2])));
+    const float2 d2 = fma2(v0, v0, fma2(v1, v1, mul2(v2, v2)));
+    if (h.count == 1) {
+      if (ina) leaf_half<0>(a, ta, node, h, th, tl, v0, v1, v2, d2, k0, ev, bad);
+      if (inb) leaf_half<1>(a, tb, node, h, th, tl, v0, v1, v2, d2, k0, ev, bad);
+    } else {
+      const bool sure = h.rhi > 0.f;
+      const bool amba = ina && !(sure && (d2.x > h.rhi || d2.x < h.rlo));
+      const bool ambb = inb && !(sure && (d2.y > h.rhi || d2.y < h.rlo));
+      bool opa = ina && d2.x < h.rlo, opb = inb && d2.y < h.rlo;
+      if (amba) opa = exact_test(a, node, ta.i);
+      if (ambb) opb = exact_test(a, node, tb.i);
+      const bool fa = ina && !opa, fb = inb && !opb;
+      const unsigned far = (fa ? 1u : 0u) + (fb ? 1u : 0u);
+      ev += far;
+      evf += far;
+      if (far && node >= a.nroots)  // a root's moments are zero
+        far_pair(a.p32[node], v0, v1, v2, d2, fa, fb, k0);
+      const unsigned ma = __ballot_sync(0xffffffffu, opa), mb = __ballot_sync(0xffffffffu, opb);
+      if (ma | mb) {
+        int nc = h.nchild;
+        if (top + nc > a.stk_cap) {  // deeper than the captured stack: flagged, step skipped
+          if (lane == 0) atomicOr(a.status, BST_STACK);
+          nc = 0;
+        }
+        if (lane < nc) {
+          const int ch = h.child_first + nc - 1 - lane;
+          StkEnt &E = st[top + lane];
+          E.h = a.w32[ch];
+          E.node = ch;
+          E.mask = ma;
+          E.mask2 = mb;
+        }
+        top += nc;
+      }
+      __syncwarp();
+    }
+  }
+  if (la) {
+    double *o = a.partw + ((size_t)sl * a.ntot + ta.i) * 3;
+    o[0] = k0.get(0, 0); o[1] = k0.get(0, 1); o[2] = k0.get(0, 2);
+  }
+  if (lb) {
+    double *o = a.partw + ((size_t)sl * a.ntot + tb.i) * 3;
+    o[0] = k0.get(1, 0); o[1] = k0.get(1, 1); o[2] = k0.get(1, 2);
+  }
+}
+
 // -------------------------------------------------------------- direct item
 // One warp, 32 consecutive targets of one system, the sources of one chunk
 // (the chunking of the single-system direct kernel), staged 32 at a time in
@@ -276,6 +437,7 @@ __device__ __forceinline__ void direct_item(const BatchArgs &a, float4 *tile, in
 // ---------------------------------------------------------- work items
 // Each warp takes the next item from a global counter until the list is
 // exhausted; the list is ordered by estimated cost, largest first.
+template <bool PAIR>
 __device__ __forceinline__ void batch_items(const BatchArgs &a) {
   extern __shared__ __align__(16) unsigned char bsm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -290,7 +452,9 @@ __device__ __forceinline__ void batch_items(const BatchArgs &a) {
     it = __shfl_sync(0xffffffffu, it, 0);
     if (it >= a.nitems) break;
     const int4 W = a.items[it];
-    if (W.x < BSPLIT)
+    if (PAIR && W.x < BSPLIT)
+      walk_item2(a, reinterpret_cast<StkEnt *>(mine), W.y, W.x, perm, ev, evf, bad);
+    else if (W.x < BSPLIT)
       walk_item(a, reinterpret_cast<StkEnt *>(mine), W.y, W.x, perm, ev, evf, bad);
     else
       direct_item(a, reinterpret_cast<float4 *>(mine), W.y, W.x - BSPLIT, W.z);
@@ -429,7 +593,10 @@ struct PackArgsB {
 // LIA stay separate launches before the forest build: the forest's moments
 // need the ghosts, and LIA keeps the single-system kernel's arithmetic (its
 // file is compiled without FMA contraction).
-__global__ void k_batch_step(BatchArgs a, UpdateArgs ub, PackArgsB pb) {
+// 80 registers: six blocks of 128 threads per SM (the pairs left to themselves take
+// 96 and run five: 3.57 ms, not 3.35, for 512 systems).
+template <bool PAIR>
+__global__ void __maxnreg__(80) k_batch_step(BatchArgs a, UpdateArgs ub, PackArgsB pb) {
   cg::grid_group grid = cg::this_grid();
   const int nthreads = gridDim.x * blockDim.x;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
@@ -441,7 +608,7 @@ __global__ void k_batch_step(BatchArgs a, UpdateArgs ub, PackArgsB pb) {
   }
   for (int q = gt; q < pb.nd; q += nthreads) batch_pack_point(q, pb.dact, a.x, pb.gi, pb.s32);
   grid.sync();
-  if (*a.status == 0) batch_items(a);
+  if (*a.status == 0) batch_items<PAIR>(a);
   grid.sync();
   if (gt == 0) *a.counter = 0;  // every fetch is done: ready for the next step
   if (*a.status) return;
@@ -455,6 +622,10 @@ struct qv_batch {
   int nsys = 0, ntot = 0;
   std::vector<int> off, meth, nchunk, clen;
   std::vector<double> dt;
+  bool pair = false;  // walk items of 64 targets
+  const void *kernel() const {
+    return pair ? (const void *)k_batch_step<true> : (const void *)k_batch_step<false>;
+  }
   int nroots = 0, n_fact = 0, nd = 0, max_chunks = 1, ngroups = 0;
   // device tables
   int *d_sysof = nullptr, *d_dact = nullptr, *d_fact = nullptr, *d_froot = nullptr;
@@ -552,7 +723,7 @@ static int launch_step(qv_batch *b, int do_ab) {
   pb.nd = b->nd; pb.dact = b->d_dact; pb.gi = c->gi; pb.s32 = b->d_src32;
   size_t smem = work_smem_per_warp(b) * b->wpb;
   void *args[] = {&a, &ub, &pb};
-  QV_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_batch_step, dim3(b->bps * c->sm_count),
+  QV_CUDA(c, cudaLaunchCooperativeKernel(b->kernel(), dim3(b->bps * c->sm_count),
                                          dim3(b->wpb * 32), args, smem, c->stream));
   QV_COUNT(c, 1);
   return QV_OK;
@@ -615,6 +786,11 @@ extern "C" int qv_batch_create(const qv_params *p, int nsys, const int *offsets,
   std::vector<int4> sys(nsys), roots, groups;
   std::vector<int2> dsrc(nsys, make_int2(0, 0));
   std::vector<double> cost;
+  long nwalk = 0;  // walk items of 32 targets
+  for (int s = 0; s < nsys; s++)
+    if (method[s] == QV_VEL_TREE) nwalk += (long)BSPLIT * nblk(offsets[s + 1] - offsets[s], 32);
+  b->pair = nwalk >= QV_BATCH_PAIR * (long)c->sm_count;
+  const int gsz = b->pair ? 64 : 32;
   for (int s = 0; s < nsys; s++) {
     const int o = offsets[s], n = offsets[s + 1] - offsets[s];
     for (int i = o; i < o + n; i++) sysof[i] = s;
@@ -636,14 +812,14 @@ extern "C" int qv_batch_create(const qv_params *p, int nsys, const int *offsets,
     } else {
       const int r = (int)roots.size();
       roots.push_back(make_int4(o, n, (int)fact.size(), n));
-      for (int q0 = 0; q0 < n; q0 += 32) {
+      for (int q0 = 0; q0 < n; q0 += gsz) {
         const int g = (int)groups.size();
-        groups.push_back(make_int4((int)fact.size() + q0, std::min(32, n - q0), r, s));
+        groups.push_back(make_int4((int)fact.size() + q0, std::min(gsz, n - q0), r, s));
         for (int sl = 0; sl < BSPLIT; sl++) {
           b->items.push_back(make_int4(sl, g, 0, 0));
           // a rough per-target walk cost: a few dozen cells per octave of N,
           // spread over the root's children
-          cost.push_back((double)std::min(32, n - q0) * 40. * std::log2((double)n + 1.) / 4.);
+          cost.push_back((double)std::min(gsz, n - q0) * 40. * std::log2((double)n + 1.) / 4.);
         }
       }
       for (int i = o; i < o + n; i++) {
@@ -709,15 +885,15 @@ extern "C" const char *qv_batch_last_error(qv_batch *b) { return b ? b->c->err :
 // The launch shape of a batch that nothing has tuned: four warps per block, as
 // many blocks per SM as are resident at once, up to six, while every warp finds
 // an item; items in their natural order (neighbouring groups share their nodes
-// in L1).  Two blocks per SM, largest items first, the shape before, left
-// the walks' latency uncovered: 512 systems (924k points) 7.40 ms a step, 3.92
-// with six; 64 systems (68k points) 0.67 and 0.46; 16 systems with 203 items
-// in all 0.195, and 0.19 with one.
+// in L1).  Two blocks per SM, largest items first, left the walks' latency
+// uncovered (with items of 32 targets, before later changes): 512 systems (924k
+// points) 7.40 ms a step, 3.92 with six; 64 systems (68k points) 0.67 and 0.46; 16
+// systems with 203 items in all 0.195, and 0.19 with one.
 static int default_shape(qv_batch *b) {
   if (b->shape_fixed) return QV_OK;
   qv_ctx *c = b->c;
   int per = 0;
-  QV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step, b->wpb * 32,
+  QV_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, b->kernel(), b->wpb * 32,
                                                            work_smem_per_warp(b) * b->wpb));
   const int want = nblk((long)b->items.size(), b->wpb * c->sm_count);
   const int bps = std::max(1, std::min({per, 6, want}));
@@ -760,7 +936,7 @@ static int size_stack(qv_batch *b) {
       drop_graph(b);
     }
     size_t smem = work_smem_per_warp(b) * 8;
-    QV_CUDA(c, cudaFuncSetAttribute(k_batch_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    QV_CUDA(c, cudaFuncSetAttribute(b->kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)std::min<size_t>(smem, 227 * 1024)));
     return default_shape(b);
   }
@@ -938,7 +1114,7 @@ extern "C" int qv_batch_tune(qv_batch *b, int reps, int *best_cfg, float *best_m
         size_t smem = work_smem_per_warp(b) * w;
         if (smem > 227 * 1024) continue;
         int per = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step, w * 32, smem) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, b->kernel(), w * 32, smem) !=
             cudaSuccess) {
           cudaGetLastError();
           continue;
@@ -987,7 +1163,7 @@ extern "C" int qv_batch_set_config(qv_batch *b, int warps_per_block, int blocks_
   int per = 0;
   size_t smem = work_smem_per_warp(b) * warps_per_block;
   if (smem > 227 * 1024 ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step, warps_per_block * 32, smem) !=
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, b->kernel(), warps_per_block * 32, smem) !=
           cudaSuccess ||
       per < blocks_per_sm) {
     cudaGetLastError();

@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(BT) k_build_local(BuildArgs a) {
 // in ascending slot order: cent (3), circ (3) and Cij (9).  The chains cannot
 // be reassociated, so their latency is the floor; the kernels below keep the
 // chain lanes fed from shared memory while other warps gather and precompute.
-#define MW 8      // warps per block (small nodes: one warp per node)
+#define MW 8      // warps per block (nodes of TN+1 to BIGN points: one warp per node)
 #define BIGN LCH  // nodes with more points: a block each, early (all made grid-wide)
 #define TN 8      // nodes with at most this many points: a thread each
 #define MC 256    // points per shared-memory chunk in the block kernel

@@ -130,9 +130,9 @@ __device__ __forceinline__ void slot_shift(int bc, int sl, double L, double *s) 
 // likewise.  Bound: instruction issue (a third of it FP64) and dependent FP64
 // latency.  Walk of the tangle (24.7k points, 27 images, theta 0.4): 1.01 ms
 // with a square root and a division per test and eight divisions per far cell,
-// 0.53 ms now; large tangle (803k points, theta 0.5): 24 -> 12.6 ms.  Taking 2
-// or 4 nodes at a time for 16 or 8 targets ran as fast (0.55 and 0.52 ms, 13.2
-// and 13.8), but a target's sums would then depend on its group.
+// 0.53 ms with these and 0.47 in the task order of task_slot; large tangle (803k
+// points, theta 0.5): 24 -> 12.6 ms.  Taking 2 or 4 nodes at a time for 16 or 8
+// targets ran no faster (0.55 and 0.52 ms against 0.53; 13.2 and 13.8), and a target's sums would then depend on its group.
 template <int BC>
 __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
   constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
@@ -256,11 +256,6 @@ __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
 }
 
 // ---------------------------------------------------------------- mixed walk
-// One target of a lane's pair: its point index and links.
-struct PairTarget {
-  int i, bi, fi;  // point index (0-based), behind, infront; bi = fi = -1 if not live
-};
-
 // Leaf pair (src/tree.f90:371-391) of half H of a lane's two targets.
 template <int H>
 __device__ __forceinline__ void leaf_half(const WalkArgs &a, int bc, int sl, int node,
@@ -674,24 +669,8 @@ __device__ __forceinline__ void walk_task2(const WalkArgs &a, StkEnt *st, int la
       evfa += fa ? 1u : 0u;
       evb += fb ? 1u : 0u;
       evfb += fb ? 1u : 0u;
-      if ((fa || fb) && node != 0) {  // the root's moments are zero
-        const WPay32 &P = a.p32[node];
-        // below 1e-25 the powers overflow either way
-        const float2 rd = make_float2(rsqrt_normal(d2.x), rsqrt_normal(d2.y));
-        const float2 rd2 = mul2(rd, rd), rd3 = mul2(rd2, rd), rd5 = mul2(rd3, rd2);
-        const float2 z0 = fma2(v0, bc2(P.C[0]), fma2(v1, bc2(P.C[3]), mul2(v2, bc2(P.C[6]))));
-        const float2 z1 = fma2(v0, bc2(P.C[1]), fma2(v1, bc2(P.C[4]), mul2(v2, bc2(P.C[7]))));
-        const float2 z2 = fma2(v0, bc2(P.C[2]), fma2(v1, bc2(P.C[5]), mul2(v2, bc2(P.C[8]))));
-        const float2 cx = sub2(fma2(bc2(P.a[1]), v2, mul2(bc2(-P.a[2]), v1)), bc2(P.b[0]));
-        const float2 cy = sub2(fma2(bc2(P.a[2]), v0, mul2(bc2(-P.a[0]), v2)), bc2(P.b[1]));
-        const float2 cz = sub2(fma2(bc2(P.a[0]), v1, mul2(bc2(-P.a[1]), v0)), bc2(P.b[2]));
-        const float2 wx = fma2(v1, z2, mul2(neg2(v2), z1));
-        const float2 wy = fma2(v2, z0, mul2(neg2(v0), z2));
-        const float2 wz = fma2(v0, z1, mul2(neg2(v1), z0));
-        const float2 t5 = mul2(bc2(3.f), rd5);
-        k0.add(fma2(cx, rd3, mul2(wx, t5)), fma2(cy, rd3, mul2(wy, t5)),
-               fma2(cz, rd3, mul2(wz, t5)), fa, fb);
-      }
+      if ((fa || fb) && node != 0)  // the root's moments are zero
+        far_pair(a.p32[node], v0, v1, v2, d2, fa, fb, k0);
       const unsigned ma = __ballot_sync(0xffffffffu, opa), mb = __ballot_sync(0xffffffffu, opb);
       if (ma | mb) {
         int nc = h.nchild;
@@ -815,7 +794,7 @@ __device__ __forceinline__ void walk32_body(const WalkArgs &a) {
 // The walks, and the same walks under a second name for the gated relaunch
 // after an overflowing root fix-up (it returns at once unless flagged), so
 // that a profile tells the two launches apart.
-// 5 blocks/SM: 0.53 ms on the tangle (unbounded 0.57, 8 0.59)
+// 5 blocks/SM: 0.53 ms on the tangle before task_slot's order (unbounded 0.57, 8 0.59)
 template <int BC>
 __global__ void __launch_bounds__(WW * 32, 5) k_walk64(WalkArgs a) { walk64_body<BC>(a); }
 template <int BC>

@@ -169,6 +169,32 @@ struct Kahan3x2 {
   }
 };
 
+// One target of a lane's pair: its point index and links.
+struct PairTarget {
+  int i, bi, fi;  // point index (0-based), behind, infront; bi = fi = -1 if not live
+};
+
+// Far-field term of a cell (payload P, d2 = |v|^2) for the targets of a pair that
+// accept it (fa, fb).
+__device__ __forceinline__ void far_pair(const WPay32 &P, float2 v0, float2 v1, float2 v2, float2 d2,
+                                         bool fa, bool fb, Kahan3x2 &k0) {
+  // below 1e-25 the powers overflow either way
+  const float2 rd = make_float2(rsqrt_normal(d2.x), rsqrt_normal(d2.y));
+  const float2 rd2 = mul2(rd, rd), rd3 = mul2(rd2, rd), rd5 = mul2(rd3, rd2);
+  const float2 z0 = fma2(v0, bc2(P.C[0]), fma2(v1, bc2(P.C[3]), mul2(v2, bc2(P.C[6]))));
+  const float2 z1 = fma2(v0, bc2(P.C[1]), fma2(v1, bc2(P.C[4]), mul2(v2, bc2(P.C[7]))));
+  const float2 z2 = fma2(v0, bc2(P.C[2]), fma2(v1, bc2(P.C[5]), mul2(v2, bc2(P.C[8]))));
+  const float2 cx = sub2(fma2(bc2(P.a[1]), v2, mul2(bc2(-P.a[2]), v1)), bc2(P.b[0]));
+  const float2 cy = sub2(fma2(bc2(P.a[2]), v0, mul2(bc2(-P.a[0]), v2)), bc2(P.b[1]));
+  const float2 cz = sub2(fma2(bc2(P.a[0]), v1, mul2(bc2(-P.a[1]), v0)), bc2(P.b[2]));
+  const float2 wx = fma2(v1, z2, mul2(neg2(v2), z1));
+  const float2 wy = fma2(v2, z0, mul2(neg2(v0), z2));
+  const float2 wz = fma2(v0, z1, mul2(neg2(v1), z0));
+  const float2 t5 = mul2(bc2(3.f), rd5);
+  k0.add(fma2(cx, rd3, mul2(wx, t5)), fma2(cy, rd3, mul2(wy, t5)),
+         fma2(cz, rd3, mul2(wz, t5)), fa, fb);
+}
+
 // Stack entry: the child's FP32 header, fetched when the child is pushed so
 // that popping it costs a shared-memory read instead of a dependent global load,
 // and the lane masks of the targets that opened the parent (mask: the warp's

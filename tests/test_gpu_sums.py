@@ -439,3 +439,32 @@ def test_large_results_into_fresh_and_offset_arrays(n):
     assert np.array_equal(b.get_points()[0], w.x)
     v = b.velocity()
     assert np.array_equal(b.get_points()[1], v)
+
+
+def test_batched_walk_with_two_targets_a_lane_equals_one():
+    """A batch large enough for walk items of 64 targets (71,040 items of 32 on 148
+    SMs): systems around multiples of 32 and 64 points, each repeated, have bit for
+    bit the velocities of the same systems in a small batch, and the same steps."""
+    from qvort_b200 import lib as L
+
+    sizes = [5, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 1000]
+    ws = [W.ring(m, 0.01 + 1e-5 * k, 1e-5, seed=k) for k, m in enumerate(sizes)]
+    reps = 160
+    p = L.default_params(boundary="open", velocity="Tree", tree_theta=0.4, box_size=0.1,
+                         precision="mixed", quant_circ=W.GAMMA_HE4, corea=W.CORE_A)
+
+    def batch(r):
+        m = len(ws) * r
+        return L.Batch(p, [(w.x, w.infront, w.behind) for w in ws] * r, ["Tree"] * m, [1e-9] * m)
+
+    small, large = batch(1), batch(reps)
+    assert 8 * reps * sum(-(-m // 32) for m in sizes) >= 71_040
+    # one item per 64 targets of a system and root child
+    assert large.stats()["items"] == 8 * reps * sum(-(-m // 64) for m in sizes)
+    assert small.stats()["items"] == 8 * sum(-(-m // 32) for m in sizes)
+    us, ul = small.velocity(), large.velocity()
+    assert np.array_equal(ul.reshape(reps, -1, 3), np.broadcast_to(us, (reps, *us.shape)))
+    small.step(3)
+    large.step(3)
+    xs, xl = small.get_points()[0], large.get_points()[0]
+    assert np.array_equal(xl.reshape(reps, -1, 3), np.broadcast_to(xs, (reps, *xs.shape)))
