@@ -628,9 +628,9 @@ __global__ void k_energy_grad(int n, const double *__restrict__ x, const double 
 //
 // A warp takes one point and one chunk of the sources, a lane per source: a
 // handful of points (quasiparticles) then still fills the chip, where a thread
-// per point left 100 threads with 24,700 sources x 27 images each.  The FW
+// per point left 100 threads with 23,500 sources x 27 images each.  The FW
 // warps of a block take neighbouring points and the same chunk, which they
-// meet in L1.  Bound: FP64 issue.  100 points, 24,700 sources, 27 images: 302
+// meet in L1.  Bound: FP64 issue.  100 points, 23,500 sources, 27 images: 302
 // ms with a thread per point, 0.23 ms per call now (copies included).
 #define FW 4
 #define FV 12  // values per point: u (3), du/dx row-major (9)

@@ -87,7 +87,7 @@ __global__ void k_scatter_active(int n, const int *__restrict__ inf, const int *
 // segment of the flags, 128 at a time (a lane loads four and keeps them as four
 // bits); a scan of the 32 warp counts gives each segment's base, and a second
 // pass over the kept bits writes the indices in order.  One block has only its
-// loads' latency to hide: four flags a load, up to 16 loads in flight (24,700 flags,
+// loads' latency to hide: four flags a load, up to 16 loads in flight (23,500 flags,
 // cold: 11 -> 9 us; five of these a step).
 __global__ void __launch_bounds__(1024) k_compact1(int n, const int *__restrict__ flag, int *out,
                                                    int *total) {
@@ -328,10 +328,10 @@ __device__ __forceinline__ TilePipe make_pipe(const void *src, int j0, int j1, c
 // ------------------------------------------------------------ FP64 kernel
 // One thread per target, each staged source summed against it in all images
 // (Seg64).  Bound: FP64 issue, about 26 operations a pair (two rsqrt_pos and
-// one div_pos are 14 of them).  24,700 points, 27 images: 70.3 ms with the
+// one div_pos are 14 of them).  23,500 points, 27 images: 70.3 ms with the
 // reference's formula pair by pair (library rsqrt and division, 1.3 waves of
-// blocks), 26.0 ms now = 6.3e11 pairs/s, 88 % of the FP64 rate (148 SM x 64
-// lanes x 1.965 GHz) at that operation count.
+// blocks), 26.0 ms now = 5.7e11 pairs/s; the FP64 pipe is busy 84 % of the
+// time (24,700 points, 28.8 ms).
 template <int BC>
 __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const int *__restrict__ act,
                                                     const double *__restrict__ x,
@@ -499,8 +499,8 @@ __device__ __forceinline__ void seg_terms(float r1s, float r2s, float dd, float 
 
 // seg_terms where cos is known to be positive and the squared distances are
 // normal numbers: f / (1 + cos).  With the square roots' and the division's
-// handling of subnormal operands left out, 24,700 points and 27 images take 13.0
-// ms, not 15.1; the MUFU pipe (three of them a pair) would take 10.6.
+// handling of subnormal operands left out, 23,500 points and 27 images take 13.0
+// ms, not 15.1; the MUFU pipe (three of them a pair) would take 9.6.
 __device__ __forceinline__ void seg_terms_pos(float r1s, float r2s, float dd, float cx, float cy,
                                               float cz, float &ox, float &oy, float &oz) {
   const float ra = rsqrt_normal(r1s), rb = rsqrt_normal(r2s);

@@ -128,9 +128,9 @@ __device__ __forceinline__ void slot_shift(int bc, int sl, double L, double *s) 
 // (StkEnt64), and the same distance vector gives the far-field term, which
 // needs one reciprocal square root; leaves off the target's own surroundings
 // likewise.  Bound: instruction issue (a third of it FP64) and dependent FP64
-// latency.  Walk of the tangle (24.7k points, 27 images, theta 0.4): 1.01 ms
+// latency.  Walk of the tangle (23.5k points, 27 images, theta 0.4): 1.01 ms
 // with a square root and a division per test and eight divisions per far cell,
-// 0.53 ms with these and 0.47 in the task order of task_slot; large tangle (803k
+// 0.53 ms with these and 0.47 in the task order of task_slot; large tangle (796k
 // points, theta 0.5): 24 -> 12.6 ms.  Taking 2 or 4 nodes at a time for 16 or 8
 // targets ran no faster (0.55 and 0.52 ms against 0.53; 13.2 and 13.8), and a target's sums would then depend on its group.
 template <int BC>
@@ -1092,7 +1092,7 @@ int qv_launch_walk(qv_ctx *c) {
 // the box).  A warp task is (32 points, one image, and for the unshifted image
 // one root child), as in the velocity walk; its partial sums are added per
 // point in the images' order, so results do not depend on the grouping.  Bound:
-// FP64 issue and the latency of a pop.  32^3 mesh through the tangle (24.7k
+// FP64 issue and the latency of a pop.  32^3 mesh through the tangle (23.5k
 // points, 27 images, theta 0.4): 19.5 ms with one warp per 32 mesh points in
 // their own order over all images and 54 divisions per far cell (20-23 ms a
 // call), 0.82 ms a call now, copies included.
