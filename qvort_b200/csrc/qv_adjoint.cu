@@ -921,7 +921,7 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
         default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", p.boundary);
       }
       if (smem > 48 * 1024)
-        QV_CUDA(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if ((rc = qv_smem_optin(c, f))) return rc;
       void *args[] = {&a};
       QV_CUDA(c, cudaLaunchKernel(f, dim3(nb), dim3(AW * 32), args, smem, c->stream));
       QV_LAUNCH_CHECK(c);

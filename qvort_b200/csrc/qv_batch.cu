@@ -935,9 +935,7 @@ static int size_stack(qv_batch *b) {
       b->stk_cap = need;
       drop_graph(b);
     }
-    size_t smem = work_smem_per_warp(b) * 8;
-    QV_CUDA(c, cudaFuncSetAttribute(b->kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::min<size_t>(smem, 227 * 1024)));
+    if ((rc = qv_smem_optin(c, b->kernel()))) return rc;
     return default_shape(b);
   }
   return qv_fail(c, QV_ERR_NOMEM, "forest did not fit after repeated growth");

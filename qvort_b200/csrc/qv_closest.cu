@@ -383,10 +383,9 @@ int qv_launch_closest_ex(qv_ctx *c, const int *d_n, const int *d_skip, int n_gri
     int nwarps = (n_grid + tpw - 1) / tpw;
     int cap = 7 * (c->tree.depth + 1) + 8;
     size_t smem = sizeof(CStkEnt) * cap * CW;
-    if (smem > 48 * 1024 && smem > c->smem_search) {  // per context: attributes are per device
-      QV_CUDA(c, cudaFuncSetAttribute(k_closest_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-      c->smem_search = smem;
+    if (smem > 48 * 1024 && !c->optin_search) {
+      if ((rc = qv_smem_optin(c, (const void *)k_closest_tree))) return rc;
+      c->optin_search = true;
     }
     const TreeBuf &t = c->tree;
     k_closest_tree<<<(nwarps + CW - 1) / CW, CW * 32, smem, c->stream>>>(

@@ -215,7 +215,7 @@ struct qv_ctx {
   TreeBuf tree;
   int sm_count = 148;
   int build_grid = 0;  // co-resident blocks of the cooperative tree build
-  size_t smem_walk = 0, smem_search = 0;  // dynamic shared memory opted in on this device
+  bool optin_walk = false, optin_search = false;  // qv_smem_optin done for those kernels
   // instrumentation
   bool profile = false;
   cudaEvent_t ev_beg[PH_N] = {}, ev_end[PH_N] = {};
@@ -244,6 +244,7 @@ int qv_fail(qv_ctx *c, int code, const char *fmt, ...);
 #define QV_LAUNCH_CHECK(ctx) QV_CUDA(ctx, cudaGetLastError())
 
 int qv_grow(qv_ctx *c, void **ptr, size_t bytes);
+int qv_smem_optin(qv_ctx *c, const void *kernel);
 void qv_phase_begin(qv_ctx *c, int ph);
 void qv_phase_end(qv_ctx *c, int ph);
 void qv_phase_end_async(qv_ctx *c, int ph);

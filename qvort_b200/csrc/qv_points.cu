@@ -31,6 +31,21 @@ int qv_grow(qv_ctx *c, void **ptr, size_t bytes) {
   return QV_OK;
 }
 
+// Lets launches of `kernel` take all the dynamic shared memory that a block can
+// have beside the kernel's own static part.  The limit belongs to the process, not
+// to a context: one fixed size per kernel cannot take away what another context's
+// (or another thread's) launches need, as a limit set to each caller's own need can.
+int qv_smem_optin(qv_ctx *c, const void *kernel) {
+  cudaFuncAttributes at;
+  int dev = 0, most = 0;
+  QV_CUDA(c, cudaFuncGetAttributes(&at, kernel));
+  QV_CUDA(c, cudaGetDevice(&dev));
+  QV_CUDA(c, cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  QV_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  most - (int)at.sharedSizeBytes));
+  return QV_OK;
+}
+
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 // ---------------------------------------------------------------- ghosts

@@ -983,9 +983,8 @@ int qv_launch_walk(qv_ctx *c) {
     QV_CUDA(c, cudaMemsetAsync(c->walk_next, 0, 4 * sizeof(int), c->stream));
     a.next = c->walk_next;
   }
-  static_assert(sizeof(StkEnt) == sizeof(StkEnt64), "one opt-in serves both walks");
   if (smem > 48 * 1024) {
-    if (smem > c->smem_walk) {  // per context: attributes are per device
+    if (!c->optin_walk) {
       const void *fs[] = {(const void *)k_walk32<QV_BC_OPEN>, (const void *)k_walk32<QV_BC_PERIODIC>,
                           (const void *)k_walk32<QV_BC_OPENX>, (const void *)k_walk32<QV_BC_OPENXY>,
                           (const void *)k_walk32_redo<QV_BC_OPEN>,
@@ -999,8 +998,8 @@ int qv_launch_walk(qv_ctx *c) {
                           (const void *)k_walk64_redo<QV_BC_OPENX>,
                           (const void *)k_walk64_redo<QV_BC_OPENXY>};
       for (const void *f : fs)
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      c->smem_walk = smem;
+        if (int rc = qv_smem_optin(c, f)) return rc;
+      c->optin_walk = true;
     }
   }
   auto launch = [&](const WalkArgs &w, int grid, cudaStream_t st) -> int {
@@ -1330,7 +1329,7 @@ extern "C" int qv_field_velocity_tree(qv_ctx *c, int m, const double *pts, doubl
     default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d not supported", c->p.boundary);
   }
   if (smem > 48 * 1024)
-    QV_CUDA(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if ((rc = qv_smem_optin(c, f))) return rc;
   for (int lo = 0; lo < m; lo += slab) {
     a.m = std::min(slab, m - lo);
     a.perm = perm + lo;

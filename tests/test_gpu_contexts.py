@@ -1,0 +1,64 @@
+"""GPU tests of what contexts of one process owe each other and their caller:
+launch attributes that belong to the process, and results and memory that belong
+to the caller."""
+import numpy as np
+import pytest
+
+from qvort_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _deep(depth, seed=0):
+    """A ring and a triangle with one side of 0.1 x 2^-depth: a tree a few levels
+    on either side of `depth` levels deep."""
+    w = W.ring(40, 0.01, 1e-5, seed=seed)
+    a = np.array([0.0323, 0.0211, 0.0157])
+    tri = np.array([a, a + 0.1 * 2.0 ** -depth * np.array([0.9, 0.7, 0.8]), a + [1e-3, -2e-3, 1e-3]])
+    w.x = np.concatenate([w.x, tri])
+    w.infront = np.concatenate([w.infront, [42, 43, 41]]).astype(np.int32)
+    w.behind = np.concatenate([w.behind, [43, 41, 42]]).astype(np.int32)
+    w.params = dict(w.params, boundary="periodic", velocity="Tree", tree_theta=0.4, box_size=0.1)
+    return w
+
+
+def _ctx(w, **kw):
+    from qvort_b200 import lib as L
+
+    c = L.Context(L.default_params(**dict(w.params, **kw)))
+    c.set_points(w.x, w.infront, w.behind)
+    return c
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_deep_trees_in_several_contexts(precision):
+    """Walks and searches whose stacks need more shared memory than a launch has by
+    default: the size a kernel may ask for belongs to the process, so a context
+    with a shallower tree must not take it from one with a deeper tree."""
+    a, b = (_ctx(_deep(d), precision=precision) for d in (44, 34))
+    ua, ub = a.velocity()[0], b.velocity()[0]
+    pts = np.random.default_rng(0).uniform(-0.05, 0.05, (40, 3))
+    fa = a.field_velocity_tree(pts)[0]
+    ca = a.closest()
+    fb, cb = b.field_velocity_tree(pts)[0], b.closest()
+    for c, u, f, s in ((a, ua, fa, ca), (b, ub, fb, cb), (a, ua, fa, ca)):
+        assert np.array_equal(c.velocity()[0], u)
+        assert np.array_equal(c.field_velocity_tree(pts)[0], f)
+        assert all(np.array_equal(p, q) for p, q in zip(c.closest(), s))
+
+
+def test_deep_trees_in_several_batches():
+    """The same for batches, with the largest blocks a batch can be given."""
+    from qvort_b200 import lib as L
+
+    def batch(depth):
+        w = _deep(depth)
+        p = L.default_params(**dict(w.params, boundary="open", precision="mixed"))
+        return L.Batch(p, [(w.x, w.infront, w.behind)], ["Tree"], [1e-12])
+
+    a, b = batch(44), batch(20)
+    ua = a.velocity()
+    for t in (a, b, a):
+        t.set_config(8, 1, 0)
+        t.velocity()
+    assert np.array_equal(a.velocity(), ua)
