@@ -127,7 +127,7 @@ __global__ void k_lia_vjp(int n, const double *__restrict__ x, const int *__rest
 // atomics.  A two-pass split (a thread per target, then a thread per source)
 // evaluates every pair twice.  Bound: FP64 issue.  6,400 points, 27 images:
 // velocity and gradient together took 333 ms with two passes, divisions in every
-// image term and 50 blocks; 7.2 ms now, 2 of them the velocity (78 % of the FP64
+// image term and 50 blocks; 6.9 ms now, 2 of them the velocity (78 % of the FP64
 // rate at about 55 operations a pair; the x shifts unrolled took 255 registers,
 // two blocks per SM and 0.4 ms more).
 #define VT 128  // sources per block
@@ -163,10 +163,12 @@ __global__ void __launch_bounds__(VT, 3) k_dvjp(int na, const int *__restrict__ 
   const int q = blockIdx.x * VT + threadIdx.x;
   const bool live = q < na;
   const int j = live ? act[q] : 0, jj = j + 1;
-  double xj[3] = {0., 0., 0.}, s[3] = {0., 0., 0.}, dx[3] = {0., 0., 0.}, dg[3] = {0., 0., 0.};
+  double xj[3] = {0., 0., 0.}, gj[3] = {0., 0., 0.}, s[3], dx[3] = {0., 0., 0.}, dg[3] = {0., 0., 0.};
   if (live)
 #pragma unroll
-    for (int c = 0; c < 3; c++) { xj[c] = x[3 * j + c]; s[c] = gi[3 * j + c] - xj[c]; }
+    for (int c = 0; c < 3; c++) { xj[c] = x[3 * j + c]; gj[c] = gi[3 * j + c]; }
+#pragma unroll
+  for (int c = 0; c < 3; c++) s[c] = gj[c] - xj[c];
   const double c2 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
   const int t0 = t_lo + blockIdx.y * chunk_len, t1 = min(t_hi, t0 + chunk_len);
   for (int t = t0; t < t1; t += VG) {
@@ -184,8 +186,8 @@ __global__ void __launch_bounds__(VT, 3) k_dvjp(int na, const int *__restrict__ 
     __syncthreads();
 #pragma unroll 1
     for (int k = 0; k < m; k++) {
-      const Seg64<BC> e(xj[0] - tx[k][0], xj[1] - tx[k][1], xj[2] - tx[k][2], s[0], s[1], s[2], c2,
-                        L);
+      const Seg64<BC> e(xj[0] - tx[k][0], xj[1] - tx[k][1], xj[2] - tx[k][2], gj[0] - tx[k][0],
+                        gj[1] - tx[k][1], gj[2] - tx[k][2], s[0], s[1], s[2], c2, L);
       // src/timestep.f90:471, 496
       const bool own = jj == ti[k], skip = !live || jj == tb[k] || (own && e.NI == 1);
       const bool fast = __all_sync(0xffffffffu, skip || (e.far(own, L) && !e.on_line()));
@@ -291,22 +293,24 @@ __device__ __forceinline__ void warp_sums(double *v, int lane) {
   }
 }
 
-// Gradients of g . f (R x s) for a straight segment off the target (d = R.(R +
-// s) > 0): dR at fixed s, dS at fixed R (see Seg64::gradient).
-__device__ __forceinline__ void seg_gradient_pos(const double *R, const double *s, const double *g,
-                                                 double A, double B, double d, double *dR,
-                                                 double *dS) {
-  const SegD t = seg_d_pos(A, B, d);
+// Gradients of g . f (R1 x R2) for a straight segment s = R2 - R1 off the target (d =
+// R1.R2 > 0): dR with respect to both ends together, dS to the second alone (see
+// Seg64::gradient).
+__device__ __forceinline__ void seg_gradient_pos(const double *R1, const double *R2,
+                                                 const double *s, const double *g, double A,
+                                                 double B, double d, double *dR, double *dS) {
   const double h[3] = {s[1] * g[2] - s[2] * g[1], s[2] * g[0] - s[0] * g[2],
                        s[0] * g[1] - s[1] * g[0]};
-  const double gr[3] = {g[1] * R[2] - g[2] * R[1], g[2] * R[0] - g[0] * R[2],
-                        g[0] * R[1] - g[1] * R[0]};
-  const double Q = R[0] * h[0] + R[1] * h[1] + R[2] * h[2];
-  const double al = Q * t.fA2, be = Q * t.fw, ga = Q * t.fc2;
+  const double gr[3] = {g[1] * R1[2] - g[2] * R1[1], g[2] * R1[0] - g[0] * R1[2],
+                        g[0] * R1[1] - g[1] * R1[0]};
+  const double Q = (B < A ? R2[0] : R1[0]) * h[0] + (B < A ? R2[1] : R1[1]) * h[1] +
+                   (B < A ? R2[2] : R1[2]) * h[2];
+  const SegD t = seg_d_pos(A, B, d, Q);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    dR[c] = fma(t.f, h[c], fma(al, R[c], be * s[c]));
-    dS[c] = fma(t.f, gr[c], fma(be, R[c], ga * s[c]));
+    const double v = fma(t.fB2, R2[c], t.fd * R1[c]);
+    dS[c] = fma(t.f, gr[c], v);
+    dR[c] = fma(t.f, h[c], fma(t.fA2, R1[c], t.fd * R2[c])) + v;
   }
 }
 
@@ -381,8 +385,8 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
           R2[0] = P.b[0] - t0; R2[1] = P.b[1] - t1; R2[2] = P.b[2] - t2;
           const double d = R[0] * R2[0] + R[1] * R2[1] + R[2] * R2[2];
           if (d > 0.0625 * (sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2])) {
-            seg_gradient_pos(R, sv, gu, d2, R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2], d, dR,
-                             dS);
+            seg_gradient_pos(R, R2, sv, gu, d2, R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2], d,
+                             dR, dS);
           } else {  // beside the segment
             double g1[3], E1[3], E2[3];
 #pragma unroll
@@ -635,22 +639,23 @@ __global__ void k_energy_grad(int n, const double *__restrict__ x, const double 
 #define FW 4
 #define FV 12  // values per point: u (3), du/dx row-major (9)
 
-// du_r/dx_k -= d(f (R x s)_r)/dR_k for one term: with v = 2 fA R + fw s,
-// d(f (R x s)_r)/dR_k = (R x s)_r v_k + f eps(r,k,l) s_l.
-__device__ __forceinline__ void add_jacobian(const SegD &t, double X, double Y, double Z, double sx,
-                                             double sy, double sz, double cx, double cy, double cz,
+// du_r/dx_k -= d(f c_r)/dR_k for one term, c = R1 x s and both ends moving together:
+// with v = (2 fA + fd) R1 + (2 fB + fd) R2, d(f c_r)/dR_k = c_r v_k + f eps(r,k,l) s_l.
+__device__ __forceinline__ void add_jacobian(const SegD &t, const double *R1, const double *R2,
+                                             double sx, double sy, double sz, const double *c,
                                              double *J) {
-  const double vx = fma(t.fA2, X, t.fw * sx), vy = fma(t.fA2, Y, t.fw * sy),
-               vz = fma(t.fA2, Z, t.fw * sz);
-  J[0] -= cx * vx;
-  J[1] -= fma(cx, vy, t.f * sz);
-  J[2] -= fma(cx, vz, -t.f * sy);
-  J[3] -= fma(cy, vx, -t.f * sz);
-  J[4] -= cy * vy;
-  J[5] -= fma(cy, vz, t.f * sx);
-  J[6] -= fma(cz, vx, t.f * sy);
-  J[7] -= fma(cz, vy, -t.f * sx);
-  J[8] -= cz * vz;
+  const double p = t.fA2 + t.fd, q = t.fB2 + t.fd;
+  const double vx = fma(p, R1[0], q * R2[0]), vy = fma(p, R1[1], q * R2[1]),
+               vz = fma(p, R1[2], q * R2[2]);
+  J[0] -= c[0] * vx;
+  J[1] -= fma(c[0], vy, t.f * sz);
+  J[2] -= fma(c[0], vz, -t.f * sy);
+  J[3] -= fma(c[1], vx, -t.f * sz);
+  J[4] -= c[1] * vy;
+  J[5] -= fma(c[1], vz, t.f * sx);
+  J[6] -= fma(c[2], vx, t.f * sy);
+  J[7] -= fma(c[2], vy, -t.f * sx);
+  J[8] -= c[2] * vz;
 }
 
 template <int BC, bool GI>
@@ -672,33 +677,27 @@ __global__ void __launch_bounds__(FW * 32) k_field(int m, const double *__restri
     const double2 *s = reinterpret_cast<const double2 *>(src + 8 * (size_t)(live ? j : j0));
     const double2 s0 = s[0], s1 = s[1], s2 = s[2];
     const double sx = s1.y, sy = s2.x, sz = s2.y, c = s[3].x;
-    const Seg64<BC> e(s0.x - X, s0.y - Y, s1.x - Z, sx, sy, sz, c, L);
+    const double dx = s0.x - X, dy = s0.y - Y, dz = s1.x - Z;
+    const Seg64<BC> e(dx, dy, dz, dx + sx, dy + sy, dz + sz, sx, sy, sz, c, L);
     const bool fast = __all_sync(0xffffffffu, !live || e.far(false, L));
     if (!live) continue;
     constexpr int NI = Seg64<BC>::NI;
     if (!GI) e.velocity(L, fast, false, v[0], v[1], v[2]);
 #pragma unroll 1
     for (int im = GI ? 0 : NI / 2; im < (GI ? NI : NI / 2 + 1); im++) {
-      double rx, ry, rz;
-      e.image(im, L, rx, ry, rz);
-      const double A = rx * rx + ry * ry + rz * rz, w = rx * sx + ry * sy + rz * sz;
-      const double cx = ry * sz - rz * sy, cy = rz * sx - rx * sz, cz = rx * sy - ry * sx;
-      const double c2 = cx * cx + cy * cy + cz * cz;
+      double R1[3], R2[3], cr[3], A, B, d;
+      e.image(im, L, R1, R2);
+      e.image_term(R1, R2, A, B, d, cr);
+      const double c2 = cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2];
       // a point on the segment's line: no term (4ac - b^2 = 0, src/timestep.f90:531)
       if (c2 == 0.) continue;
-      SegD q;
-      if (fast) {
-        q = seg_d_pos(A, A + 2. * w + c, A + w);
-      } else {
-        const double ex = rx + sx, ey = ry + sy, ez = rz + sz;
-        q = seg_d_any(A, ex * ex + ey * ey + ez * ez, A + w, c2);
-      }
+      const SegD q = fast ? seg_d_pos(A, B, d, 1.) : seg_d_any(A, B, d, c2, 1.);
       if (GI) {
-        v[0] += q.f * cx;
-        v[1] += q.f * cy;
-        v[2] += q.f * cz;
+        v[0] += q.f * cr[0];
+        v[1] += q.f * cr[1];
+        v[2] += q.f * cr[2];
       }
-      add_jacobian(q, rx, ry, rz, sx, sy, sz, cx, cy, cz, v + 3);
+      add_jacobian(q, R1, R2, sx, sy, sz, cr, v + 3);
     }
   }
 #pragma unroll

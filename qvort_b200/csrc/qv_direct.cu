@@ -362,7 +362,8 @@ __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const in
     for (int k = 0; k < m; k++) {
       const double *s = tile + 8 * k;
       const int jj = (int)s[7];
-      const Seg64<BC> e(s[0] - xi0, s[1] - xi1, s[2] - xi2, s[3], s[4], s[5], s[6], L);
+      const double dx = s[0] - xi0, dy = s[1] - xi1, dz = s[2] - xi2;
+      const Seg64<BC> e(dx, dy, dz, dx + s[3], dy + s[4], dz + s[5], s[3], s[4], s[5], s[6], L);
       // src/timestep.f90:471, 496
       const bool own = jj == ii, skip = !live || jj == bi || (own && e.NI == 1);
       // one form for the whole warp
@@ -404,8 +405,10 @@ __global__ void __launch_bounds__(D64S) k_direct64_small(int n, const double *__
     const bool live = j < n && inf[j] != 0;
     const int k = live ? j : i;
     const double y0 = x[3 * k], y1 = x[3 * k + 1], y2 = x[3 * k + 2];
-    const double s0 = gi[3 * k] - y0, s1 = gi[3 * k + 1] - y1, s2 = gi[3 * k + 2] - y2;
-    const Seg64<BC> e(y0 - x0, y1 - x1, y2 - x2, s0, s1, s2, s0 * s0 + s1 * s1 + s2 * s2, L);
+    const double g0 = gi[3 * k], g1 = gi[3 * k + 1], g2 = gi[3 * k + 2];
+    const double s0 = g0 - y0, s1 = g1 - y1, s2 = g2 - y2;
+    const Seg64<BC> e(y0 - x0, y1 - x1, y2 - x2, g0 - x0, g1 - x1, g2 - x2, s0, s1, s2,
+                      s0 * s0 + s1 * s1 + s2 * s2, L);
     // src/timestep.f90:471, 496
     const bool own = j == i, skip = !live || j + 1 == bi || (own && e.NI == 1);
     const bool fast = __all_sync(0xffffffffu, skip || e.far(own, L));

@@ -52,41 +52,41 @@ __device__ __forceinline__ double seg_f_any(double A, double B, double d, double
   return (a + b) / (ab * e);
 }
 
-// f and its partial derivatives as a function of A = |R1|^2, w = R1.s and
-// c = |s|^2 (B = A + 2 w + c, d = A + w): with a = |R1|, b = |R2|, m = a b, q =
-// 1 / m, e = m + d and g = f / e (1 / m + 1 / B and the like written through the
-// reciprocals at hand; the sum a + b in f = (a + b) / (m e) cancels from the
-// derivatives of its logarithm)
-//   2 fA = -(f ((1/a - 1/b)^2 + q) + g ((A + B) q + 2))
-//   2 fc = -(1/b^3 + f A q) / e,   fw = 2 fc - g.
-// The gradients of u = f (R1 x s) follow by the chain rule.
+// f and its partial derivatives as a function of A = |R1|^2, B = |R2|^2 and d =
+// R1.R2: with a = |R1|, b = |R2| and e = a b + d, f = (a + b) / (a b e) and
+//   2 fA = -(1/a^2 + f b) / (a e),   2 fB = -(1/b^2 + f a) / (b e),   fd = -f / e,
+// sums of one sign, so a target near either end keeps every digit, as long as R2
+// and the products above are formed from R2 itself.  (The derivatives by R1 and
+// s, B = |R1|^2 + 2 R1.s + |s|^2, save a vector sum but cancel near R2's end: 5e-14
+// of the gradient at 0.07 |s| from it.)  The gradients of u = f (R1 x R2) follow by
+// the chain rule.
 struct SegD {
-  double f, fA2, fw, fc2;  // f, 2 df/dA, df/dw, 2 df/dc
+  double f, fA2, fB2, fd;  // f, and Q times 2 df/dA, 2 df/dB, df/dd
 };
-__device__ __forceinline__ SegD seg_d_of(double A, double B, double ra, double rb, double q,
-                                         double ie) {
+__device__ __forceinline__ SegD seg_d_of(double A, double B, double ra, double rb, double ie,
+                                         double Q) {
   SegD r;
   r.f = (ra + rb) * ie;
-  const double g = r.f * ie, dr = ra - rb;
-  r.fc2 = -ie * fma(rb * rb, rb, r.f * (A * q));
-  r.fw = r.fc2 - g;
-  r.fA2 = -fma(r.f, fma(dr, dr, q), g * fma(A + B, q, 2.));
+  const double qe = -Q * ie;
+  r.fA2 = (qe * ra) * fma(ra, ra, r.f * (B * rb));
+  r.fB2 = (qe * rb) * fma(rb, rb, r.f * (A * ra));
+  r.fd = qe * r.f;
   return r;
 }
 // d > 0
-__device__ __forceinline__ SegD seg_d_pos(double A, double B, double d) {
+__device__ __forceinline__ SegD seg_d_pos(double A, double B, double d, double Q) {
   const double ra = rsqrt_pos(A), rb = rsqrt_pos(B), q = ra * rb;
-  return seg_d_of(A, B, ra, rb, q, div_pos(q, fma(d, q, 1.)));
+  return seg_d_of(A, B, ra, rb, div_pos(q, fma(d, q, 1.)), Q);
 }
 // any d; c2 = |R1 x s|^2 (0: a point on the segment's line, no term)
-__device__ __forceinline__ SegD seg_d_any(double A, double B, double d, double c2) {
+__device__ __forceinline__ SegD seg_d_any(double A, double B, double d, double c2, double Q) {
   if (!(c2 > 0.) || !(B > 0.)) {
     const double z = c2 != c2 ? c2 : 0.;
     return SegD{z, z, z, z};
   }
   const double a = sqrt(A), b = sqrt(B), m = a * b;
   const double e = d < 0. ? c2 / (m - d) : m + d;
-  return seg_d_of(A, B, 1. / a, 1. / b, 1. / m, 1. / e);
+  return seg_d_of(A, B, 1. / a, 1. / b, 1. / e, Q);
 }
 
 // ------------------------------------------------------------ image sums
@@ -115,43 +115,67 @@ __device__ __forceinline__ double least(const double *v) {
 }
 
 // One source segment against one target in every image.  Per axis and shift:
-// R1 = x_j + shift - x_i (r) and the parts of |R1|^2 (p) and R1.R2 (g); the sum
-// over the axes gives an image's value.
+// R1 = x_j + shift - x_i (r), R2 = ghost_j + shift - x_i (e) and the parts of
+// |R1|^2 (p), |R2|^2 (t) and R1.R2 (g); the sum over the axes gives an image's value.
 template <int BC>
 struct Seg64 {
   static constexpr int PX = Img<BC>::PX, PY = Img<BC>::PY, PZ = Img<BC>::PZ;
   static constexpr int NI = PX * PY * PZ;
   double sx, sy, sz, c;  // segment vector s and |s|^2
-  double rx[PX], ry[PY], rz[PZ], px[PX], py[PY], pz[PZ], gx[PX], gy[PY], gz[PZ];
-  __device__ __forceinline__ Seg64(double dx, double dy, double dz, double sx_, double sy_,
-                                   double sz_, double c_, double L)
+  double rx[PX], ry[PY], rz[PZ], ex[PX], ey[PY], ez[PZ];
+  double px[PX], py[PY], pz[PZ], tx[PX], ty[PY], tz[PZ], gx[PX], gy[PY], gz[PZ];
+  // (dx, dy, dz) = R1 and (fx, fy, fz) = R2 of the unshifted image
+  __device__ __forceinline__ Seg64(double dx, double dy, double dz, double fx, double fy, double fz,
+                                   double sx_, double sy_, double sz_, double c_, double L)
       : sx(sx_), sy(sy_), sz(sz_), c(c_) {
-    axis_shifts<PX>(dx, L, rx);
-    axis_shifts<PY>(dy, L, ry);
-    axis_shifts<PZ>(dz, L, rz);
+    axis<PX>(dx, fx, L, rx, ex, px, tx, gx);
+    axis<PY>(dy, fy, L, ry, ey, py, ty, gy);
+    axis<PZ>(dz, fz, L, rz, ez, pz, tz, gz);
+  }
+  template <int P>
+  __device__ __forceinline__ static void axis(double d, double f, double L, double *r, double *e,
+                                              double *p, double *t, double *g) {
+    axis_shifts<P>(d, L, r);
+    axis_shifts<P>(f, L, e);
 #pragma unroll
-    for (int e = 0; e < PX; e++) { px[e] = rx[e] * rx[e]; gx[e] = fma(rx[e], sx, px[e]); }
-#pragma unroll
-    for (int e = 0; e < PY; e++) { py[e] = ry[e] * ry[e]; gy[e] = fma(ry[e], sy, py[e]); }
-#pragma unroll
-    for (int e = 0; e < PZ; e++) { pz[e] = rz[e] * rz[e]; gz[e] = fma(rz[e], sz, pz[e]); }
+    for (int k = 0; k < P; k++) { p[k] = r[k] * r[k]; t[k] = e[k] * e[k]; g[k] = r[k] * e[k]; }
   }
   // Whether R1.R2 > |s|^2 / 16 in every image that is summed: the _pos forms
-  // hold there, and |R2|^2 = R1.R2 + R1.s + |s|^2 keeps its digits (both ends
-  // lie well off the target).  Every point's own neighbours pass, so only
-  // points about to reconnect take the general form.  The least R1.R2 over
-  // the images is the sum of the axes' least parts.  skip_main (the point's
-  // own segment): the other images lie a box side away.
+  // hold there (both ends lie off the target, by 0.06 |s| at least).  Every
+  // point's own neighbours pass, so only points about to reconnect take the
+  // general form.  The least R1.R2 over the images is the sum of the axes' least
+  // parts.  skip_main (the point's own segment): the other images lie a box side
+  // away.
   __device__ __forceinline__ bool far(bool skip_main, double L) const {
     if (skip_main) return c < 0.25 * L * L;
     return least<PX>(gx) + least<PY>(gy) + least<PZ>(gz) > 0.0625 * c;
   }
-  // R1 of image m (m = (a PY + b) PZ + k, shifts ascending)
-  __device__ __forceinline__ void image(int m, double L, double &X, double &Y, double &Z) const {
-    const int a = m / (PY * PZ), b = (m / PZ) % PY, k = m % PZ;
-    X = PX == 3 ? rx[PX / 2] + (a - 1) * L : rx[0];
-    Y = PY == 3 ? ry[PY / 2] + (b - 1) * L : ry[0];
-    Z = PZ == 3 ? rz[PZ / 2] + (k - 1) * L : rz[0];
+  // R1 and R2 of image m (m = (a PY + b) PZ + k, shifts ascending)
+  __device__ __forceinline__ void image(int m, double L, double *R1, double *R2) const {
+    const double X = PX == 3 ? (m / (PY * PZ) - 1) * L : 0.,
+                 Y = PY == 3 ? ((m / PZ) % PY - 1) * L : 0., Z = PZ == 3 ? (m % PZ - 1) * L : 0.;
+    R1[0] = rx[PX / 2] + X; R1[1] = ry[PY / 2] + Y; R1[2] = rz[PZ / 2] + Z;
+    R2[0] = ex[PX / 2] + X; R2[1] = ey[PY / 2] + Y; R2[2] = ez[PZ / 2] + Z;
+  }
+  // A, B, d and R1 x s = R2 x s of an image, the product from the nearer end: the
+  // other one's cancels beside the segment's line.  The target is on that line
+  // where R1 x s vanishes.
+  __device__ __forceinline__ void image_term(const double *R1, const double *R2, double &A,
+                                             double &B, double &d, double *cr) const {
+    A = R1[0] * R1[0] + R1[1] * R1[1] + R1[2] * R1[2];
+    B = R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2];
+    d = R1[0] * R2[0] + R1[1] * R2[1] + R1[2] * R2[2];
+    cross_s(R1, cr);
+    if (B < A && (cr[0] != 0. || cr[1] != 0. || cr[2] != 0.)) {
+      double q[3];
+      cross_s(R2, q);
+      if (q[0] != 0. || q[1] != 0. || q[2] != 0.) { cr[0] = q[0]; cr[1] = q[1]; cr[2] = q[2]; }
+    }
+  }
+  __device__ __forceinline__ void cross_s(const double *R, double *cr) const {
+    cr[0] = R[1] * sz - R[2] * sy;
+    cr[1] = R[2] * sx - R[0] * sz;
+    cr[2] = R[0] * sy - R[1] * sx;
   }
   // Adds the velocity terms of every image (the unshifted one unless skip_main)
   // to (ax, ay, az).  s is the same in all of them, so f and f R1 are summed
@@ -163,28 +187,24 @@ struct Seg64 {
     if (!fast) {
 #pragma unroll 1
       for (int m = 0; m < NI; m++) {
-        if (skip_main && m == NI / 2) continue;  // the middle one is unshifted
-        double X, Y, Z;
-        image(m, L, X, Y, Z);
-        const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
-        const double cx = Y * sz - Z * sy, cy = Z * sx - X * sz, cz = X * sy - Y * sx;
-        const double ex = X + sx, ey = Y + sy, ez = Z + sz;
-        const double f =
-            seg_f_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
-        ax += f * cx;
-        ay += f * cy;
-        az += f * cz;
+        if (skip_main && m == NI / 2) continue;
+        double R1[3], R2[3], cr[3], A, B, d;
+        image(m, L, R1, R2);
+        image_term(R1, R2, A, B, d, cr);
+        const double f = seg_f_any(A, B, d, cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+        ax += f * cr[0];
+        ay += f * cr[1];
+        az += f * cr[2];
       }
       return;
     }
     double fx[PX], fy[PY], fz[PZ];  // sum of f at each shift of an axis
-    double tx[PX], ty[PY], tz[PZ];  // parts of |R2|^2 = R1.R2 + R1.s + |s|^2
 #pragma unroll
-    for (int k = 0; k < PX; k++) { fx[k] = 0.; tx[k] = fma(rx[k], sx, gx[k] + c); }
+    for (int k = 0; k < PX; k++) fx[k] = 0.;
 #pragma unroll
-    for (int k = 0; k < PY; k++) { fy[k] = 0.; ty[k] = fma(ry[k], sy, gy[k]); }
+    for (int k = 0; k < PY; k++) fy[k] = 0.;
 #pragma unroll
-    for (int k = 0; k < PZ; k++) { fz[k] = 0.; tz[k] = fma(rz[k], sz, gz[k]); }
+    for (int k = 0; k < PZ; k++) fz[k] = 0.;
 #pragma unroll
     for (int a = 0; a < PX; a++) {
 #pragma unroll
@@ -238,81 +258,85 @@ struct Seg64 {
       for (int k = 0; k < PZ; k++) z |= rz[k] * sx - rx[a] * sz == 0.;
     return z;
   }
-  // For an upstream g, the gradient of g . sum over images of f (R1 x s): dR
+  // For an upstream g, the gradient of g . sum over images of f (R1 x R2): dR
   // with respect to x_j at fixed s (minus the target's), dS with respect to s.
-  // With h = s x g, Q = g.(R1 x s) = R1.h, alpha = 2 Q fA, beta = Q fw:
-  //   dR = h sum f + sum alpha R1 + s sum beta
-  //   dS = g x sum f R1 + sum beta R1 + s sum Q 2 fc
+  // With h = s x g, Q = g.(R1 x R2) = R1.h = R2.h, alpha = 2 Q fA, beta = 2 Q fB and
+  // gamma = Q fd:
+  //   dS = g x sum f R1 + sum beta R2 + sum gamma R1
+  //   dR = h sum f + sum alpha R1 + sum gamma R2 + sum beta R2 + sum gamma R1
+  // and sum gamma R2 = sum gamma R1 + s sum gamma.  Q is taken from the end that is
+  // nearer in the nearest image: beside the segment's line the other one cancels.
   // fast: far() holds and on_line() does not.
   __device__ __forceinline__ void gradient(double ux, double uy, double uz, double L, bool fast,
                                            bool skip_main, double *dR, double *dS) const {
     const double hx = sy * uz - sz * uy, hy = sz * ux - sx * uz, hz = sx * uy - sy * ux;
-    double f0 = 0., b0 = 0., c0 = 0.;
-    double fX = 0., fY = 0., fZ = 0., aX = 0., aY = 0., aZ = 0., bX = 0., bY = 0., bZ = 0.;
+    double f0 = 0., g0 = 0.;
+    double fX = 0., fY = 0., fZ = 0., aX = 0., aY = 0., aZ = 0.;  // sums of f R1, alpha R1,
+    double bX = 0., bY = 0., bZ = 0., cX = 0., cY = 0., cZ = 0.;  // beta R2 and gamma R1
     if (fast) {
-      double ty[PY], tz[PZ], qy[PY], qz[PZ];
-#pragma unroll
-      for (int k = 0; k < PY; k++) { ty[k] = fma(ry[k], sy, gy[k]); qy[k] = ry[k] * hy; }
-#pragma unroll
-      for (int k = 0; k < PZ; k++) { tz[k] = fma(rz[k], sz, gz[k]); qz[k] = rz[k] * hz; }
+      const bool near2 = least<PX>(tx) + least<PY>(ty) + least<PZ>(tz) <
+                         least<PX>(px) + least<PY>(py) + least<PZ>(pz);
 #pragma unroll 1  // a third of the code and registers: three blocks per SM
       for (int a = 0; a < PX; a++) {
-        const double xa = PX == 3 ? rx[PX / 2] + (a - 1) * L : rx[0], pa = xa * xa,
-                     ga = fma(xa, sx, pa), ta = fma(xa, sx, ga + c), qa = xa * hx;
-        double fa = 0., aa = 0., ba = 0.;  // sums over the shifts (b, k) of this a
+        const double sh = PX == 3 ? (a - 1) * L : 0., xa = rx[PX / 2] + sh, ea = ex[PX / 2] + sh,
+                     pa = xa * xa, ga = xa * ea, ta = ea * ea, qa = (near2 ? ea : xa) * hx;
+        double fa = 0., aa = 0., ba = 0., ca = 0.;  // sums over the shifts (b, k) of this a
 #pragma unroll
         for (int b = 0; b < PY; b++) {
-          const double pxy = pa + py[b], gxy = ga + gy[b], txy = ta + ty[b],
-                       qxy = qa + qy[b];
-          double fb = 0., ab = 0., bb = 0.;
+          // from r and e again, an fma where p, t and g need an addition: those
+          // arrays would take more registers than there are
+          const double pxy = fma(ry[b], ry[b], pa), gxy = fma(ry[b], ey[b], ga),
+                       txy = fma(ey[b], ey[b], ta), qxy = fma(near2 ? ey[b] : ry[b], hy, qa);
+          double fb = 0., ab = 0., bb = 0., cb = 0.;
 #pragma unroll
           for (int k = 0; k < PZ; k++) {
-            double A = pxy + pz[k], B = txy + tz[k], d = gxy + gz[k];
-            double Q = qxy + qz[k];
+            double A = fma(rz[k], rz[k], pxy), B = fma(ez[k], ez[k], txy);
+            double d = fma(rz[k], ez[k], gxy), Q = fma(near2 ? ez[k] : rz[k], hz, qxy);
             const bool own = skip_main && (a * PY + b) * PZ + k == NI / 2;
             if (own) A = B = d = 1.;
-            SegD t = seg_d_pos(A, B, d);
-            if (own) t.f = Q = 0.;
-            const double al = Q * t.fA2, be = Q * t.fw;
-            c0 = fma(Q, t.fc2, c0);
-            fb += t.f; ab += al; bb += be;
+            if (own) Q = 0.;
+            SegD t = seg_d_pos(A, B, d, Q);
+            if (own) t.f = 0.;
+            fb += t.f; ab += t.fA2; bb += t.fB2; cb += t.fd;
             fZ = fma(t.f, rz[k], fZ);
-            aZ = fma(al, rz[k], aZ);
-            bZ = fma(be, rz[k], bZ);
+            aZ = fma(t.fA2, rz[k], aZ);
+            bZ = fma(t.fB2, ez[k], bZ);
+            cZ = fma(t.fd, rz[k], cZ);
           }
-          fa += fb; aa += ab; ba += bb;
+          fa += fb; aa += ab; ba += bb; ca += cb;
           fY = fma(fb, ry[b], fY);
           aY = fma(ab, ry[b], aY);
-          bY = fma(bb, ry[b], bY);
+          bY = fma(bb, ey[b], bY);
+          cY = fma(cb, ry[b], cY);
         }
-        f0 += fa; b0 += ba;
+        f0 += fa; g0 += ca;
         fX = fma(fa, xa, fX);
         aX = fma(aa, xa, aX);
-        bX = fma(ba, xa, bX);
+        bX = fma(ba, ea, bX);
+        cX = fma(ca, xa, cX);
       }
     } else {
 #pragma unroll 1
       for (int m = 0; m < NI; m++) {
         if (skip_main && m == NI / 2) continue;
-        double X, Y, Z;
-        image(m, L, X, Y, Z);
-        const double A = X * X + Y * Y + Z * Z, w = X * sx + Y * sy + Z * sz;
-        const double cx = Y * sz - Z * sy, cy = Z * sx - X * sz, cz = X * sy - Y * sx;
-        const double ex = X + sx, ey = Y + sy, ez = Z + sz;
-        const SegD t =
-            seg_d_any(A, ex * ex + ey * ey + ez * ez, A + w, cx * cx + cy * cy + cz * cz);
-        const double Q = X * hx + Y * hy + Z * hz, al = Q * t.fA2, be = Q * t.fw;
-        f0 += t.f; b0 += be; c0 += Q * t.fc2;
-        fX += t.f * X; fY += t.f * Y; fZ += t.f * Z;
-        aX += al * X; aY += al * Y; aZ += al * Z;
-        bX += be * X; bY += be * Y; bZ += be * Z;
+        double R1[3], R2[3], cr[3], A, B, d;
+        image(m, L, R1, R2);
+        image_term(R1, R2, A, B, d, cr);
+        const SegD t = seg_d_any(A, B, d, cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2],
+                                 cr[0] * ux + cr[1] * uy + cr[2] * uz);
+        const double al = t.fA2, be = t.fB2, ga = t.fd;
+        f0 += t.f; g0 += ga;
+        fX += t.f * R1[0]; fY += t.f * R1[1]; fZ += t.f * R1[2];
+        aX += al * R1[0]; aY += al * R1[1]; aZ += al * R1[2];
+        bX += be * R2[0]; bY += be * R2[1]; bZ += be * R2[2];
+        cX += ga * R1[0]; cY += ga * R1[1]; cZ += ga * R1[2];
       }
     }
-    dR[0] = fma(hx, f0, fma(sx, b0, aX));
-    dR[1] = fma(hy, f0, fma(sy, b0, aY));
-    dR[2] = fma(hz, f0, fma(sz, b0, aZ));
-    dS[0] = fma(sx, c0, bX) + (uy * fZ - uz * fY);
-    dS[1] = fma(sy, c0, bY) + (uz * fX - ux * fZ);
-    dS[2] = fma(sz, c0, bZ) + (ux * fY - uy * fX);
+    dS[0] = bX + cX + (uy * fZ - uz * fY);
+    dS[1] = bY + cY + (uz * fX - ux * fZ);
+    dS[2] = bZ + cZ + (ux * fY - uy * fX);
+    dR[0] = fma(hx, f0, fma(sx, g0, aX + cX)) + (bX + cX);
+    dR[1] = fma(hy, f0, fma(sy, g0, aY + cY)) + (bY + cY);
+    dR[2] = fma(hz, f0, fma(sz, g0, aZ + cZ)) + (bZ + cZ);
   }
 };
