@@ -339,7 +339,6 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
     int ma = 0, mb = 0, mc = 0;
     if (sl >= ANSPLIT) qv_img_shift(BC, sl - ANSPLIT, &ma, &mb, &mc);
     const double s[3] = {shift_of(ma, a.L), shift_of(mb, a.L), shift_of(mc, a.L)};
-    const double t0 = xi[0] - s[0], t1 = xi[1] - s[1], t2 = xi[2] - s[2];
     // the root's own decision; the unshifted image's tasks then take one child
     const bool lone = r.count == 1;
     const bool go = live && (lone ? sl == 0 || sl >= ANSPLIT
@@ -357,7 +356,10 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
       const int node = e.x;
       const bool in = (((unsigned)e.y) >> lane) & 1u;
       const WNode64 h = a.w64[node];
-      const double v[3] = {t0 - h.cx, t1 - h.cy, t2 - h.cz};
+      // x - (cent + shift) with the velocity walk's roundings: x - shift - cent
+      // differs by a unit of the box, which for a small cell is more than the
+      // margin of the test below
+      const double v[3] = {xi[0] - (h.cx + s[0]), xi[1] - (h.cy + s[1]), xi[2] - (h.cz + s[2])};
       const double d2 = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));
       bool open = false, far = false, leaf = false;
       double w[16];
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
         leaf = j != ii && j != bi && j != fi;
       } else if (in) {
         const double rc = fma(h.width, ith, a.extra ? h.geo : 0.), rc2 = rc * rc;
-        // node_test as in the velocity walk: the reference's expression near rc
+        // as in the velocity walk (fill_ent64): the reference's expression near rc
         open = !sure || !(fabs(d2 - rc2) > 1e-11 * rc2)
                    ? exact_open(exact_dist(xi, h, s), h, a.theta, a.extra)
                    : d2 < rc2;
@@ -382,7 +384,8 @@ __global__ void __launch_bounds__(AW * 32, 4) k_walk_vjp(WalkVjpArgs a) {
           double sv[3], R2[3];
 #pragma unroll
           for (int c = 0; c < 3; c++) sv[c] = P.b[c] - P.a[c];
-          R2[0] = P.b[0] - t0; R2[1] = P.b[1] - t1; R2[2] = P.b[2] - t2;
+#pragma unroll
+          for (int c = 0; c < 3; c++) R2[c] = P.b[c] + s[c] - xi[c];
           const double d = R[0] * R2[0] + R[1] * R2[1] + R[2] * R2[2];
           if (d > 0.0625 * (sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2])) {
             seg_gradient_pos(R, R2, sv, gu, d2, R2[0] * R2[0] + R2[1] * R2[1] + R2[2] * R2[2], d,
