@@ -197,7 +197,8 @@ int qv_steps(qv_ctx *ctx, int itime0, int nsteps);
 /* ------------------------------------------------------------- derivatives
  * Hand-written derivatives of the path (no counterpart in the reference, which
  * has no adjoint; they serve gradient-based studies and the stiff solver). */
-/* calc_velocity for every active point into a device array u (3n). */
+/* calc_velocity for every active point into a device array u (3n); on an error u
+ * is left as it was. */
 int qv_velocity_device(qv_ctx *ctx, double *u);
 /* x_bar = J^T u_bar of calc_velocity (src/timestep.f90:180-309) at the
  * context's positions, through LIA, the direct sum or the tree walk (topology

@@ -757,15 +757,18 @@ extern "C" int qv_velocity(qv_ctx *c, double *u, double *u_li, double *u_bs, lon
   return velocity_collect(c, eval_count);
 }
 
-// The velocities into a device array, in one wait.
+// The velocities into a device array, which is written only once the status is
+// known: after an error it holds what it held.
 extern "C" int qv_velocity_device(qv_ctx *c, double *u_out) {
   if (!c || !u_out) return QV_ERR_ARG;
   if (c->n == 0) return QV_OK;
   int rc = velocity_launch(c);
   if (rc) return rc;
+  if ((rc = velocity_collect(c, nullptr))) return rc;
   QV_CUDA(c, cudaMemcpyAsync(u_out, c->u, sizeof(double) * 3 * (size_t)c->n,
                              cudaMemcpyDeviceToDevice, c->stream));
-  return velocity_collect(c, nullptr);
+  QV_CUDA(c, cudaStreamSynchronize(c->stream));
+  return QV_OK;
 }
 
 extern "C" int qv_step_ab(qv_ctx *c) {

@@ -62,3 +62,22 @@ def test_deep_trees_in_several_batches():
         t.set_config(8, 1, 0)
         t.velocity()
     assert np.array_equal(a.velocity(), ua)
+
+
+def test_velocity_device_leaves_the_array_alone_on_a_singularity():
+    import torch
+
+    from qvort_b200 import lib as L
+
+    w = W.ring(40, 0.01, 1e-5)
+    w.x[20] = w.x[3] + [1e-16, 0.0, 0.0]  # not neighbours, within epsilon
+    c = _ctx(w, velocity="Tree", tree_theta=0.4, precision="fp64")
+    u = torch.full((w.n, 3), 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with pytest.raises(L.QvError):
+        c.velocity_device(u.data_ptr())
+    assert (u == 7.0).all()
+    w.x[20] = W.ring(40, 0.01, 1e-5).x[20]
+    c.set_points(w.x, w.infront, w.behind)
+    c.velocity_device(u.data_ptr())
+    assert np.array_equal(u.cpu().numpy(), c.velocity()[0])
