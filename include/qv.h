@@ -326,7 +326,8 @@ int qv_get_links(qv_ctx *ctx, int *infront, int *behind);
 /* Instrumentation (no reference counterpart beyond the seg_fault trace flags,
  * src/run.f90:31-166, and eval_counter, src/tree.f90:40).  With profiling on,
  * the phases below are bracketed by CUDA events on the context's stream and
- * their device times accumulate into ms[QV_NPHASES]. */
+ * their device times accumulate into ms[QV_NPHASES].  Ghosts and local term
+ * are one launch without profiling and two with it. */
 /* ghosts, tree build, local term, non-local sum, update, search, wrap, two
  * parts of the tree build (the level-synchronous construction and the
  * moments), the line operations (pinsert, premove), and inside the non-local

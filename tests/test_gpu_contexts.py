@@ -81,3 +81,22 @@ def test_velocity_device_leaves_the_array_alone_on_a_singularity():
     c.set_points(w.x, w.infront, w.behind)
     c.velocity_device(u.data_ptr())
     assert np.array_equal(u.cpu().numpy(), c.velocity()[0])
+
+
+@pytest.mark.parametrize("bc", ["open", "periodic"])
+@pytest.mark.parametrize("rk3", [0, 1])
+@pytest.mark.parametrize("velocity", ["BS", "Tree"])
+def test_profiled_steps_report_ghosts_and_local_term(velocity, rk3, bc):
+    """Each phase of a step has its own time, and profiling changes no bit."""
+    w = W.ring(300, 0.01, 1e-5, seed=1)
+    kw = dict(velocity=velocity, tree_theta=0.4 if velocity == "Tree" else 0.0, boundary=bc,
+              runge_kutta=rk3, precision="fp64")
+    a, b = _ctx(w, **kw), _ctx(w, **kw)
+    a.profile(True)
+    for k in range(1, 5):
+        a.step(k)
+        b.step(k)
+    t = a.phase_times()
+    for ph in ("ghosts", "local", "nonlocal", "update", "wrap"):
+        assert t[ph] > 0.0, ph
+    assert all(np.array_equal(p, q) for p, q in zip(a.get_points(), b.get_points()))
