@@ -641,6 +641,7 @@ __global__ void k_energy_grad(int n, const double *__restrict__ x, const double 
 // ms with a thread per point, 0.23 ms per call now (copies included).
 #define FW 4
 #define FV 12  // values per point: u (3), du/dx row-major (9)
+#define QV_FIELD_SLAB (1 << 20)  // points per launch (bounds the partial sums: 101 MB)
 
 // du_r/dx_k -= d(f c_r)/dR_k for one term, c = R1 x s and both ends moving together:
 // with v = (2 fA + fd) R1 + (2 fB + fd) R2, d(f c_r)/dR_k = c_r v_k + f eps(r,k,l) s_l.
@@ -715,9 +716,9 @@ __global__ void __launch_bounds__(FW * 32) k_field(int m, const double *__restri
 }
 
 // Sum of the chunks' partial values, a warp per value (lanes stride over the
-// chunks, in a fixed order): out = u (3m), du/dx (9m).
+// chunks, in a fixed order).
 __global__ void k_field_reduce(int m, int nchunk, const double *__restrict__ part, double scale,
-                               double *out) {
+                               double *u, double *dudx) {
   const long e = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long tot = (long)m * FV;
@@ -728,7 +729,7 @@ __global__ void k_field_reduce(int m, int nchunk, const double *__restrict__ par
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   const long t = e / FV;
   const int k = (int)(e - t * FV);
-  if (lane == 0) out[k < 3 ? 3 * t + k : 3L * m + 9 * t + (k - 3)] = s * scale;
+  if (lane == 0) (k < 3 ? u[3 * t + k] : dudx[9 * t + (k - 3)]) = s * scale;
 }
 
 // ------------------------------------------------------------------ host side
@@ -1006,46 +1007,46 @@ extern "C" int qv_field_velocity(qv_ctx *c, int m, const double *pts, int grad_i
   const int na = c->n_act;
   // about four warps for each of the chip's FP64-saturating slots (16 per SM);
   // a chunk holds at least one source per lane
-  const int ng = nblk(m, FW);
-  const int want = (int)std::max(1L, 64L * c->sm_count / m);
+  const int slab = std::min(m, QV_FIELD_SLAB);
+  const int want = (int)std::max(1L, 64L * c->sm_count / slab);
   const int chunk_len = std::max(1, nblk(nblk(na, want), 32)) * 32;
   const int nchunk = std::max(1, nblk(na, chunk_len));
-  const size_t np = 3 * (size_t)m, nv = FV * (size_t)m;
-  // points, results and partial sums
-  const size_t need = sizeof(double) * (np + nv * (1 + (size_t)nchunk));
-  if (need > c->field_bytes) {
-    c->field_bytes = 0;  // the old buffer goes first
-    if ((rc = qv_grow(c, (void **)&c->field_buf, need))) return rc;
-    c->field_bytes = need;
-  }
-  double *dp = c->field_buf, *du = dp + np, *part = du + nv;
+  const size_t np = 3 * (size_t)m;
+  // points, results and a slab's partial sums
+  FieldBuf buf(c);
+  if ((rc = buf.reserve(sizeof(double) * (5 * np + FV * (size_t)slab * nchunk)))) return rc;
+  double *dp = c->field_buf, *du = dp + np, *dj = du + np, *part = dj + 3 * np;
   QV_CUDA(c, cudaMemcpyAsync(dp, pts, sizeof(double) * np, cudaMemcpyHostToDevice, c->stream));
-  const unsigned nb = (unsigned)ng * nchunk;
   const double L = c->p.box_size;
-  switch (c->p.boundary) {
+  for (int lo = 0; lo < m; lo += slab) {
+    const int ms = std::min(slab, m - lo);
+    const double *p = dp + 3 * (size_t)lo;
+    const unsigned nb = (unsigned)nblk(ms, FW) * nchunk;
+    switch (c->p.boundary) {
 #define QV_FIELD_CASE(BCV)                                                                        \
   case BCV:                                                                                       \
     if (grad_images && BCV != QV_BC_OPEN)                                                         \
-      k_field<BCV, true><<<nb, FW * 32, 0, c->stream>>>(m, dp, na, c->src64, chunk_len, nchunk, L, \
+      k_field<BCV, true><<<nb, FW * 32, 0, c->stream>>>(ms, p, na, c->src64, chunk_len, nchunk, L, \
                                                         part);                                    \
     else                                                                                          \
-      k_field<BCV, false><<<nb, FW * 32, 0, c->stream>>>(m, dp, na, c->src64, chunk_len, nchunk,  \
+      k_field<BCV, false><<<nb, FW * 32, 0, c->stream>>>(ms, p, na, c->src64, chunk_len, nchunk,  \
                                                          L, part);                                \
     break;
-    QV_FIELD_CASE(QV_BC_OPEN)
-    QV_FIELD_CASE(QV_BC_PERIODIC)
-    QV_FIELD_CASE(QV_BC_OPENX)
-    QV_FIELD_CASE(QV_BC_OPENXY)
+      QV_FIELD_CASE(QV_BC_OPEN)
+      QV_FIELD_CASE(QV_BC_PERIODIC)
+      QV_FIELD_CASE(QV_BC_OPENX)
+      QV_FIELD_CASE(QV_BC_OPENXY)
 #undef QV_FIELD_CASE
-    default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", c->p.boundary);
+      default: return qv_fail(c, QV_ERR_UNSUPPORTED, "boundary %d", c->p.boundary);
+    }
+    QV_LAUNCH_CHECK(c);
+    k_field_reduce<<<(unsigned)(((size_t)ms * FV * 32 + 255) / 256), 256, 0, c->stream>>>(
+        ms, nchunk, part, c->p.quant_circ / (4. * QV_PI), du + 3 * (size_t)lo, dj + 9 * (size_t)lo);
+    QV_LAUNCH_CHECK(c);
+    QV_COUNT(c, 2);
   }
-  QV_LAUNCH_CHECK(c);
-  k_field_reduce<<<(unsigned)((nv * 32 + 255) / 256), 256, 0, c->stream>>>(
-      m, nchunk, part, c->p.quant_circ / (4. * QV_PI), du);
-  QV_LAUNCH_CHECK(c);
-  QV_COUNT(c, 2);
   QV_CUDA(c, cudaMemcpyAsync(u, du, sizeof(double) * np, cudaMemcpyDeviceToHost, c->stream));
-  QV_CUDA(c, cudaMemcpyAsync(dudx, du + np, sizeof(double) * 9 * (size_t)m, cudaMemcpyDeviceToHost,
+  QV_CUDA(c, cudaMemcpyAsync(dudx, dj, sizeof(double) * 9 * (size_t)m, cudaMemcpyDeviceToHost,
                              c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
   return QV_OK;

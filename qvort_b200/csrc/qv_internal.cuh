@@ -245,6 +245,29 @@ int qv_fail(qv_ctx *c, int code, const char *fmt, ...);
 
 int qv_grow(qv_ctx *c, void **ptr, size_t bytes);
 int qv_smem_optin(qv_ctx *c, const void *kernel);
+
+// The field points' buffer for one call: grown on need, and freed at the end of the
+// call when it is larger than QV_FIELD_KEEP, so that one large mesh does not hold
+// device memory for the context's whole life.
+#define QV_FIELD_KEEP ((size_t)256 << 20)
+struct FieldBuf {
+  qv_ctx *c;
+  explicit FieldBuf(qv_ctx *ctx) : c(ctx) {}
+  FieldBuf(const FieldBuf &) = delete;
+  int reserve(size_t bytes) {
+    if (bytes <= c->field_bytes) return QV_OK;
+    c->field_bytes = 0;  // the old buffer goes first
+    const int rc = qv_grow(c, (void **)&c->field_buf, bytes);
+    if (!rc) c->field_bytes = bytes;
+    return rc;
+  }
+  ~FieldBuf() {
+    if (c->field_bytes <= QV_FIELD_KEEP) return;
+    cudaFree(c->field_buf);
+    c->field_buf = nullptr;
+    c->field_bytes = 0;
+  }
+};
 void qv_phase_begin(qv_ctx *c, int ph);
 void qv_phase_end(qv_ctx *c, int ph);
 void qv_phase_end_async(qv_ctx *c, int ph);

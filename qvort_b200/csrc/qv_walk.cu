@@ -1297,11 +1297,8 @@ extern "C" int qv_field_velocity_tree(qv_ctx *c, int m, const double *pts, doubl
   const int ncell = 1 << (3 * b);
   const size_t np = 3 * (size_t)m, npart = 3 * (size_t)slab * nslot;
   const size_t need = sizeof(double) * (2 * np + npart) + sizeof(int) * ((size_t)m + ncell + 2);
-  if (need > c->field_bytes) {
-    c->field_bytes = 0;  // the old buffer goes first
-    if ((rc = qv_grow(c, (void **)&c->field_buf, need))) return rc;
-    c->field_bytes = need;
-  }
+  FieldBuf buf(c);
+  if ((rc = buf.reserve(need))) return rc;
   double *dp = c->field_buf, *du = dp + np, *part = du + np;
   int *perm = (int *)(part + npart), *cell = perm + m;
   QV_CUDA(c, cudaMemcpyAsync(dp, pts, sizeof(double) * np, cudaMemcpyHostToDevice, c->stream));

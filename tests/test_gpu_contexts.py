@@ -100,3 +100,43 @@ def test_profiled_steps_report_ghosts_and_local_term(velocity, rk3, bc):
     for ph in ("ghosts", "local", "nonlocal", "update", "wrap"):
         assert t[ph] > 0.0, ph
     assert all(np.array_equal(p, q) for p, q in zip(a.get_points(), b.get_points()))
+
+
+def _used():
+    import torch
+
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+@pytest.mark.parametrize("tree,m", [(False, 3_000_000), (True, 6_000_000)])
+def test_field_calls_give_large_buffers_back(tree, m):
+    """A context keeps at most 256 MB for its field points between calls."""
+    w = W.ring(5, 0.01, 1e-5)
+    c = _ctx(w, velocity="Tree" if tree else "BS", tree_theta=0.4 if tree else 0.0,
+             precision="fp64")
+    few = np.random.default_rng(1).uniform(-0.05, 0.05, (100, 3))
+    call = c.field_velocity_tree if tree else c.field_velocity
+    u = call(few)[0]
+    used = _used()
+    pts = np.broadcast_to(few, (m // 100, 100, 3)).reshape(m, 3)
+    v = call(pts)[0]
+    assert np.array_equal(v.reshape(-1, 100, 3), np.broadcast_to(u, (m // 100, 100, 3)))
+    assert _used() - used <= (256 << 20) + (4 << 20)  # and the allocator's granularity
+
+
+@pytest.mark.parametrize("m", [1_048_575, 1_048_577, 1_050_000])
+def test_field_points_in_several_launches(m):
+    """Direct field points either side of the largest launch: each has the value and
+    the Jacobian of a call of its own."""
+    w = W.ring(33, 0.01, 1e-5)
+    c = _ctx(w, precision="fp64")
+    rng = np.random.default_rng(m)
+    pts = rng.uniform(-0.05, 0.05, (m, 3))
+    u, J = c.field_velocity(pts)
+    at = np.unique(np.r_[0, rng.integers(0, m, 200), np.arange(1_048_570, m)[:40], m - 1])
+    v, K = c.field_velocity(pts[at])
+    # a small call cuts the sources in chunks: sums in another order
+    assert np.abs(u[at] - v).max() <= 1e-13 * np.abs(v).max()
+    assert np.abs(J[at] - K).max() <= 1e-13 * np.abs(K).max()
