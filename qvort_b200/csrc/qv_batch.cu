@@ -41,13 +41,15 @@ static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 #define BSPLIT 8   // walk items per target group: the root's children
 #define BDT 128    // source tile of the single-system direct kernel (chunk rounding)
 
-// Walk items carry 64 targets, two a lane, when there are at least this many of 32
-// targets per SM (20 for each of its 24 resident warps), and 32 otherwise, where
-// fewer and longer items leave warps idle at the end.  32 and 64 targets: 512
-// systems (175k items) 3.59 and 3.35 ms a step, 512 of 2000 to 8000 points (556k)
-// 8.85 and 7.92, 128 systems (44k) 1.11 both, 64 (22k) 0.71 and 0.73, one of 8000
-// points 0.31 and 0.36.
-#define QV_BATCH_PAIR 480
+// Walk items carry 64 targets, two a lane, when that saves at least this many items
+// per SM, and 32 otherwise: with few items the longer ones leave warps idle at the
+// end, and systems of at most 32 points fill half of a pair whatever their number
+// (9,600 of 32 points: 0.77 ms a step with items of 32 and 0.79 with 64).  32 and 64,
+// from 24,000 items saved on: 3,000 systems of 33 points 0.31 and 0.29 ms, 3,000 of 65
+// 0.54 and 0.51, 190 of 1000 points 0.82 and 0.79, 38 of 2000 to 8000 1.01 and 0.98,
+// 512 (88,000 saved) 3.59 and 3.35; below: 128 systems (22,000) 1.11 both, 64
+// (11,000) 0.71 and 0.73, one of 8000 points 0.31 and 0.36.
+#define QV_BATCH_PAIR 160
 
 // status bits
 #define BST_SINGULAR 1
@@ -786,10 +788,13 @@ extern "C" int qv_batch_create(const qv_params *p, int nsys, const int *offsets,
   std::vector<int4> sys(nsys), roots, groups;
   std::vector<int2> dsrc(nsys, make_int2(0, 0));
   std::vector<double> cost;
-  long nwalk = 0;  // walk items of 32 targets
-  for (int s = 0; s < nsys; s++)
-    if (method[s] == QV_VEL_TREE) nwalk += (long)BSPLIT * nblk(offsets[s + 1] - offsets[s], 32);
-  b->pair = nwalk >= QV_BATCH_PAIR * (long)c->sm_count;
+  // walk items that 64 targets an item save
+  long saved = 0;
+  for (int s = 0; s < nsys; s++) {
+    const int n = offsets[s + 1] - offsets[s];
+    if (method[s] == QV_VEL_TREE) saved += (long)BSPLIT * (nblk(n, 32) - nblk(n, 64));
+  }
+  b->pair = saved >= QV_BATCH_PAIR * (long)c->sm_count;
   const int gsz = b->pair ? 64 : 32;
   for (int s = 0; s < nsys; s++) {
     const int o = offsets[s], n = offsets[s + 1] - offsets[s];

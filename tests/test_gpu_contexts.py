@@ -140,3 +140,19 @@ def test_field_points_in_several_launches(m):
     # a small call cuts the sources in chunks: sums in another order
     assert np.abs(u[at] - v).max() <= 1e-13 * np.abs(v).max()
     assert np.abs(J[at] - K).max() <= 1e-13 * np.abs(K).max()
+
+
+@pytest.mark.parametrize("small,large,pair", [(9000, 0, False), (8000, 800, False),
+                                              (3000, 3000, True), (0, 2900, False),
+                                              (0, 3000, True)])
+def test_batched_walk_takes_pairs_where_they_save_items(small, large, pair):
+    """Systems of at most 32 points gain nothing from items of 64 targets, whatever
+    their number: the choice counts the items saved (160 per SM, 23,680 on 148)."""
+    from qvort_b200 import lib as L
+
+    w, v = W.ring(32, 0.01, 1e-5), W.ring(64, 0.01, 1e-5)
+    ws = [(w.x, w.infront, w.behind)] * small + [(v.x, v.infront, v.behind)] * large
+    b = L.Batch(L.default_params(**dict(w.params, velocity="Tree", tree_theta=0.4,
+                                        precision="mixed")), ws, ["Tree"] * len(ws),
+                [1e-9] * len(ws))
+    assert b.stats()["items"] == 8 * (small + (1 if pair else 2) * large)
