@@ -366,6 +366,9 @@ int qv_test_root_speculation(int mode, double bound_scale);
  * terms after its launch (results within the mixed walk's rounding of the
  * other path, same evaluation counts); 0: never; 1: always.  Process-wide. */
 int qv_test_late_level1(int mode);
+/* Test hook, no counterpart in the reference: r = 1/sqrt(a) and q = b/a of n
+ * positive normal numbers (host arrays) by the FP64 sums' own helpers. */
+int qv_test_f64(int n, const double *a, const double *b, double *r, double *q);
 /* The number of root tests the last estimate-started build left undecided
  * (see qv_test_root_speculation; 0 when the build waited for the exact sum). */
 int qv_root_undecided(qv_ctx *ctx, int *count);

@@ -29,6 +29,34 @@
 
 static inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
+// Test hook (qv_test_f64): the FP64 helpers on host arrays.
+__global__ void k_test_f64(int n, const double *__restrict__ a, const double *__restrict__ b,
+                           double *r, double *q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  r[i] = rsqrt_pos(a[i]);
+  q[i] = div_pos(b[i], a[i]);
+}
+extern "C" int qv_test_f64(int n, const double *a, const double *b, double *r, double *q) {
+  if (n < 0 || (n > 0 && (!a || !b || !r || !q))) return QV_ERR_ARG;
+  if (n == 0) return QV_OK;
+  const size_t v = sizeof(double) * (size_t)n;
+  double *d = nullptr;
+  if (cudaMalloc((void **)&d, 4 * v) != cudaSuccess) {
+    cudaGetLastError();
+    return QV_ERR_NOMEM;
+  }
+  bool ok = cudaMemcpy(d, a, v, cudaMemcpyHostToDevice) == cudaSuccess &&
+            cudaMemcpy(d + n, b, v, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) {
+    k_test_f64<<<nblk(n, 256), 256>>>(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n);
+    ok = cudaMemcpy(r, d + 2 * (size_t)n, v, cudaMemcpyDeviceToHost) == cudaSuccess &&
+         cudaMemcpy(q, d + 3 * (size_t)n, v, cudaMemcpyDeviceToHost) == cudaSuccess;
+  }
+  cudaFree(d);
+  return ok && cudaGetLastError() == cudaSuccess ? QV_OK : QV_ERR_CUDA;
+}
+
 #define DTILE 128
 #define D64_BLOCKS 3  // FP64 kernel: resident blocks per SM (2, 3 and 4 run within 2 %)
 

@@ -141,6 +141,7 @@ _SIGS = {
     "qv_test_stage_timeout": [C.c_int],
     "qv_test_root_speculation": [C.c_int, C.c_double],
     "qv_test_late_level1": [C.c_int],
+    "qv_test_f64": [C.c_int, _P, _P, _P, _P],
     "qv_root_undecided": [_P, _I],
     "qv_velocity_direct_noalloc": [C.POINTER(QvParams), C.c_int, _P, _P, _P, _P, _P],
     "qv_velocity_device": [_P, _P],
@@ -606,6 +607,17 @@ def test_root_speculation(mode: int = -1, bound_scale: float = 1.0) -> None:
     rc = _lib.qv_test_root_speculation(int(mode), float(bound_scale))
     if rc < 0:
         raise QvError(rc, "bad root speculation setting")
+
+
+def test_f64(a, b):
+    """Test hook: (1/sqrt(a), b/a) by the FP64 sums' helpers."""
+    a, b = _f64(a), _f64(b)
+    assert a.shape == b.shape
+    r, q = np.empty_like(a), np.empty_like(a)
+    rc = _lib.qv_test_f64(a.size, _ptr(a), _ptr(b), _ptr(r), _ptr(q))
+    if rc < 0:
+        raise QvError(rc, "qv_test_f64 failed")
+    return r, q
 
 
 def probe_fp32(stream: int | None = None) -> float:
