@@ -935,12 +935,14 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
         m.nb = c->adj_nb; m.xb = c->adj_xb; m.gib = c->adj_gib;
         const int ntop = std::min(t.n_nodes, MV_TOP);
         k_moment_vjp_top<<<dim3(ntop - 1, MV_SPLIT), 256, 0, c->stream>>>(m, ntop);
-        if (t.n_nodes > ntop)
-          k_moment_vjp<<<nblk(t.n_nodes - ntop, 8), 256, 0, c->stream>>>(m, ntop, t.n_nodes);
-        QV_LAUNCH_CHECK(c);
         QV_COUNT(c, 1);
+        if (t.n_nodes > ntop) {
+          k_moment_vjp<<<nblk(t.n_nodes - ntop, 8), 256, 0, c->stream>>>(m, ntop, t.n_nodes);
+          QV_COUNT(c, 1);
+        }
+        QV_LAUNCH_CHECK(c);
       }
-      QV_COUNT(c, 2);
+      QV_COUNT(c, 1);
     }
   }
   k_ghost_vjp<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->infront, c->behind, c->adj_xb,

@@ -156,3 +156,26 @@ def test_batched_walk_takes_pairs_where_they_save_items(small, large, pair):
                                         precision="mixed")), ws, ["Tree"] * len(ws),
                 [1e-9] * len(ws))
     assert b.stats()["items"] == 8 * (small + (1 if pair else 2) * large)
+
+
+def test_launch_count_of_a_tree_gradient():
+    """A tree of at most 585 nodes needs one moment kernel, a larger one two."""
+    import torch
+
+    from qvort_b200 import lib as L
+
+    n = []
+    for m in (64, 2000):
+        w = W.ring(m, 0.01, 1e-5)
+        c = L.Context(L.default_params(**dict(w.params, velocity="Tree", tree_theta=0.4,
+                                              precision="fp64")), stream=1)
+        c.set_points(w.x, w.infront, w.behind)
+        c.velocity()
+        nodes = c.tree_info()[0]
+        assert (nodes <= 585) == (m == 64)
+        x, y = (torch.ones(m, 3, dtype=torch.float64, device="cuda") for _ in range(2))
+        c.velocity_vjp(x.data_ptr(), y.data_ptr())
+        k = c.counters()["launches"]
+        c.velocity_vjp(x.data_ptr(), y.data_ptr())
+        n.append(c.counters()["launches"] - k)
+    assert n[1] == n[0] + 1
