@@ -366,6 +366,11 @@ int qv_test_root_speculation(int mode, double bound_scale);
  * terms after its launch (results within the mixed walk's rounding of the
  * other path, same evaluation counts); 0: never; 1: always.  Process-wide. */
 int qv_test_late_level1(int mode);
+/* Test hook, no counterpart in the reference: the FP64 direct sum takes its kernel
+ * for few points up to small_slots slots (0: always the tile kernel), and its
+ * gradient at most vjp_part_bytes of partial sums a launch (at least 32 targets);
+ * -1: the defaults, 4096 slots and 256 MB.  Process-wide. */
+int qv_test_direct_split(int small_slots, long long vjp_part_bytes);
 /* Test hook, no counterpart in the reference: r = 1/sqrt(a) and q = b/a of n
  * positive normal numbers (host arrays) by the FP64 sums' own helpers. */
 int qv_test_f64(int n, const double *a, const double *b, double *r, double *q);

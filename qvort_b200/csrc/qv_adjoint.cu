@@ -132,7 +132,7 @@ __global__ void k_lia_vjp(int n, const double *__restrict__ x, const int *__rest
 // two blocks per SM and 0.4 ms more).
 #define VT 128  // sources per block
 #define VG 32   // targets per shared-memory tile
-#define QV_DVJP_PART ((size_t)256 << 20)  // bytes of per-target partial sums per launch
+size_t g_dvjp_part = QV_DVJP_PART;  // qv_test_direct_split lowers it
 
 // Sum of (v0, v1, v2) over the warp: lanes 0, 8 and 16 return the three sums.
 __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
@@ -855,7 +855,7 @@ extern "C" int qv_velocity_vjp(qv_ctx *c, const double *ubar, double *xbar) {
       // targets are taken in several launches.
       const int nsb = nblk(na, VT);
       const size_t row = sizeof(double) * 3 * (size_t)nsb;
-      const int slab = (int)std::min<size_t>(na, std::max<size_t>(VG, QV_DVJP_PART / row / VG * VG));
+      const int slab = (int)std::min<size_t>(na, std::max<size_t>(VG, g_dvjp_part / row / VG * VG));
       // ten blocks per resident slot (3 per SM; with five the last wave cost 5 %),
       // each with enough pairs (targets x images) to outweigh its start and its
       // partial sums

@@ -466,10 +466,16 @@ __global__ void __launch_bounds__(D64S) k_direct64_small(int n, const double *__
 // 4,000 145 and 130, 6,000 218 and 230; periodic 120 and 56, 143 and 105, 885 and
 // 838, 1,805 and 1,791.  Above, the tile kernel reads each source once for 128
 // targets and the call no longer hangs on its launches.  The test hook of the
-// tile kernels' waits keeps them in use.
+// tile kernels' waits keeps them in use, and qv_test_direct_split moves the limit.
 #define QV_D64_SMALL 4096
+static int g_small_slots = QV_D64_SMALL;
 bool qv_direct_small(const qv_params *p, int n) {
-  return p->precision == QV_PREC_FP64 && n <= QV_D64_SMALL && !g_stage_fail;
+  return p->precision == QV_PREC_FP64 && n <= g_small_slots && !g_stage_fail;
+}
+extern "C" int qv_test_direct_split(int small_slots, long long vjp_part_bytes) {
+  g_small_slots = small_slots < 0 ? QV_D64_SMALL : small_slots;
+  g_dvjp_part = vjp_part_bytes < 0 ? QV_DVJP_PART : (size_t)vjp_part_bytes;
+  return QV_OK;
 }
 
 static int launch_direct_small(cudaStream_t st, const qv_params *p, int n, const double *x,

@@ -282,6 +282,9 @@ int qv_launch_ghosts_wrap(qv_ctx *c);  // ghostp, wrap and NaN test at the end o
 int qv_launch_direct(qv_ctx *c);
 // whether the direct sum of n slots takes a block per target (no active list)
 bool qv_direct_small(const qv_params *p, int n);
+// Bytes of per-target partial sums that one launch of its gradient takes.
+#define QV_DVJP_PART ((size_t)256 << 20)
+extern size_t g_dvjp_part;
 int qv_launch_tree_build(qv_ctx *c);
 // Join the exact root centroid and re-pack the root with it, and join the late
 // level-1 moments and payloads (no-op when both are in already).  Every reader

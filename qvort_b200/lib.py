@@ -141,6 +141,7 @@ _SIGS = {
     "qv_test_stage_timeout": [C.c_int],
     "qv_test_root_speculation": [C.c_int, C.c_double],
     "qv_test_late_level1": [C.c_int],
+    "qv_test_direct_split": [C.c_int, C.c_longlong],
     "qv_test_f64": [C.c_int, _P, _P, _P, _P],
     "qv_root_undecided": [_P, _I],
     "qv_velocity_direct_noalloc": [C.POINTER(QvParams), C.c_int, _P, _P, _P, _P, _P],
@@ -607,6 +608,12 @@ def test_root_speculation(mode: int = -1, bound_scale: float = 1.0) -> None:
     rc = _lib.qv_test_root_speculation(int(mode), float(bound_scale))
     if rc < 0:
         raise QvError(rc, "bad root speculation setting")
+
+
+def test_direct_split(small_slots: int = -1, vjp_part_bytes: int = -1) -> None:
+    """Test hook: the slots up to which the FP64 direct sum takes a block per target,
+    and the bytes of partial sums of one launch of its gradient; -1: the defaults."""
+    _lib.qv_test_direct_split(int(small_slots), int(vjp_part_bytes))
 
 
 def test_f64(a, b):
