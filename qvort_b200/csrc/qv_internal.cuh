@@ -346,8 +346,9 @@ void qv_populate(void *p, size_t bytes);
 
 // ---------------------------------------------------------------- helpers
 // 1/sqrt(a) and 1/a of a normal number: what rsqrtf and the fast division give
-// there, without their handling of subnormal operands (three instructions of a
-// square root's four).  A subnormal a gives infinity.
+// there, from PTX's approximate instructions, which take subnormal operands as
+// zeros: a subnormal a gives infinity.  Mixed direct sum of 23,500 points and 27
+// images: 15.1 -> 13.0 ms.
 __device__ __forceinline__ float rsqrt_normal(float a) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));

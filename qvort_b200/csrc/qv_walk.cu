@@ -132,7 +132,8 @@ __device__ __forceinline__ void slot_shift(int bc, int sl, double L, double *s) 
 // with a square root and a division per test and eight divisions per far cell,
 // 0.53 ms with these and 0.47 in the task order of task_slot; large tangle (796k
 // points, theta 0.5): 24 -> 12.6 ms.  Taking 2 or 4 nodes at a time for 16 or 8
-// targets ran no faster (0.55 and 0.52 ms against 0.53; 13.2 and 13.8), and a target's sums would then depend on its group.
+// targets ran no faster (0.55 and 0.52 ms against 0.53; 13.2 and 13.8), and a
+// target's sums would then depend on its group.
 template <int BC>
 __device__ __forceinline__ void walk64_body(const WalkArgs &a) {
   constexpr int NIMG = BC == QV_BC_PERIODIC ? 26 : BC == QV_BC_OPENX ? 8 : BC == QV_BC_OPENXY ? 2 : 0;
@@ -869,8 +870,9 @@ __global__ void k_root_fix(WalkArgs a, int bc, const int4 *__restrict__ unc, int
 // The root children's far-field terms that the mixed walk deferred (late_cell),
 // once their moments and payloads are in: for each (task slot, target) whose
 // byte is set, the reference's far-cell term (src/tree.f90:394-413) of each
-// flagged child, in child order, in FP64 from the FP64 header and payload, as
-// the FP64 walk takes it, added to that task's partial sum after the walk's
+// flagged child, in child order, in FP64 from the FP64 header and payload (with a
+// rounded square root and divisions: a few terms a target, far_term64's reciprocal
+// root would gain nothing), added to that task's partial sum after the walk's
 // compensated FP32 sum.
 __global__ void k_walk_l1_fix(WalkArgs a, int bc, int ntask) {
   const size_t tot = (size_t)ntask * a.n_act;
