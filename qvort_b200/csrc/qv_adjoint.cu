@@ -120,16 +120,16 @@ __global__ void k_lia_vjp(int n, const double *__restrict__ x, const int *__rest
 // One pass over all (source, target) pairs gives both ends' gradients: a thread
 // holds one source and sums its own (dL/dx_j at fixed s, dL/ds) over a chunk of
 // targets, while each target's gradient -- minus the sum over sources -- is
-// reduced over the warp (12 shuffles a target against 27 images x ~45 FP64
+// reduced over the warp (12 shuffles a target against 27 images x ~50 FP64
 // operations a lane) and over the block's warps in shared memory.  Partial
 // sums per (source block, target) and per (target chunk, source) are added in
 // a fixed order by k_dvjp_reduce, so results are deterministic, with no
 // atomics.  A two-pass split (a thread per target, then a thread per source)
 // evaluates every pair twice.  Bound: FP64 issue.  6,400 points, 27 images:
 // velocity and gradient together took 333 ms with two passes, divisions in every
-// image term and 50 blocks; 6.9 ms now, 2 of them the velocity (78 % of the FP64
-// rate at about 55 operations a pair; the x shifts unrolled took 255 registers,
-// two blocks per SM and 0.4 ms more).
+// image term and 50 blocks; 6.9 ms now, 2 of them the velocity (this kernel 4.7,
+// 77 % of the FP64 rate at 52 operations a pair and image; the x shifts unrolled
+// took 255 registers, two blocks per SM and 0.4 ms more).
 #define VT 128  // sources per block
 #define VG 32   // targets per shared-memory tile
 size_t g_dvjp_part = QV_DVJP_PART;  // qv_test_direct_split lowers it
@@ -250,7 +250,7 @@ __global__ void k_dvjp_reduce(int na, const int *__restrict__ act, int t_lo, int
 // the far-field gradient need one reciprocal square root, as in the velocity
 // walk.
 //
-// Bound: instruction issue (36 % of it FP64).  50,000 points, 27 images, theta
+// Bound: instruction issue (a third of it FP64).  50,000 points, 27 images, theta
 // 0.4: 2.28 ms with a rounded square root and division per test, 15 separate
 // warp sums and 15 atomics by one lane per node; 0.97 ms now.  Two or four
 // nodes at a time for 16 or 8 targets send two to four times the atomics,

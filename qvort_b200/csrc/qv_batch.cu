@@ -592,7 +592,7 @@ struct PackArgsB {
 // (the pack, the items and the update used to be separate launches with the
 // same order).  Nothing is updated when any status bit is set (a forest or
 // stack overflow makes the host resize and run the step again).  Ghosts and
-// LIA stay separate launches before the forest build: the forest's moments
+// LIA stay a launch of their own before the forest build: the forest's moments
 // need the ghosts, and LIA keeps the single-system kernel's arithmetic (its
 // file is compiled without FMA contraction).
 // 80 registers: six blocks of 128 threads per SM (the pairs left to themselves take

@@ -355,11 +355,11 @@ __device__ __forceinline__ TilePipe make_pipe(const void *src, int j0, int j1, c
 
 // ------------------------------------------------------------ FP64 kernel
 // One thread per target, each staged source summed against it in all images
-// (Seg64).  Bound: FP64 issue, about 26 operations a pair (two rsqrt_pos and
-// one div_pos are 14 of them).  23,500 points, 27 images: 70.3 ms with the
+// (Seg64).  Bound: FP64 issue, about 27 operations a pair (two rsqrt_pos and
+// one div_pos are 14 of them).  23,457 points, 27 images: 70.3 ms with the
 // reference's formula pair by pair (library rsqrt and division, 1.3 waves of
-// blocks), 26.0 ms now = 5.7e11 pairs/s; the FP64 pipe is busy 84 % of the
-// time (24,700 points, 28.8 ms).
+// blocks), 25.5 ms now = 5.8e11 pairs/s; the FP64 pipe is busy 85 % of the
+// time.
 template <int BC>
 __global__ void __launch_bounds__(DTILE, D64_BLOCKS) k_direct64(int na, const int *__restrict__ act,
                                                     const double *__restrict__ x,
