@@ -773,16 +773,48 @@ extern "C" int qv_velocity(qv_ctx *c, double *u, double *u_li, double *u_bs, lon
   return velocity_collect(c, eval_count);
 }
 
-// The velocities into a device array, which is written only once the status is
-// known: after an error it holds what it held.
+// Copies n values unless the status word reports an error.
+__global__ void k_copy_if_ok(size_t n, const double *__restrict__ src, double *__restrict__ dst,
+                             const int *__restrict__ status) {
+  if (*status) return;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
+       e += (size_t)gridDim.x * blockDim.x)
+    dst[e] = src[e];
+}
+
+// Whether p[0 .. n) is aligned and begins and ends in memory of the current device.
+static bool on_device(const double *p, size_t n) {
+  int dev = 0;
+  cudaPointerAttributes a, b;
+  const bool ok = reinterpret_cast<size_t>(p) % sizeof(double) == 0 &&
+                  cudaGetDevice(&dev) == cudaSuccess &&
+                  cudaPointerGetAttributes(&a, p) == cudaSuccess &&
+                  cudaPointerGetAttributes(&b, p + n - 1) == cudaSuccess &&
+                  a.type == cudaMemoryTypeDevice && a.device == dev &&
+                  b.type == cudaMemoryTypeDevice && b.device == dev;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// The velocities into a device array, which after an error holds what it held: the
+// copy looks at the status word where the call would otherwise wait for it first (a
+// second wait: 1000 points, direct sum, 79 us against 72).  Anything but memory of
+// this device goes to the runtime, which knows what it can copy to.
 extern "C" int qv_velocity_device(qv_ctx *c, double *u_out) {
   if (!c || !u_out) return QV_ERR_ARG;
   if (c->n == 0) return QV_OK;
   int rc = velocity_launch(c);
   if (rc) return rc;
+  const size_t n = 3 * (size_t)c->n;
+  if (on_device(u_out, n)) {
+    k_copy_if_ok<<<(int)std::min<size_t>((n + 255) / 256, 8 * (size_t)c->sm_count), 256, 0,
+                   c->stream>>>(n, c->u, u_out, c->dstatus);
+    QV_LAUNCH_CHECK(c);
+    QV_COUNT(c, 1);
+    return velocity_collect(c, nullptr);
+  }
   if ((rc = velocity_collect(c, nullptr))) return rc;
-  QV_CUDA(c, cudaMemcpyAsync(u_out, c->u, sizeof(double) * 3 * (size_t)c->n,
-                             cudaMemcpyDeviceToDevice, c->stream));
+  QV_CUDA(c, cudaMemcpyAsync(u_out, c->u, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
   QV_CUDA(c, cudaStreamSynchronize(c->stream));
   return QV_OK;
 }

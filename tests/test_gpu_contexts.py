@@ -179,3 +179,25 @@ def test_launch_count_of_a_tree_gradient():
         c.velocity_vjp(x.data_ptr(), y.data_ptr())
         n.append(c.counters()["launches"] - k)
     assert n[1] == n[0] + 1
+
+@pytest.mark.parametrize("n", [5, 1000, 100_000])
+def test_velocity_device_writes_its_array_and_nothing_else(n):
+    """Into the middle of a device array (copied by a kernel) and of a pinned one (by the
+    runtime): the velocities of the host call, and nothing around them."""
+    import torch
+
+    w = W.ring(n, 0.01, 1e-5)
+    c = _ctx(w, velocity="LIA" if n > 5000 else "BS", precision="fp64")
+    u = c.velocity()[0]
+    for kw in (dict(device="cuda"), dict(pin_memory=True)):
+        a = torch.full((3 * n + 9,), 7.0, dtype=torch.float64, **kw)
+        torch.cuda.synchronize()
+        c.velocity_device(a.data_ptr() + 8 * 4)
+        a = a.cpu().numpy()
+        assert np.array_equal(a[4:4 + 3 * n].reshape(n, 3), u)
+        assert (a[:4] == 7.0).all() and (a[4 + 3 * n:] == 7.0).all()
+    # an address that is no multiple of eight: the runtime's copy as well
+    b = torch.zeros(24 * n + 4, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    c.velocity_device(b.data_ptr() + 4)
+    assert np.array_equal(b.cpu().numpy()[4:].view(np.float64).reshape(n, 3), u)
