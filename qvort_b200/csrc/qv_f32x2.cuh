@@ -1,4 +1,4 @@
-// qv_f32x2.cuh -- packed FP32 pairs on sm_100 (FADD2 / FMUL2 / FFMA2).
+// qv_f32x2.cuh -- packed FP32 pairs on sm_100 (PTX add, mul and fma on f32x2).
 //
 // A kernel that computes the same FP32 expression for two targets keeps the
 // two values of each operand in one float2 and issues one packed instruction
