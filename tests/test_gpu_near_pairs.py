@@ -2,7 +2,7 @@
 target close to either end of a segment (filaments about to reconnect, a
 quasiparticle beside a line).
 
-The checker takes every derivative by a complex step of 1e-40 in 80-bit long
+The comparison takes every derivative by a complex step of 1e-40 in 80-bit long
 doubles, exact to their 5e-20, from the segment factor written with R1 and R2
 themselves.  All coordinates are multiples of 2^-40, so x_j - x_i, ghost_j - x_i and
 ghost_j - x_j hold exactly in FP64 and every error is the kernel's own.  Bound:
